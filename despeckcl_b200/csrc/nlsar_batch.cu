@@ -22,6 +22,7 @@
 #include "../../include/despeckcl_b200.h"
 #include "dcl_internal.h"
 #include "nlsar_plan.h"
+#include "nlsar_split.h"
 
 struct dcl_nlsar_batch {
   dcl::Plan pl;
@@ -33,6 +34,10 @@ struct dcl_nlsar_batch {
   char* scratch = nullptr;
   dcl::SceneDesc* d_desc = nullptr;
   size_t smem = 0;
+  bool split = false;  // two kernels around a volume of weight indices (nlsar_split.cu)
+  dcl::SplitLayout lay;
+  dcl::SplitSeg* d_segs = nullptr;
+  uint32_t* d_vol = nullptr;
   int variant = 0;
   bool tuned = false;
   cudaStream_t cap = nullptr;
@@ -91,6 +96,7 @@ int enqueue(dcl_nlsar_batch* b, cudaStream_t st) {
     const int rc = launch_prep(b->pl, b->geo[i], b->desc[i], b->a1[i], b->a2[i], b->phi[i], nullptr, st);
     if (rc) return rc;
   }
+  if (b->split) return launch_split_all(b->pl, b->pl.P, b->lay, b->d_desc, b->d_segs, b->d_vol, st);
   return launch_fused(b->pl, b->pl.P, b->d_desc, b->smem, st, b->variant);
 }
 
@@ -140,7 +146,7 @@ void tune_store_locked() {
 }
 
 int autotune(dcl_nlsar_batch* b, cudaStream_t st) {
-  if (!uses_specialised_kernel(b->pl)) return DCL_OK;
+  if (b->split || !uses_specialised_kernel(b->pl)) return DCL_OK;
   const std::string key = tune_key(b);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -266,7 +272,27 @@ extern "C" dcl_nlsar_batch* dcl_nlsar_batch_create(int n, const float* const* a1
   }
   const size_t desc_bytes = (n * sizeof(SceneDesc) + 255) / 256 * 256;
   const size_t wtab_bytes = b->pl.wtab.size() * sizeof(float);
-  cudaError_t e = cudaMalloc(&b->scratch, total + desc_bytes + wtab_bytes);
+  const size_t wtab_pad = (wtab_bytes + 255) / 256 * 256;
+  // the two-kernel path unless a variant of the fused kernel is asked for; a
+  // smaller volume, then the fused kernel, where the device has no room
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::vector<SplitJob> jobs;
+  for (int i = 0; i < n; ++i) jobs.push_back({i, 0, b->geo[i].vH + 1});
+  size_t budget = kSplitBudgetBytes / sizeof(uint32_t), seg_bytes = 0;
+  b->split = !(flags & (DCL_BATCH_VARIANT1 | DCL_BATCH_VARIANT2)) && split_supported(b->pl.P, false) &&
+             split_layout(b->pl, b->geo, jobs, budget, sm_count(dev), b->lay);
+  cudaError_t e = cudaSuccess;
+  for (;;) {
+    seg_bytes = b->split ? (b->lay.segs.size() * sizeof(SplitSeg) + 255) / 256 * 256 : 0;
+    const size_t vol = b->split ? b->lay.vol_words * sizeof(uint32_t) : 0;
+    e = cudaMalloc(&b->scratch, total + desc_bytes + wtab_pad + seg_bytes + vol);
+    if (e != cudaErrorMemoryAllocation || !b->split) break;
+    cudaGetLastError();
+    budget /= 4;
+    b->split = budget >= kSplitMinBudgetBytes / sizeof(uint32_t) &&
+               split_layout(b->pl, b->geo, jobs, budget, sm_count(dev), b->lay);
+  }
   if (e != cudaSuccess) {
     cuda_error(e, "cudaMalloc(batch scratch)");
     release(b);
@@ -279,6 +305,12 @@ extern "C" dcl_nlsar_batch* dcl_nlsar_batch_create(int n, const float* const* a1
     return nullptr;
   }
   e = cudaMemcpy(d_wtab, b->pl.wtab.data(), wtab_bytes, cudaMemcpyHostToDevice);
+  if (b->split) {
+    b->d_segs = reinterpret_cast<SplitSeg*>(b->scratch + total + desc_bytes + wtab_pad);
+    b->d_vol = reinterpret_cast<uint32_t*>(b->scratch + total + desc_bytes + wtab_pad + seg_bytes);
+    if (e == cudaSuccess)
+      e = cudaMemcpy(b->d_segs, b->lay.segs.data(), b->lay.segs.size() * sizeof(SplitSeg), cudaMemcpyHostToDevice);
+  }
   if (e != cudaSuccess) {
     cuda_error(e, "cudaMemcpy(batch weight tables)");
     release(b);
@@ -345,7 +377,7 @@ extern "C" int dcl_nlsar_batch_launches(const dcl_nlsar_batch* b) {
   if (!b) return 0;
   int used = 0;
   for (char u : b->pl.slot_used) used += u ? 1 : 0;
-  return (int)b->desc.size() * (1 + used) + 1;
+  return (int)b->desc.size() * (1 + used) + (b->split ? split_launches(b->lay) : 1);
 }
 
 extern "C" void dcl_nlsar_batch_destroy(dcl_nlsar_batch* b) { release(b); }

@@ -32,19 +32,16 @@
 
 #include <cuda_runtime.h>
 
-#include <cuda_fp16.h>
-
 #include <cstdint>
 #include <mutex>
 
 #include "dcl_internal.h"
 #include "nlsar_common.cuh"
+#include "nlsar_math.cuh"
 
 namespace dcl {
 
 namespace {
-
-__host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
 
 // Shared-memory layout and launch shape of one instantiation: staging halo
 // PHX_ (the call's largest patch half), at most NPX_ patch sizes per pass,
@@ -107,11 +104,6 @@ struct FastL {
   static_assert(TH % PX == 0 && TH % 4 == 0, "tile rows");
 };
 
-template <int PH0, int PH1, int PH2>
-__host__ __device__ constexpr int np_of() {
-  return (PH0 >= 0) + (PH1 >= 0) + (PH2 >= 0);
-}
-
 // ---- TMA staging through one mbarrier --------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -172,100 +164,6 @@ __device__ __forceinline__ bool stage_wait(const FilterParams& P, uint64_t* bar,
 }
 
 __global__ void take_stage_timeouts_kernel() { g_stage_taken = atomicExch(&g_stage_timeouts, 0); }
-
-// Arithmetic variants of the similarity and the sums (the precision study;
-// kPrecRatio is the default):
-//   kPrecRatio  the GLR as one base-2 log of the ratio
-//               det(A+B)^2 / (2^4 det A det B) (sim_measures.h:52-64 is the
-//               natural log of that ratio), with 1/(4 det) of every staged
-//               pixel precomputed; the similarities and patch sums are in
-//               log2 units and the weight lookup scales by ln 2.  No large
-//               logs cancel, so the similarity keeps about 1e-7 absolute
-//               accuracy where the log form loses the ulps of ln det (~1e-6)
-//   kPrecLog2   the log form 2 ln det(A+B) - ln det A - ln det B - 4 ln 2 with
-//               the per-pixel ln det staged and an approximate base-2 log
-//   kPrecLogf   the log form with the correctly rounded logf, the reference's
-//               arithmetic
-//   kPrecKahan  kPrecRatio with Kahan-compensated patch sums and accumulators
-//   kPrecHalf   kPrecRatio with every similarity rounded to FP16, as FP16
-//               staging of the similarity map would store it
-enum { kPrecRatio = 0, kPrecLog2 = 1, kPrecLogf = 2, kPrecKahan = 3, kPrecHalf = 4 };
-
-template <int PV>
-__host__ __device__ constexpr bool ratio_form() {
-  return PV == kPrecRatio || PV == kPrecKahan || PV == kPrecHalf;
-}
-
-// det of a staged scaled covariance, rounded like the prep kernel's
-// (sim_measures.h:31-34)
-__device__ __forceinline__ float det_of(const float4 c) {
-  return __fsub_rn(__fmul_rn(c.x, c.y), __fadd_rn(__fmul_rn(c.z, c.z), __fmul_rn(c.w, c.w)));
-}
-
-// The per-pixel term of a staged pixel: ln det (log forms) or 1/(4 det)
-// (ratio form; NaN for a negative det, whose log is NaN, +inf for det 0).
-template <int PV>
-__device__ __forceinline__ float pixel_term(const float4 c) {
-  const float d = det_of(c);
-  if (!ratio_form<PV>()) return logf(d);
-  return d >= 0.0f ? __fdiv_rn(0.25f, fabsf(d)) : __int_as_float(0x7fffffff);
-}
-
-// load of one float from a 32-bit shared-memory address, for tables that
-// stay unchanged while they are read (the compiler may schedule it freely)
-__device__ __forceinline__ float lds_f32(uint32_t addr) {
-  float v;
-  asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-  return v;
-}
-
-__device__ __forceinline__ float lg2_ftz(float x) {
-  float y;
-  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-__device__ __forceinline__ float kahan_add(float s, float x, float& c) {
-  const float y = x - c;
-  const float t = s + y;
-  c = (t - s) - y;
-  return t;
-}
-
-template <int PV>
-__device__ __forceinline__ float glr_sim(const float4 a, float la, const float4 b, float lb, float c2d) {
-  // sim_measures.h:52-64 with nlooks 1 and the per-pixel terms precomputed;
-  // NaN -> 0.  Each form is exactly symmetric in (A, B), which gives the
-  // mirrored half window the reference's values (copy_symm_weights.cl:56-76).
-  const float2 d01 = __fadd2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y));
-  const float2 d23 = __fadd2_rn(make_float2(a.z, a.w), make_float2(b.z, b.w));
-  const float s00 = d01.x, s11 = d01.y, sre = d23.x, sim = d23.y;
-  const float det = (s00 * s11) - (sre * sre + sim * sim);
-  float r;
-  if (ratio_form<PV>()) {
-    // log2 of det |det| / (16 det A det B): negative (NaN log) when det < 0
-    r = lg2_ftz((det * fabsf(det)) * (la * lb));
-    if (PV == kPrecHalf) r = __half2float(__float2half_rn(r));
-  } else {
-    const float t = (la + lb) + c2d;
-    r = (PV == kPrecLogf) ? 2.0f * logf(det) - t : fmaf(2.0f * 0.69314718f, __log2f(det), -t);
-  }
-  if (r != r) r = 0.0f;
-  return r;
-}
-
-// patch half size of pass component j (compile time)
-template <int PH0, int PH1, int PH2>
-__device__ __forceinline__ constexpr int ph_of(int j) {
-  return j == 0 ? PH0 : (j == 1 ? PH1 : PH2);
-}
-
-// Selection state of a thread's PX pixels, kept across the passes.
-template <int PX, int NM>
-struct Best {
-  float e[PX], a[PX], s0[PX], m[PX][NM];
-  int rank[PX], combo[PX];
-};
 
 // One pass (one scale, the patch halves PH0 < PH1 < PH2 of this pass, -1
 // where unused) over all search-window offsets, on the staged tile; its
@@ -557,35 +455,7 @@ __device__ __forceinline__ void fast_pass(const FilterParams& P, const PassParam
         A[a] = (i & 1) ? acc[i / 2][j][a].y : acc[i / 2][j][a].x;
         if (PV == kPrecKahan && a < NKC) A[a] -= (i & 1) ? kc[i / 2][j][a].y : kc[i / 2][j][a].x;
       }
-      const float s0 = A[0], s1 = A[1], s2 = A[2], s3 = A[3], s4 = A[4], s5 = A[5], s6 = A[6], s7 = A[7];
-      const float enl = s0 * s0 / s1;
-      const float i0 = s2 / s0, i1 = s3 / s0;
-      const float v0 = s4 / s0 - i0 * i0, v1 = s5 / s0 - i1 * i1;
-      float alpha = 0.0f;
-      alpha = fmaxf(alpha, fmaxf(0.0f, (v0 - i0 * i0) / v0));
-      alpha = fmaxf(alpha, fmaxf(0.0f, (v1 - i1 * i1) / v1));
-      if (P.alpha_zero) alpha = 0.0f;
-      const float oma = 1.0f - alpha;
-      const float enb = enl / (oma * oma + (alpha * alpha + 2.0f * alpha * (1.0f - alpha) / s0) * enl);
-      const int combo = pp.combo[j];
-      const int rank = P.combo[combo].rank;
-      const bool take = (P.select_mode == 0) || (enb > best.e[i]) || (enb == best.e[i] && rank < best.rank[i]);
-      const bool take_fb = !take && best.combo[i] < 0 && combo == P.fallback_combo;
-      if (take) {
-        best.e[i] = enb;
-        best.rank[i] = rank;
-      }
-      if (take || take_fb) {
-        best.combo[i] = combo;
-        best.a[i] = alpha;
-        best.s0[i] = s0;
-        best.m[i][0] = s2;
-        best.m[i][1] = s3;
-        best.m[i][2] = s6;
-        best.m[i][3] = s7;
-#pragma unroll
-        for (int e = 4; e < NM; ++e) best.m[i][e] = A[(e + 4) % NA];
-      }
+      select_combo(P, pp.combo[j], A, i, best);
     }
   }
 }
@@ -701,35 +571,9 @@ __global__ void __launch_bounds__(FastK<WSH, PHX, A0, A1, A2, B0, B1, B2, PX_, T
       const int ox = (vx < S.W - 1) ? vx : (vx == S.vW ? S.W - 1 : -1);
       if (oy < 0 || ox < 0) continue;
       const int ci = (y + WSH) * RO + (lane + WSH);
-      const float4 c = sCo[ci];
-      const float alpha = best.a[i], s0 = best.s0[i];
-      const float oma = 1.0f - alpha;
-      const float c00 = oma * best.m[i][0] / s0 + alpha * c.x;
-      const float c11 = oma * best.m[i][1] / s0 + alpha * c.y;
-      const float cre = oma * best.m[i][2] / s0 + alpha * c.z;
-      const float cim = oma * best.m[i][3] / s0 + alpha * c.w;
-      const size_t o = (size_t)oy * S.W + ox;
-      if (FULL8) {
-        // planes {Re, Im} of C00, C01, C10, C11; the second staged float4 is
-        // {Im C00, Re C10, Im C10, Im C11}
-        const float4 c2 = sCo2[ci];
-        const size_t n = (size_t)S.H * S.W;
-        S.cov_out[o] = c00;
-        S.cov_out[n + o] = oma * best.m[i][4 % NM] / s0 + alpha * c2.x;
-        S.cov_out[2 * n + o] = cre;
-        S.cov_out[3 * n + o] = cim;
-        S.cov_out[4 * n + o] = oma * best.m[i][5 % NM] / s0 + alpha * c2.y;
-        S.cov_out[5 * n + o] = oma * best.m[i][6 % NM] / s0 + alpha * c2.z;
-        S.cov_out[6 * n + o] = c11;
-        S.cov_out[7 * n + o] = oma * best.m[i][7 % NM] / s0 + alpha * c2.w;
-      } else {
-        const float am = sqrtf(c00), as = sqrtf(c11);
-        const float r = 0.5f * (am + as);
-        S.ref[o] = r * r;
-        S.phase[o] = atan2f(cim, cre);
-        S.coh[o] = sqrtf(cim * cim + cre * cre) / (am * as);
-      }
-      if (S.sel_out) S.sel_out[o] = best.combo[i];
+      float4 c2 = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (FULL8) c2 = sCo2[ci];
+      write_pixel<FULL8>(S, (size_t)oy * S.W + ox, sCo[ci], c2, i, best);
     }
   }
 }

@@ -25,6 +25,7 @@
 #include "dcl_internal.h"
 #include "nlsar_common.cuh"
 #include "nlsar_plan.h"
+#include "nlsar_split.h"
 
 namespace dcl {
 
@@ -291,6 +292,8 @@ int choose_k(const Plan& pl, size_t& smem_bytes) {
   return 0;
 }
 
+static size_t pad256(size_t b) { return (b + 255) / 256 * 256; }
+
 SceneGeom scene_geom(const Plan& pl, int H, int W) {
   SceneGeom g;
   g.H = H;
@@ -465,24 +468,51 @@ int launch_prep(const Plan& pl, const SceneGeom& g, const SceneDesc& d, const fl
   return launch_prep_rows(pl, g, d, a1, a2, phi, cov_in, 0, g.Hp, 0, g.Hp, st);
 }
 
-int launch_fused(const Plan& pl, const FilterParams& F, const SceneDesc* d_scenes, size_t smem, cudaStream_t st,
-                 int variant) {
+// CUDA events around one call's filter launches while dcl_profile_begin is active
+template <class Launch>
+static cudaError_t profiled(cudaStream_t st, int kernels, Launch launch) {
   cudaEvent_t a = nullptr, b = nullptr;
   if (g_prof.on) {
     cudaEventCreate(&a);
     cudaEventCreate(&b);
     cudaEventRecord(a, st);
   }
-  const bool fast = pl.fast && fast_kernel_supported(F, pl.full8);
-  const cudaError_t e = fast ? launch_nlsar_fast(F, d_scenes, F.total_tiles, st, variant, pl.full8)
-                             : launch_nlsar_fused(pl.full8, F, d_scenes, smem, F.total_tiles, st);
+  const cudaError_t e = launch();
   if (g_prof.on) {
     cudaEventRecord(b, st);
     g_prof.ev.push_back({a, b});
-    g_prof.launches += 1;
+    g_prof.launches += kernels;
   }
+  return e;
+}
+
+int launch_fused(const Plan& pl, const FilterParams& F, const SceneDesc* d_scenes, size_t smem, cudaStream_t st,
+                 int variant) {
+  const bool fast = pl.fast && fast_kernel_supported(F, pl.full8);
+  const cudaError_t e = profiled(st, 1, [&] {
+    return fast ? launch_nlsar_fast(F, d_scenes, F.total_tiles, st, variant, pl.full8)
+                : launch_nlsar_fused(pl.full8, F, d_scenes, smem, F.total_tiles, st);
+  });
   if (e != cudaSuccess) return cuda_error(e, "NL-SAR fused launch");
   return DCL_OK;
+}
+
+int launch_split_all(const Plan& pl, const FilterParams& F, const SplitLayout& lay, const SceneDesc* d_scenes,
+                     const SplitSeg* d_segs, uint32_t* vol, cudaStream_t st) {
+  const cudaError_t e = profiled(st, split_launches(lay), [&] {
+    cudaError_t r = cudaSuccess;
+    for (size_t i = 0; i < lay.chunks.size() && r == cudaSuccess; ++i)
+      r = launch_split(pl, F, lay, (int)i, d_scenes, d_segs, vol, st);
+    return r;
+  });
+  if (e != cudaSuccess) return cuda_error(e, "NL-SAR index and mean launches");
+  return DCL_OK;
+}
+
+int sm_count(int dev) {
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
+  return sms;
 }
 
 // ---------------------------------------------------------------------------
@@ -519,18 +549,42 @@ int run_device(const Plan& pl0, const std::vector<SceneIO>& io, cudaStream_t st)
     if (t + tiles > 0x7fffffff) return set_error(DCL_ERR_INVALID_ARGUMENT, "scene too large");
     tiles += (int)t;
   }
-  const size_t desc_bytes = io.size() * sizeof(SceneDesc);
-  const size_t wtab_bytes = pl.wtab.size() * sizeof(float);
+  // the two-kernel path where it serves the call; a smaller volume where the
+  // device has no room for the usual one, the fused kernel where it has none
+  SplitLayout lay;
+  std::vector<SplitJob> jobs;
+  for (size_t i = 0; i < io.size(); ++i) jobs.push_back({(int)i, 0, geo[i].vH + 1});
+  size_t budget = kSplitBudgetBytes / sizeof(uint32_t);
+  bool split = split_supported(pl.P, pl.full8) && split_layout(pl, geo, jobs, budget, sm_count(dev), lay);
+  const size_t desc_bytes = pad256(io.size() * sizeof(SceneDesc));
+  const size_t wtab_bytes = pad256(pl.wtab.size() * sizeof(float));
+  size_t seg_bytes = 0;
   char* scratch = nullptr;
-  cudaError_t e = cudaMallocAsync(&scratch, total + desc_bytes + wtab_bytes + 512, st);
+  cudaError_t e = cudaSuccess;
+  total = pad256(total);
+  for (;;) {
+    seg_bytes = split ? pad256(lay.segs.size() * sizeof(SplitSeg)) : 0;
+    const size_t vol = split ? lay.vol_words * sizeof(uint32_t) : 0;
+    e = cudaMallocAsync(&scratch, total + desc_bytes + wtab_bytes + seg_bytes + vol, st);
+    if (e != cudaErrorMemoryAllocation || !split) break;
+    cudaGetLastError();
+    budget /= 4;
+    split = budget >= kSplitMinBudgetBytes / sizeof(uint32_t) &&
+            split_layout(pl, geo, jobs, budget, sm_count(dev), lay);
+  }
   if (e != cudaSuccess) return cuda_error(e, "cudaMallocAsync(scratch)");
-  SceneDesc* d_desc = reinterpret_cast<SceneDesc*>(scratch + (total + 255) / 256 * 256);
-  float* d_wtab = reinterpret_cast<float*>(reinterpret_cast<char*>(d_desc) + (desc_bytes + 255) / 256 * 256);
+  SceneDesc* d_desc = reinterpret_cast<SceneDesc*>(scratch + total);
+  float* d_wtab = reinterpret_cast<float*>(scratch + total + desc_bytes);
+  SplitSeg* d_segs = reinterpret_cast<SplitSeg*>(scratch + total + desc_bytes + wtab_bytes);
+  uint32_t* d_vol = reinterpret_cast<uint32_t*>(scratch + total + desc_bytes + wtab_bytes + seg_bytes);
 
-  std::vector<SceneDesc> desc(io.size());
+  // descriptors, weight tables and segments go up in one copy
+  std::vector<char> up(desc_bytes + wtab_bytes + seg_bytes);
+  SceneDesc* desc = reinterpret_cast<SceneDesc*>(up.data());
+  std::memcpy(up.data() + desc_bytes, pl.wtab.data(), pl.wtab.size() * sizeof(float));
+  if (split) std::memcpy(up.data() + desc_bytes + wtab_bytes, lay.segs.data(), lay.segs.size() * sizeof(SplitSeg));
   int tb = 0;
   for (size_t i = 0; i < io.size(); ++i) {
-    std::memset(&desc[i], 0, sizeof(SceneDesc));
     rc = carve_scene(pl, geo[i], scratch + offs[i], desc[i]);
     if (rc) {
       cudaFreeAsync(scratch, st);
@@ -545,8 +599,7 @@ int run_device(const Plan& pl0, const std::vector<SceneIO>& io, cudaStream_t st)
     tb += geo[i].tiles_x * geo[i].tiles_y;
     launch_prep(pl, geo[i], desc[i], io[i].a1, io[i].a2, io[i].phi, io[i].cov_in, st);
   }
-  e = cudaMemcpyAsync(d_desc, desc.data(), desc_bytes, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d_wtab, pl.wtab.data(), wtab_bytes, cudaMemcpyHostToDevice, st);
+  e = cudaMemcpyAsync(d_desc, up.data(), up.size(), cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) {
     cudaFreeAsync(scratch, st);
     return cuda_error(e, "cudaMemcpyAsync(params)");
@@ -554,13 +607,13 @@ int run_device(const Plan& pl0, const std::vector<SceneIO>& io, cudaStream_t st)
   pl.P.wtab = d_wtab;
   pl.P.n_scenes = (int)io.size();
   pl.P.total_tiles = tiles;
-  rc = launch_fused(pl, pl.P, d_desc, smem, st);
+  rc = split ? launch_split_all(pl, pl.P, lay, d_desc, d_segs, d_vol, st) : launch_fused(pl, pl.P, d_desc, smem, st);
   e = cudaGetLastError();
   cudaFreeAsync(scratch, st);
   if (rc) return rc;
   if (e != cudaSuccess) return cuda_error(e, "NL-SAR launch");
-  // the host vectors above were staged by cudaMemcpyAsync (pageable source),
-  // so they may go out of scope now
+  // the host vector above was staged by cudaMemcpyAsync (pageable source), so
+  // it may go out of scope now
   return DCL_OK;
 }
 
@@ -591,8 +644,7 @@ constexpr int kBandWaves = 8;  // fewest waves of tiles (one CTA per SM) per ban
                                // ends in a partly filled wave, so small scenes stay in one band
 
 int band_count(int dev, long long tiles, int tile_rows) {
-  int sms = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
+  const int sms = sm_count(dev);
   int nb = (int)std::max(1LL, std::min<long long>(std::min(kMaxBands, tile_rows),
                                                   tiles / ((long long)kBandWaves * sms)));
   // DESPECKCL_B200_BANDS=n forces n bands (at most one per tile row): the
@@ -644,25 +696,57 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
 
   cudaStream_t st = cudaStreamPerThread;
   const size_t n = (size_t)H * W, b = n * sizeof(float);
-  const size_t scratch = (scratch_bytes(pl, g) + 255) / 256 * 256;
-  const size_t desc_bytes = (nb * sizeof(SceneDesc) + 255) / 256 * 256;
+  const size_t scratch = pad256(scratch_bytes(pl, g));
+  const size_t desc_bytes = pad256(nb * sizeof(SceneDesc));
   const size_t wtab_bytes = pl.wtab.size() * sizeof(float);
-  const size_t io_bytes = ((size_t)(nin + nout) * b + 255) / 256 * 256;
-  const size_t wtab_pad = (wtab_bytes + 255) / 256 * 256;
+  const size_t io_bytes = pad256((size_t)(nin + nout) * b);
+  const size_t wtab_pad = pad256(wtab_bytes);
+  // band b covers tile rows [tb[b], tb[b+1])
+  std::vector<int> tb(nb + 1);
+  for (int i = 0; i <= nb; ++i) tb[i] = (int)((long long)g.tiles_y * i / nb);
+  // the two-kernel path: every band's segments share one volume (the same
+  // fallbacks as run_device)
+  std::vector<SplitLayout> lay(nb);
+  std::vector<SplitSeg> segs;
+  std::vector<size_t> seg0(nb);
+  size_t vol_words = 0;
+  auto layouts = [&](size_t budget) {
+    segs.clear();
+    vol_words = 0;
+    for (int i = 0; i < nb; ++i) {
+      const SplitJob j{0, tb[i] * pl.P.tile_h, tb[i + 1] * pl.P.tile_h};
+      if (!split_layout(pl, {g}, {j}, budget, sm_count(dev), lay[i])) return false;
+      seg0[i] = segs.size();
+      segs.insert(segs.end(), lay[i].segs.begin(), lay[i].segs.end());
+      vol_words = std::max(vol_words, lay[i].vol_words);
+    }
+    return true;
+  };
+  size_t budget = kSplitBudgetBytes / sizeof(uint32_t);
+  bool split = split_supported(pl.P, pl.full8) && layouts(budget);
+  size_t seg_pad = 0;
   char* mem = nullptr;
-  // ... + one word: this call's count of thread blocks whose staging wait ran out
-  cudaError_t e = cudaMallocAsync(&mem, io_bytes + scratch + desc_bytes + wtab_pad + 256, st);
+  cudaError_t e = cudaSuccess;
+  for (;;) {
+    seg_pad = split ? pad256(segs.size() * sizeof(SplitSeg)) : 0;
+    const size_t vol = split ? vol_words * sizeof(uint32_t) : 0;
+    // ... + one word: this call's count of thread blocks whose staging wait ran out
+    e = cudaMallocAsync(&mem, io_bytes + scratch + desc_bytes + wtab_pad + 256 + seg_pad + vol, st);
+    if (e != cudaErrorMemoryAllocation || !split) break;
+    cudaGetLastError();
+    budget /= 4;
+    split = budget >= kSplitMinBudgetBytes / sizeof(uint32_t) && layouts(budget);
+  }
   if (e != cudaSuccess) return cuda_error(e, "cudaMallocAsync(io + scratch)");
   float* buf = reinterpret_cast<float*>(mem);  // [nin][H][W] inputs, then [nout][H][W] outputs
   float* dout = buf + (size_t)nin * n;
   SceneDesc* d_desc = reinterpret_cast<SceneDesc*>(mem + io_bytes + scratch);
   float* d_wtab = reinterpret_cast<float*>(mem + io_bytes + scratch + desc_bytes);
   int* d_timeouts = reinterpret_cast<int*>(mem + io_bytes + scratch + desc_bytes + wtab_pad);
+  SplitSeg* d_segs = reinterpret_cast<SplitSeg*>(mem + io_bytes + scratch + desc_bytes + wtab_pad + 256);
+  uint32_t* d_vol = reinterpret_cast<uint32_t*>(mem + io_bytes + scratch + desc_bytes + wtab_pad + 256 + seg_pad);
   *hp->h_timeouts = 0;
 
-  // band b covers tile rows [tb[b], tb[b+1])
-  std::vector<int> tb(nb + 1);
-  for (int i = 0; i <= nb; ++i) tb[i] = (int)((long long)g.tiles_y * i / nb);
   std::vector<SceneDesc> desc(nb);
   std::memset(desc.data(), 0, nb * sizeof(SceneDesc));
   rc = carve_scene(pl, g, mem + io_bytes, desc[0]);
@@ -681,6 +765,8 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
   if (rc == DCL_OK) {
     e = cudaMemcpyAsync(d_desc, desc.data(), nb * sizeof(SceneDesc), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_wtab, pl.wtab.data(), wtab_bytes, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && split)
+      e = cudaMemcpyAsync(d_segs, segs.data(), segs.size() * sizeof(SplitSeg), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_timeouts, 0, sizeof(int), st);
     if (e == cudaSuccess) e = cudaEventRecord(ev_alloc, st);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(hp->h2d, ev_alloc, 0);
@@ -720,7 +806,9 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
     cs_done = cs_need;
     FilterParams F = pl.P;
     F.total_tiles = (tb[i + 1] - tb[i]) * g.tiles_x;
-    if (F.total_tiles > 0) rc = launch_fused(pl, F, d_desc + i, smem, st);
+    if (F.total_tiles > 0)
+      rc = split ? launch_split_all(pl, F, lay[i], d_desc + i, d_segs + seg0[i], d_vol, st)
+                 : launch_fused(pl, F, d_desc + i, smem, st);
     e = cudaGetLastError();
     if (rc == DCL_OK && e != cudaSuccess) rc = cuda_error(e, "NL-SAR launch");
     if (rc == DCL_OK && (e = cudaEventRecord(ev_out[i], st)) != cudaSuccess) rc = cuda_error(e, "event");

@@ -1,0 +1,78 @@
+// Host interface of the two-kernel NL-SAR path (nlsar_split.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <cstdint>
+#include <vector>
+
+#include "nlsar_common.cuh"
+#include "nlsar_plan.h"
+
+namespace dcl {
+
+// Rows of a mean-kernel tile: InSAR input, 8-plane covariance input.
+constexpr int kSplitTileH = 16;
+constexpr int kSplitTileH8 = 24;
+// Volume of weight indices held at a time.
+constexpr size_t kSplitBudgetBytes = size_t(2) << 30;
+constexpr size_t kSplitMinBudgetBytes = size_t(32) << 20;  // below it the fused kernel filters
+constexpr size_t kSplitSmem = 227 * 1024;
+constexpr int kSplitShapes = 2;  // different pass shapes of one call
+
+// A run of virtual rows of one scene with its volume
+// [pass][half-window offset][rows][pitch] of 32-bit words.
+struct SplitSeg {
+  int scene;
+  int vy0, vy1;        // virtual rows filtered
+  int row0, rows;      // virtual row of the volume's first row (vy0 - wsh), row count
+  int pitch;           // words per row; volume column c is virtual column c - wsh
+  int tiles_x, tile_begin;                // mean kernel: tiles per row, first tile in the chunk
+  int idx_begin[kSplitShapes], idx_bx[kSplitShapes], idx_R[kSplitShapes];  // index kernel: blocks, columns, rows
+  size_t vol;          // first word
+};
+
+// Segments filtered together: one index launch per pass shape, one mean launch.
+struct SplitChunk {
+  int seg0, seg1, tiles;
+  int idx_blocks[kSplitShapes], idx_z[kSplitShapes];
+  size_t idx_smem[kSplitShapes];
+};
+
+// Passes of one shape.
+struct PassList {
+  int n;
+  int id[kMaxPasses];
+};
+
+// Virtual rows [row0, row1) of a scene, row0 on a tile row.
+struct SplitJob {
+  int scene, row0, row1;
+};
+
+struct SplitLayout {
+  std::vector<SplitSeg> segs;
+  std::vector<SplitChunk> chunks;
+  size_t vol_words;
+  int nshape, shape[kSplitShapes];
+  PassList passes[kSplitShapes];
+};
+
+// Whether the two-kernel path serves a call (the specialised kernel's shapes
+// in its default arithmetic).
+bool split_supported(const FilterParams& F, bool full8);
+bool split_layout(const Plan& pl, const std::vector<SceneGeom>& geo, const std::vector<SplitJob>& jobs,
+                  size_t budget_words, int sms, SplitLayout& out);
+// Kernels a layout launches.
+int split_launches(const SplitLayout& lay);
+// Launches chunk `chunk`: index kernels, then the mean kernel.
+cudaError_t launch_split(const Plan& pl, const FilterParams& F, const SplitLayout& lay, int chunk,
+                         const SceneDesc* d_scenes, const SplitSeg* d_segs, uint32_t* vol, cudaStream_t st);
+
+// All chunks of a layout (nlsar_host.cu), timed as one launch by the profile.
+int launch_split_all(const Plan& pl, const FilterParams& F, const SplitLayout& lay, const SceneDesc* d_scenes,
+                     const SplitSeg* d_segs, uint32_t* vol, cudaStream_t st);
+int sm_count(int dev);
+
+}  // namespace dcl
