@@ -37,7 +37,7 @@ struct dcl_nlsar_batch {
   bool split = false;  // two kernels around a volume of weight indices (nlsar_split.cu)
   dcl::SplitLayout lay;
   dcl::SplitSeg* d_segs = nullptr;
-  uint32_t* d_vol = nullptr;
+  char* d_vol = nullptr;
   int variant = 0;
   bool tuned = false;
   cudaStream_t cap = nullptr;
@@ -279,18 +279,18 @@ extern "C" dcl_nlsar_batch* dcl_nlsar_batch_create(int n, const float* const* a1
   cudaGetDevice(&dev);
   std::vector<SplitJob> jobs;
   for (int i = 0; i < n; ++i) jobs.push_back({i, 0, b->geo[i].vH + 1});
-  size_t budget = kSplitBudgetBytes / sizeof(uint32_t), seg_bytes = 0;
-  b->split = !(flags & (DCL_BATCH_VARIANT1 | DCL_BATCH_VARIANT2)) && split_supported(b->pl.P, false) &&
+  size_t budget = kSplitBudgetBytes, seg_bytes = 0;
+  b->split = !(flags & (DCL_BATCH_VARIANT1 | DCL_BATCH_VARIANT2)) && split_supported(b->pl) &&
              split_layout(b->pl, b->geo, jobs, budget, sm_count(dev), b->lay);
   cudaError_t e = cudaSuccess;
   for (;;) {
     seg_bytes = b->split ? (b->lay.segs.size() * sizeof(SplitSeg) + 255) / 256 * 256 : 0;
-    const size_t vol = b->split ? b->lay.vol_words * sizeof(uint32_t) : 0;
+    const size_t vol = b->split ? b->lay.vol_bytes : 0;
     e = cudaMalloc(&b->scratch, total + desc_bytes + wtab_pad + seg_bytes + vol);
     if (e != cudaErrorMemoryAllocation || !b->split) break;
     cudaGetLastError();
     budget /= 4;
-    b->split = budget >= kSplitMinBudgetBytes / sizeof(uint32_t) &&
+    b->split = budget >= kSplitMinBudgetBytes &&
                split_layout(b->pl, b->geo, jobs, budget, sm_count(dev), b->lay);
   }
   if (e != cudaSuccess) {
@@ -307,7 +307,7 @@ extern "C" dcl_nlsar_batch* dcl_nlsar_batch_create(int n, const float* const* a1
   e = cudaMemcpy(d_wtab, b->pl.wtab.data(), wtab_bytes, cudaMemcpyHostToDevice);
   if (b->split) {
     b->d_segs = reinterpret_cast<SplitSeg*>(b->scratch + total + desc_bytes + wtab_pad);
-    b->d_vol = reinterpret_cast<uint32_t*>(b->scratch + total + desc_bytes + wtab_pad + seg_bytes);
+    b->d_vol = b->scratch + total + desc_bytes + wtab_pad + seg_bytes;
     if (e == cudaSuccess)
       e = cudaMemcpy(b->d_segs, b->lay.segs.data(), b->lay.segs.size() * sizeof(SplitSeg), cudaMemcpyHostToDevice);
   }

@@ -498,7 +498,7 @@ int launch_fused(const Plan& pl, const FilterParams& F, const SceneDesc* d_scene
 }
 
 int launch_split_all(const Plan& pl, const FilterParams& F, const SplitLayout& lay, const SceneDesc* d_scenes,
-                     const SplitSeg* d_segs, uint32_t* vol, cudaStream_t st) {
+                     const SplitSeg* d_segs, char* vol, cudaStream_t st) {
   const cudaError_t e = profiled(st, split_launches(lay), [&] {
     cudaError_t r = cudaSuccess;
     for (size_t i = 0; i < lay.chunks.size() && r == cudaSuccess; ++i)
@@ -554,8 +554,8 @@ int run_device(const Plan& pl0, const std::vector<SceneIO>& io, cudaStream_t st)
   SplitLayout lay;
   std::vector<SplitJob> jobs;
   for (size_t i = 0; i < io.size(); ++i) jobs.push_back({(int)i, 0, geo[i].vH + 1});
-  size_t budget = kSplitBudgetBytes / sizeof(uint32_t);
-  bool split = split_supported(pl.P, pl.full8) && split_layout(pl, geo, jobs, budget, sm_count(dev), lay);
+  size_t budget = kSplitBudgetBytes;
+  bool split = split_supported(pl) && split_layout(pl, geo, jobs, budget, sm_count(dev), lay);
   const size_t desc_bytes = pad256(io.size() * sizeof(SceneDesc));
   const size_t wtab_bytes = pad256(pl.wtab.size() * sizeof(float));
   size_t seg_bytes = 0;
@@ -564,19 +564,19 @@ int run_device(const Plan& pl0, const std::vector<SceneIO>& io, cudaStream_t st)
   total = pad256(total);
   for (;;) {
     seg_bytes = split ? pad256(lay.segs.size() * sizeof(SplitSeg)) : 0;
-    const size_t vol = split ? lay.vol_words * sizeof(uint32_t) : 0;
+    const size_t vol = split ? lay.vol_bytes : 0;
     e = cudaMallocAsync(&scratch, total + desc_bytes + wtab_bytes + seg_bytes + vol, st);
     if (e != cudaErrorMemoryAllocation || !split) break;
     cudaGetLastError();
     budget /= 4;
-    split = budget >= kSplitMinBudgetBytes / sizeof(uint32_t) &&
+    split = budget >= kSplitMinBudgetBytes &&
             split_layout(pl, geo, jobs, budget, sm_count(dev), lay);
   }
   if (e != cudaSuccess) return cuda_error(e, "cudaMallocAsync(scratch)");
   SceneDesc* d_desc = reinterpret_cast<SceneDesc*>(scratch + total);
   float* d_wtab = reinterpret_cast<float*>(scratch + total + desc_bytes);
   SplitSeg* d_segs = reinterpret_cast<SplitSeg*>(scratch + total + desc_bytes + wtab_bytes);
-  uint32_t* d_vol = reinterpret_cast<uint32_t*>(scratch + total + desc_bytes + wtab_bytes + seg_bytes);
+  char* d_vol = scratch + total + desc_bytes + wtab_bytes + seg_bytes;
 
   // descriptors, weight tables and segments go up in one copy
   std::vector<char> up(desc_bytes + wtab_bytes + seg_bytes);
@@ -709,33 +709,33 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
   std::vector<SplitLayout> lay(nb);
   std::vector<SplitSeg> segs;
   std::vector<size_t> seg0(nb);
-  size_t vol_words = 0;
+  size_t vol_bytes = 0;
   auto layouts = [&](size_t budget) {
     segs.clear();
-    vol_words = 0;
+    vol_bytes = 0;
     for (int i = 0; i < nb; ++i) {
       const SplitJob j{0, tb[i] * pl.P.tile_h, tb[i + 1] * pl.P.tile_h};
       if (!split_layout(pl, {g}, {j}, budget, sm_count(dev), lay[i])) return false;
       seg0[i] = segs.size();
       segs.insert(segs.end(), lay[i].segs.begin(), lay[i].segs.end());
-      vol_words = std::max(vol_words, lay[i].vol_words);
+      vol_bytes = std::max(vol_bytes, lay[i].vol_bytes);
     }
     return true;
   };
-  size_t budget = kSplitBudgetBytes / sizeof(uint32_t);
-  bool split = split_supported(pl.P, pl.full8) && layouts(budget);
+  size_t budget = kSplitBudgetBytes;
+  bool split = split_supported(pl) && layouts(budget);
   size_t seg_pad = 0;
   char* mem = nullptr;
   cudaError_t e = cudaSuccess;
   for (;;) {
     seg_pad = split ? pad256(segs.size() * sizeof(SplitSeg)) : 0;
-    const size_t vol = split ? vol_words * sizeof(uint32_t) : 0;
+    const size_t vol = split ? vol_bytes : 0;
     // ... + one word: this call's count of thread blocks whose staging wait ran out
     e = cudaMallocAsync(&mem, io_bytes + scratch + desc_bytes + wtab_pad + 256 + seg_pad + vol, st);
     if (e != cudaErrorMemoryAllocation || !split) break;
     cudaGetLastError();
     budget /= 4;
-    split = budget >= kSplitMinBudgetBytes / sizeof(uint32_t) && layouts(budget);
+    split = budget >= kSplitMinBudgetBytes && layouts(budget);
   }
   if (e != cudaSuccess) return cuda_error(e, "cudaMallocAsync(io + scratch)");
   float* buf = reinterpret_cast<float*>(mem);  // [nin][H][W] inputs, then [nout][H][W] outputs
@@ -744,7 +744,7 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
   float* d_wtab = reinterpret_cast<float*>(mem + io_bytes + scratch + desc_bytes);
   int* d_timeouts = reinterpret_cast<int*>(mem + io_bytes + scratch + desc_bytes + wtab_pad);
   SplitSeg* d_segs = reinterpret_cast<SplitSeg*>(mem + io_bytes + scratch + desc_bytes + wtab_pad + 256);
-  uint32_t* d_vol = reinterpret_cast<uint32_t*>(mem + io_bytes + scratch + desc_bytes + wtab_pad + 256 + seg_pad);
+  char* d_vol = mem + io_bytes + scratch + desc_bytes + wtab_pad + 256 + seg_pad;
   *hp->h_timeouts = 0;
 
   std::vector<SceneDesc> desc(nb);

@@ -77,22 +77,31 @@ __device__ __forceinline__ float kahan_add(float s, float x, float& c) {
   return t;
 }
 
+// det(A + B), with every rounding explicit so that all kernels share it
+__device__ __forceinline__ float det_sum(const float4 a, const float4 b) {
+  const float2 d01 = __fadd2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y));
+  const float2 d23 = __fadd2_rn(make_float2(a.z, a.w), make_float2(b.z, b.w));
+  return __fmaf_rn(d01.x, d01.y, -__fmaf_rn(d23.x, d23.x, __fmul_rn(d23.y, d23.y)));
+}
+
+// The ratio form: log2 of det |det| / (16 det A det B); NaN (the log of a
+// negative number) when det < 0
+__device__ __forceinline__ float glr_ratio(const float4 a, float la, const float4 b, float lb) {
+  const float det = det_sum(a, b);
+  return lg2_ftz(__fmul_rn(__fmul_rn(det, fabsf(det)), __fmul_rn(la, lb)));
+}
+
 template <int PV>
 __device__ __forceinline__ float glr_sim(const float4 a, float la, const float4 b, float lb, float c2d) {
   // sim_measures.h:52-64 with nlooks 1 and the per-pixel terms precomputed;
   // NaN -> 0.  Each form is exactly symmetric in (A, B), which gives the
   // mirrored half window the reference's values (copy_symm_weights.cl:56-76).
-  const float2 d01 = __fadd2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y));
-  const float2 d23 = __fadd2_rn(make_float2(a.z, a.w), make_float2(b.z, b.w));
-  const float s00 = d01.x, s11 = d01.y, sre = d23.x, sim = d23.y;
-  // explicitly rounded: every kernel contracts it this way
-  const float det = __fmaf_rn(s00, s11, -__fmaf_rn(sre, sre, __fmul_rn(sim, sim)));
   float r;
   if (ratio_form<PV>()) {
-    // log2 of det |det| / (16 det A det B): negative (NaN log) when det < 0
-    r = lg2_ftz((det * fabsf(det)) * (la * lb));
+    r = glr_ratio(a, la, b, lb);
     if (PV == kPrecHalf) r = __half2float(__float2half_rn(r));
   } else {
+    const float det = det_sum(a, b);
     const float t = (la + lb) + c2d;
     r = (PV == kPrecLogf) ? 2.0f * logf(det) - t : fmaf(2.0f * 0.69314718f, __log2f(det), -t);
   }

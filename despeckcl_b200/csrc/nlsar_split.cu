@@ -32,6 +32,8 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "dcl_internal.h"
@@ -42,15 +44,25 @@ namespace dcl {
 
 namespace {
 
-// A weight's field in a word: 9 bits, the table entry or kZeroField.  Field j
-// sits at bits 6 + 9 j (the third wraps around), so that a masked word (the
-// second and third field after a shift or rotation) is the byte offset of the
-// entry in a table with 16 interleaved copies.
-constexpr int kZeroField = 256;
-constexpr int kLutCopies = 16;
-constexpr int kOneField = 257;  // the centre's weight
-constexpr int kLutWords = (kOneField + 1) * kLutCopies;  // one table
-constexpr uint32_t kFieldMask = 0x1FFu << 6;
+// A weight's code: one byte, its table entry, or kZeroCode for weight 0
+// (d > dmax).  Entry 255 is reached only where the scaled sum rounds to
+// exactly 1; it is coded as 254, so a call whose tables have 256 entries needs
+// entries 254 and 255 equal (split_supported).
+constexpr int kZeroCode = 255;
+
+// The codes of a pass of NP patch sizes at one (offset, pixel).
+template <int NP>
+struct WordOf {
+  using T = uint32_t;
+};
+template <>
+struct WordOf<1> {
+  using T = uint8_t;
+};
+template <>
+struct WordOf<2> {
+  using T = uint16_t;
+};
 
 constexpr int kIdxWarps = 16;
 constexpr int kIdxThreads = 32 * kIdxWarps;
@@ -93,8 +105,9 @@ template <int PH0, int PH1, int PH2>
 __global__ void __launch_bounds__(kIdxThreads, 1)
     nlsar_index_kernel(const __grid_constant__ FilterParams P, const SceneDesc* __restrict__ scenes,
                        const SplitSeg* __restrict__ segs, int nseg, const __grid_constant__ PassList passes,
-                       int shape, uint32_t* __restrict__ vol) {
+                       int shape, char* __restrict__ vol) {
   constexpr int NP = np_of<PH0, PH1, PH2>();
+  using Word = typename WordOf<NP>::T;
   constexpr int PHM = cmax(PH0, cmax(PH1, PH2));
   constexpr int HL = IdxL<PHM>::HL, VC = IdxL<PHM>::VC;
   constexpr int ND = PHM - PH0;  // rows the first patch's field waits
@@ -165,19 +178,23 @@ __global__ void __launch_bounds__(kIdxThreads, 1)
   const int c = VC * bx + 4 * (lane - HL);  // this lane's first volume column
   const bool writes = lane >= HL && lane < 32 - HL && c < S.pitch;
   const size_t plane = (size_t)S.rows * S.pitch;
-  uint32_t* out0 = vol + S.vol + (size_t)ps * nhalf * plane + (size_t)r0 * S.pitch + c;
+  Word* out0 = reinterpret_cast<Word*>(vol + S.vol + S.pass[ps]) + (ptrdiff_t)r0 * S.pitch + c;
 
   for (int u = (int)blockIdx.y * kIdxWarps + warp; u < nhalf; u += kIdxWarps * (int)gridDim.y) {
     // lower half window, row-major: (0, 1) .. (0, wsh), (1, -wsh) ..
     const int v = u + wsh + 1;
     const int dy = v / sws, dx = v - dy * sws - wsh;
+    // neighbour of column j: pixel t + j of the staged row, t = left + dx plus
+    // four per lane; M = t mod 4 fixes the slots of all four relative to the
+    // first's
+    const int t0 = left + dx;
+    Word* out = out0 + (size_t)u * plane;
     const float4* ctr = sC + 5 * (lane + (left >> 2));
-    int ns[4];  // slots of the four neighbours
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int t = left + dx + j;
-      ns[j] = dy * SP + 5 * (lane + (t >> 2)) + (t & 3);
-    }
+    const int n0 = dy * SP + 5 * (lane + (t0 >> 2)) + (t0 & 3);
+    auto walk = [&](auto m_tag) {
+    constexpr int M = decltype(m_tag)::value;
+    const float4* nbr = sC + n0;
+    const float* nld = sL + n0;
     // partial vertical sums: vs[j][k]: last k + 1 rows of patch j, columns in pairs
     float2 vs[NP][2 * PHM][2];
     uint32_t pend[ND > 0 ? ND : 1][4];
@@ -191,7 +208,6 @@ __global__ void __launch_bounds__(kIdxThreads, 1)
     for (int k = 0; k < ND; ++k)
 #pragma unroll
       for (int o = 0; o < 4; ++o) pend[k][o] = 0;
-    uint32_t* out = out0 + (size_t)u * plane;
     for (int i = 0; i < R + 2 * PHM; ++i) {
       // ---- similarities of the lane's four columns
       float s[4 + 2 * PHM];
@@ -199,11 +215,14 @@ __global__ void __launch_bounds__(kIdxThreads, 1)
         const float4 la = ctr[4];
         const float la4[4] = {la.x, la.y, la.z, la.w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) s[PHM + j] = glr_sim<kPrecRatio>(ctr[j], la4[j], sC[ns[j]], sL[ns[j]], 0.0f);
+        for (int j = 0; j < 4; ++j) {
+          const int n = j + (M + j >= 4 ? 1 : 0);
+          s[PHM + j] = glr_ratio(ctr[j], la4[j], nbr[n], nld[n]);
+        }
       }
       ctr += SP;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) ns[j] += SP;
+      nbr += SP;
+      nld += SP;
 #pragma unroll
       for (int k = 1; k <= PHM; ++k) {
         s[PHM - k] = __shfl_up_sync(0xffffffffu, s[PHM + 3 - (k - 1) % 4], (k + 3) / 4);
@@ -211,16 +230,27 @@ __global__ void __launch_bounds__(kIdxThreads, 1)
       }
       // ---- horizontal sums (nested rings)
       float hs[NP][4];
+      auto rings = [&] {
 #pragma unroll
-      for (int o = 0; o < 4; ++o) {
-        float ring = s[o + PHM];
+        for (int o = 0; o < 4; ++o) {
+          float ring = s[o + PHM];
 #pragma unroll
-        for (int b = 1; b <= PHM; ++b) {
-          ring += s[o + PHM - b] + s[o + PHM + b];
+          for (int b = 1; b <= PHM; ++b) {
+            ring += s[o + PHM - b] + s[o + PHM + b];
 #pragma unroll
-          for (int j = 0; j < NP; ++j)
-            if (ph_of<PH0, PH1, PH2>(j) == b) hs[j][o] = ring;
+            for (int j = 0; j < NP; ++j)
+              if (ph_of<PH0, PH1, PH2>(j) == b) hs[j][o] = ring;
+          }
         }
+      };
+      rings();
+      // a NaN similarity counts as 0; the largest rings of the first and last
+      // column hold every similarity, so one test finds any NaN
+      if (isnan(hs[NP - 1][0]) || isnan(hs[NP - 1][3])) {
+#pragma unroll
+        for (int k = 0; k < 4 + 2 * PHM; ++k)
+          if (isnan(s[k])) s[k] = 0.0f;
+        rings();
       }
       // ---- vertical sums, the weight's table index
       uint32_t field[NP][4];
@@ -234,39 +264,56 @@ __global__ void __launch_bounds__(kIdxThreads, 1)
 #pragma unroll
           for (int k = n - 1; k > 0; --k) vs[j][k][q] = __fadd2_rn(vs[j][k - 1][q], h);
           vs[j][0][q] = h;
+          // saturating FMA (clamps, NaN to 0), round-toward-zero add of 2^23:
+          // the low mantissa bits are the index; d > dmax: weight 0
+          const float2 u2 = make_float2(__saturatef(fmaf(d2.x, inv_span[j], nbias[j])),
+                                        __saturatef(fmaf(d2.y, inv_span[j], nbias[j])));
+          const float2 t2 = __ffma2_rz(u2, make_float2(lm1[j], lm1[j]), make_float2(8388608.0f, 8388608.0f));
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const float d = e ? d2.y : d2.x;
-            // saturating FMA (clamps, NaN to 0), round-toward-zero add of
-            // 2^23: the low mantissa bits are the index; d > dmax: weight 0
-            const float uu = __saturatef(fmaf(d, inv_span[j], nbias[j]));
-            const float t = __fmaf_rz(uu, lm1[j], 8388608.0f);
-            field[j][2 * q + e] = d > dmax[j] ? 0x4B000000u + kZeroField : __float_as_uint(t);
+            const uint32_t code = min(__float_as_uint(e ? t2.y : t2.x), 0x4B000000u + (kZeroCode - 1));
+            field[j][2 * q + e] = (e ? d2.y : d2.x) > dmax[j] ? (uint32_t)kZeroCode : code;  // the low byte counts
           }
         }
       }
-      // ---- the words of row i - 2 PHM; the exponent bits of field 0 are
-      // taken out, those of the others are shifted out
+      // ---- the words of row i - 2 PHM: byte j is the code of patch j
       uint32_t w[4];
 #pragma unroll
       for (int o = 0; o < 4; ++o) {
-        auto part = [&](int wait) {
-          uint32_t f = 0;
+        uint32_t next = 0;
+#pragma unroll
+        for (int k = ND; k >= 0; --k) {  // rows waited, the smallest patch first
+          uint32_t v = k < ND ? pend[k][o] : 0u;
 #pragma unroll
           for (int j = 0; j < NP; ++j)
-            if (PHM - ph_of<PH0, PH1, PH2>(j) == wait)
-              f += j == 0 ? field[0][o] - 0x4B000000u : field[j][o] << (9 * j);
-          return f;
-        };
-        w[o] = (ND > 0 ? pend[0][o] : 0u) + part(0);
-#pragma unroll
-        for (int k = 0; k < ND; ++k) pend[k][o] = (k + 1 < ND ? pend[k + 1][o] : 0u) + part(k + 1);
-        w[o] = __funnelshift_l(w[o], w[o], 6);
+            if (PHM - ph_of<PH0, PH1, PH2>(j) == k)
+              v = j == 0 ? field[0][o] : __byte_perm(v, field[j][o], j == 1 ? 0x0040 : 0x0410);
+          if (k < ND) pend[k][o] = next;
+          next = v;
+        }
+        w[o] = next;
       }
       if (i >= 2 * PHM) {
-        if (writes) *reinterpret_cast<uint4*>(out) = make_uint4(w[0], w[1], w[2], w[3]);
+        if (writes) {
+          if constexpr (NP == 3) {
+            *reinterpret_cast<uint4*>(out) = make_uint4(w[0], w[1], w[2], w[3]);
+          } else if constexpr (NP == 2) {
+            *reinterpret_cast<uint2*>(out) =
+                make_uint2(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410));
+          } else {
+            *reinterpret_cast<uint32_t*>(out) =
+                __byte_perm(__byte_perm(w[0], w[1], 0x0040), __byte_perm(w[2], w[3], 0x0040), 0x5410);
+          }
+        }
         out += S.pitch;
       }
+    }
+    };
+    switch (t0 & 3) {
+      case 0: walk(std::integral_constant<int, 0>{}); break;
+      case 1: walk(std::integral_constant<int, 1>{}); break;
+      case 2: walk(std::integral_constant<int, 2>{}); break;
+      default: walk(std::integral_constant<int, 3>{});
     }
   }
 }
@@ -275,242 +322,234 @@ __global__ void __launch_bounds__(kIdxThreads, 1)
 // mean kernel
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                   static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// Tile rows, threads and shared memory: 32 x TH outputs, two vertically
-// adjacent pixels per thread (their accumulators packed in pairs).  InSAR
-// input: 16 rows, 8 warps, two blocks per SM; 8-plane input: 24 rows, 12
-// warps, one block per SM (12 accumulators per pixel and patch size).
-template <bool FULL8>
+// One block: a 32 x TH tile of outputs, one pixel per thread, one row per
+// warp.  Of the accumulators that share a weight, six (ten with 8-plane input)
+// are updated two per packed (f32x2) FMA.  Bound by issue slots (about 35 per
+// pixel, offset and scale) and FMA cycles (packed FMAs take two) in about
+// equal parts; measured and slower at 4096^2 (40.7 ms): two pixels per thread
+// in 16 warps (42.4), two scales per sweep with patch sizes packed in pairs
+// (42.9), the words through a TMA ring (48.5: one thread's issue sets the
+// pace).
+//
+// Weight tables: one copy per lane, so the gathers have no bank conflicts.
+// Tables 0 and 1 interleave in 256-byte entries and table 2 has them to
+// itself, so one byte permute of the word and 4 lane gives an entry's byte
+// offset.
+template <int WSH_, int TH_, bool FULL8_, int NPX_>
 struct MeanL {
-  static constexpr int TH = FULL8 ? kSplitTileH8 : kSplitTileH, PX = 2;
-  static constexpr int WARPS = TH / PX, THREADS = 32 * WARPS;
-  static constexpr int BLOCKS = FULL8 ? 1 : 2;
+  static constexpr int WSH = WSH_, TH = TH_, NPX = NPX_;  // NPX: patch sizes of the largest pass
+  static constexpr bool FULL8 = FULL8_;
+  static constexpr int WARPS = TH, THREADS = 32 * WARPS;
   static constexpr int NA = FULL8 ? 12 : 8, NM = FULL8 ? 8 : 4;
+  static constexpr int SWS = 2 * WSH + 1;
+  // window columns per run, the words in flight ahead: 32 warps hide their
+  // latency with 7, fewer warps want a whole window row (1024^2 in 16-row
+  // tiles: 2.86 ms with 7, 2.68 with 21)
+  static constexpr int K = TH > 16 ? 7 : 21;
+  static constexpr int RUNS = SWS * SWS / K, MID = RUNS / 2, ROWRUNS = SWS / K;
+  static constexpr int RO = 32 + 2 * WSH, ROH = TH + 2 * WSH;  // staged covariance
+  static constexpr int PLANE = RO * ROH;                        // float4 per staged plane
+  static constexpr int NPL = FULL8 ? 2 : 1;
+  static constexpr int OFF_CO = (NPX + 1) / 2 * 256 * 256;      // bytes, after the tables
+  static constexpr int OFF_ONE = OFF_CO + NPL * PLANE * 16;
+  static constexpr int BYTES = OFF_ONE + 16;
+  static_assert(SWS % K == 0 && K > WSH % K, "runs tile a window row");
+  static_assert(ROWRUNS % 2 == 1 && K % 2 == 1, "the centre is the middle of the middle run");
+  static_assert(BYTES <= 227 * 1024, "shared memory");
 };
 
-__host__ __device__ inline int mean_region(int wsh, int th) { return (32 + 2 * wsh) * (th + 2 * wsh); }
-// float4 planes, then the weight tables, then one {volume, tile} offset pair
-// per search-window position
-__host__ __device__ inline size_t mean_smem(int wsh, int np, bool full8, int n_off) {
-  const int th = full8 ? kSplitTileH8 : kSplitTileH;
-  return (size_t)mean_region(wsh, th) * 16 * (full8 ? 2 : 1) + (size_t)np * kLutWords * 4 + (size_t)n_off * 8;
-}
-
-// One pass of NP patch sizes over the window: `words` points at the thread's
-// first pixel in the pass's volume.
-template <int NP, bool FULL8>
-__device__ __forceinline__ void mean_pass(const FilterParams& P, const PassParams& pp, const uint32_t* words,
-                                          int wpitch, const float4* sCo, const float4* sCo2, float* sLut,
-                                          const int2* sOff, int RO, int ci,
-                                          Best<MeanL<FULL8>::PX, MeanL<FULL8>::NM>& best) {
-  using L = MeanL<FULL8>;
-  constexpr int PX = L::PX, NA = L::NA;
-  const int tid = threadIdx.x, lane = tid & 31;
+// One pass of NP patch sizes over the window.  lane_off: the word of the
+// thread's pixel in a plane of the volume.
+template <class L, int NP>
+__device__ __forceinline__ void mean_pass(const FilterParams& P, int ps, const char* __restrict__ vol,
+                                          const SplitSeg& G, uint32_t lane_off, Best<1, L::NM>& best) {
+  using Word = typename WordOf<NP>::T;
+  constexpr int NA = L::NA, K = L::K, SWS = L::SWS, WSH = L::WSH, RO = L::RO;
+  static_assert(NP <= L::NPX, "tables");
+  extern __shared__ float4 smem4[];
+  char* sm = reinterpret_cast<char*>(smem4);
+  const PassParams& pp = P.pass[ps];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   __syncthreads();  // the previous pass's tables are no longer read
-  for (int i = tid; i < NP * kLutWords; i += L::THREADS) {
-    const int j = i / kLutWords;
-    const int e = (i - j * kLutWords) / kLutCopies;
-    sLut[i] = e < kMaxLut ? P.wtab[pp.combo[j] * kMaxLut + e] : (e == kOneField ? 1.0f : 0.0f);
+  for (int i = tid; i < NP * 256 * 8; i += L::THREADS) {
+    const int m = i >> 11, e = (i >> 3) & 255;
+    const float w = e == kZeroCode ? 0.0f : P.wtab[pp.combo[m] * kMaxLut + e];
+    *reinterpret_cast<float4*>(sm + (m >> 1) * 65536 + e * 256 + (m & 1) * 128 + (i & 7) * 16) =
+        make_float4(w, w, w, w);
   }
   __syncthreads();
-  float2 acc[NP][NA];  // .x: the upper pixel, .y: the lower one
+  float sw[NP], sww[NP];        // sum w, sum w^2
+  float2 acc[NP][NA / 2 - 1];  // sums of w (I0, I1), w (I0^2, I1^2), w C01, 8-plane input's other four
 #pragma unroll
-  for (int j = 0; j < NP; ++j)
+  for (int j = 0; j < NP; ++j) {
+    sw[j] = sww[j] = 0.0f;
 #pragma unroll
-    for (int a = 0; a < NA; ++a) acc[j][a] = make_float2(0.f, 0.f);
-  const uint32_t copy = 4u * (lane & (kLutCopies - 1));
-  const char* lut = reinterpret_cast<const char*>(sLut);
-
-  // two pixels per packed (f32x2) operation; each component is rounded like
-  // the scalar add / multiply / fma
-  auto accumulate = [&](const float2 (&ww)[NP], int oa) {
-    const float4 va = sCo[oa], vb = sCo[oa + RO];
-    const float2 vx = make_float2(va.x, vb.x), vy = make_float2(va.y, vb.y);
-    const float2 vz = make_float2(va.z, vb.z), vw = make_float2(va.w, vb.w);
-    const float2 x2 = __fmul2_rn(vx, vx), y2 = __fmul2_rn(vy, vy);
-    float2 ex[4];
-    if (FULL8) {
-      const float4 ea = sCo2[oa], eb = sCo2[oa + RO];
-      ex[0] = make_float2(ea.x, eb.x);
-      ex[1] = make_float2(ea.y, eb.y);
-      ex[2] = make_float2(ea.z, eb.z);
-      ex[3] = make_float2(ea.w, eb.w);
-    }
-#pragma unroll
-    for (int j = 0; j < NP; ++j) {
-      float2* A = acc[j];
-      A[0] = __fadd2_rn(A[0], ww[j]);
-      A[1] = __ffma2_rn(ww[j], ww[j], A[1]);
-      A[2] = __ffma2_rn(ww[j], vx, A[2]);
-      A[3] = __ffma2_rn(ww[j], vy, A[3]);
-      A[4] = __ffma2_rn(ww[j], x2, A[4]);
-      A[5] = __ffma2_rn(ww[j], y2, A[5]);
-      A[6] = __ffma2_rn(ww[j], vz, A[6]);
-      A[7] = __ffma2_rn(ww[j], vw, A[7]);
-      if (FULL8) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) A[(8 + e) % NA] = __ffma2_rn(ww[j], ex[e], A[(8 + e) % NA]);
-      }
-    }
-  };
+    for (int a = 0; a < NA / 2 - 1; ++a) acc[j][a] = make_float2(0.f, 0.f);
+  }
+  const uint32_t lane4 = 4u * lane;
   auto weight = [&](uint32_t w, int j) {
-    const uint32_t f = j == 0 ? w : (j == 1 ? w >> 9 : __funnelshift_r(w, w, 18));
-    return *reinterpret_cast<const float*>(lut + j * kLutWords * 4 + ((f & kFieldMask) | copy));
+    return *reinterpret_cast<const float*>(sm + (j >> 1) * 65536 + (j & 1) * 128 +
+                                           __byte_perm(w, lane4, 0x5504 | (j << 4)));
   };
-
-  // words of the next D offsets in flight while D are accumulated (their
-  // latency is that of HBM; n_off is a multiple of 8)
-  constexpr int D = 4;
-  const int n = P.n_off;
-  uint32_t nxt[D][PX];
-#pragma unroll
-  for (int k = 0; k < D; ++k) {
-    const uint32_t* p = words + sOff[k].x;
-    nxt[k][0] = __ldcg(p);
-    nxt[k][1] = __ldcg(p + wpitch);
-  }
-  for (int t = 0; t < n; t += D) {
-    uint32_t cur[D][PX];
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-      cur[k][0] = nxt[k][0];
-      cur[k][1] = nxt[k][1];
+  // each component of a packed operation is rounded like the scalar add /
+  // multiply / fma
+  auto accumulate = [&](const float (&w)[NP], const float4* v) {
+    const float4 a = v[0];
+    const float2 i01 = make_float2(a.x, a.y), c01 = make_float2(a.z, a.w);
+    const float2 sq = __fmul2_rn(i01, i01);
+    float2 ex[2];
+    if constexpr (L::FULL8) {
+      const float4 e = v[L::PLANE];
+      ex[0] = make_float2(e.x, e.y);
+      ex[1] = make_float2(e.z, e.w);
     }
-    if (t + D < n) {
-#pragma unroll
-      for (int k = 0; k < D; ++k) {
-        const uint32_t* p = words + sOff[t + D + k].x;
-        nxt[k][0] = __ldcg(p);
-        nxt[k][1] = __ldcg(p + wpitch);
-      }
-    }
-    if (2 * t == n) {  // the centre, between the two halves (routines.cpp:151-157)
-      // weight 1 from the table: with the constant the compiler folds w I^2 + A
-      // into one fused multiply-add of I, rounded once instead of twice
-      float2 ww[NP];
-#pragma unroll
-      for (int j = 0; j < NP; ++j) {
-        const float one = sLut[j * kLutWords + kOneField * kLutCopies];
-        ww[j] = make_float2(one, one);
-      }
-      accumulate(ww, ci);
-    }
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-      float2 ww[NP];
-#pragma unroll
-      for (int j = 0; j < NP; ++j) ww[j] = make_float2(weight(cur[k][0], j), weight(cur[k][1], j));
-      accumulate(ww, ci + sOff[t + k].y);
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < PX; ++i)
 #pragma unroll
     for (int j = 0; j < NP; ++j) {
-      float A[NA];
-#pragma unroll
-      for (int a = 0; a < NA; ++a) A[a] = (i & 1) ? acc[j][a].y : acc[j][a].x;
-      select_combo(P, pp.combo[j], A, i, best);
+      const float2 ww = make_float2(w[j], w[j]);
+      sw[j] = __fadd_rn(sw[j], w[j]);
+      sww[j] = __fmaf_rn(w[j], w[j], sww[j]);
+      acc[j][0] = __ffma2_rn(ww, i01, acc[j][0]);
+      acc[j][1] = __ffma2_rn(ww, sq, acc[j][1]);
+      acc[j][2] = __ffma2_rn(ww, c01, acc[j][2]);
+      if constexpr (L::FULL8) {
+        acc[j][3] = __ffma2_rn(ww, ex[0], acc[j][3]);
+        acc[j][4] = __ffma2_rn(ww, ex[1], acc[j][4]);
+      }
     }
+  };
+
+  // Words: offset q = (dy, dx), linear index l = dy SWS + dx: lower half
+  // (l > 0) word l - 1 of the pixel, upper half word -l - 1 of the pixel at q.
+  // So the word's place moves by `step` per offset: in the upper half back one
+  // plane and on one column (at a row's end on to the next row's first), in
+  // the lower half on one plane.  The words of the next run are in flight
+  // while one is accumulated; word k is refilled as soon as it is used.
+  const uint32_t plane = (uint32_t)G.rows * G.pitch;
+  const Word* words = reinterpret_cast<const Word*>(vol + G.vol + G.pass[ps]);
+  uint32_t off = lane_off + (uint32_t)(P.n_off / 2 - 1) * plane - (uint32_t)WSH * G.pitch - (uint32_t)WSH;
+  uint32_t step = 1u - plane;
+  const uint32_t row_step = (uint32_t)G.pitch - SWS;
+  uint32_t buf[K];
+  auto load = [&](int k) {
+    buf[k] = __ldcg(words + off);
+    off += step;
+  };
+#pragma unroll
+  for (int k = 0; k < K; ++k) load(k);
+  if (L::ROWRUNS == 1) off += row_step;
+  const float4* v = reinterpret_cast<const float4*>(sm + L::OFF_CO) + warp * RO + lane;
+  int rr = 1 % L::ROWRUNS;  // place of the next run in its window row
+  for (int run = 0; run < L::RUNS; ++run) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      float w[NP];
+      if (k == K / 2 && run == L::MID) {
+        // the centre: weight 1 (routines.cpp:151-157), read from memory: with
+        // the constant the compiler folds w I^2 + A into one fused
+        // multiply-add of I, rounded once instead of twice
+        const float one = *reinterpret_cast<const float*>(sm + L::OFF_ONE);
+#pragma unroll
+        for (int j = 0; j < NP; ++j) w[j] = one;
+      } else {
+#pragma unroll
+        for (int j = 0; j < NP; ++j) w[j] = weight(buf[k], j);
+      }
+      if (k == K / 2 && run + 1 == L::MID) {
+        // the next run's centre has no word; its lower half starts at word 0
+        off = lane_off;
+        step = plane;
+      } else if (run + 1 < L::RUNS) {
+        load(k);
+      }
+      accumulate(w, v + k);
+    }
+    v += K;
+    if (rr == 0) v += RO - SWS;  // this run was its row's last
+    if (++rr == L::ROWRUNS) {
+      rr = 0;
+      // the run after the next starts a row
+      if (run + 1 < L::MID) off += row_step;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < NP; ++j) {
+    float A[NA] = {sw[j], sww[j]};
+#pragma unroll
+    for (int a = 0; a < NA / 2 - 1; ++a) {
+      A[2 + 2 * a] = acc[j][a].x;
+      A[3 + 2 * a] = acc[j][a].y;
+    }
+    select_combo(P, pp.combo[j], A, 0, best);
+  }
 }
 
-// One block: one 32 x TH tile of a segment, all passes.
-template <int NPX, bool FULL8>
-__global__ void __launch_bounds__(MeanL<FULL8>::THREADS, MeanL<FULL8>::BLOCKS)
+template <class L>
+__global__ void __launch_bounds__(L::THREADS, 1)
     nlsar_mean_kernel(const __grid_constant__ FilterParams P, const SceneDesc* __restrict__ scenes,
-                      const SplitSeg* __restrict__ segs, int nseg, const uint32_t* __restrict__ vol) {
-  using L = MeanL<FULL8>;
-  constexpr int PX = L::PX, NM = L::NM;
+                      const SplitSeg* __restrict__ segs, int nseg, const char* __restrict__ vol) {
+  constexpr int WSH = L::WSH, RO = L::RO, NM = L::NM;
   extern __shared__ float4 smem4[];
+  char* sm = reinterpret_cast<char*>(smem4);
+  float4* sCo = reinterpret_cast<float4*>(sm + L::OFF_CO);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int lo = 0, hi = nseg - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (segs[mid].tile_begin <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
   }
-  const SplitSeg G = segs[lo];
+  const SplitSeg& G = segs[lo];
   const SceneDesc& S = scenes[G.scene];
   const int lt = (int)blockIdx.x - G.tile_begin;
   const int ty = lt / G.tiles_x, tx = lt - ty * G.tiles_x;
   const int vy0 = G.vy0 + ty * L::TH, vx0 = tx * kTileW;
-  const int wsh = P.wsh, sws = P.sws, RO = kTileW + 2 * wsh, ROH = L::TH + 2 * wsh;
-  float4* sCo = smem4;
-  float4* sCo2 = sCo + RO * ROH;  // 8-plane input only
-  float* sLut = reinterpret_cast<float*>(sCo + (FULL8 ? 2 : 1) * RO * ROH);
-  int2* sOff = reinterpret_cast<int2*>(sLut + NPX * kLutWords);
 
-  // the original covariance of the tile and the window's halo; frame rows end
-  // at tiles of P.tile_h rows, so the last rows are clamped (outputs that
-  // exist never use a clamped one)
+  // frame rows end at tiles of P.tile_h rows, so the last rows are clamped
+  // (outputs that exist never use a clamped one)
   {
     const int Hp = S.tiles_y * P.tile_h + 2 * P.G;
-    for (int r = warp; r < ROH; r += L::WARPS) {
-      const size_t row = (size_t)min(vy0 - wsh + P.G + r, Hp - 1) * S.pitch + (vx0 - wsh + P.G);
-      for (int c = lane; c < RO; c += 32) {
-        cp_async16(sCo + r * RO + c, S.cori + row + c);
-        if (FULL8) cp_async16(sCo2 + r * RO + c, S.cori2 + row + c);
+    for (int r = warp; r < L::ROH; r += L::WARPS) {
+      const size_t row = (size_t)min(vy0 - WSH + P.G + r, Hp - 1) * S.pitch + (vx0 - WSH + P.G);
+#pragma unroll
+      for (int q = 0; q < (RO + 31) / 32; ++q) {
+        const int c = lane + 32 * q;
+        if (c < RO) {
+          sCo[r * RO + c] = S.cori[row + c];
+          if constexpr (L::FULL8) sCo[L::PLANE + r * RO + c] = S.cori2[row + c];
+        }
       }
     }
+    if (tid == 0) *reinterpret_cast<float*>(sm + L::OFF_ONE) = 1.0f;
   }
-  // offset t of the window without its centre: the word's place relative to
-  // the pixel's in the volume of a pass, and the neighbour's in the tile
-  const int nhalf = P.n_off / 2;
-  const int plane = G.rows * G.pitch;
-  for (int t = tid; t < P.n_off; t += L::THREADS) {
-    const int v = t < nhalf ? t : t + 1;
-    const int dy = v / sws - wsh, dx = v - (v / sws) * sws - wsh;
-    sOff[t] = make_int2(t < nhalf ? (nhalf - 1 - t) * plane + dy * G.pitch + dx : (t - nhalf) * plane, dy * RO + dx);
-  }
-  cp_async_wait_all();
-  __syncthreads();
 
-  const int y0 = warp * PX;
-  const int ci = (y0 + wsh) * RO + lane + wsh;
   // pixels past the last virtual row and column repeat it: their words exist
-  const int wy = min(vy0 + y0, S.vH) - G.row0, wx = min(vx0 + lane, S.vW) + wsh;
-  const int wpitch = vy0 + y0 < S.vH ? G.pitch : 0;
-  const uint32_t* words = vol + G.vol + (size_t)wy * G.pitch + wx;
+  const uint32_t lane_off = (uint32_t)(min(vy0 + warp, G.vy1 - 1) - G.row0) * G.pitch + min(vx0 + lane, S.vW) + WSH;
 
-  Best<PX, NM> best;
+  Best<1, NM> best;
+  best.e[0] = -1.0f;
+  best.rank[0] = 0x7fffffff;
+  best.combo[0] = -1;
+  best.a[0] = 0.f;
+  best.s0[0] = 1.f;
 #pragma unroll
-  for (int i = 0; i < PX; ++i) {
-    best.e[i] = -1.0f;
-    best.rank[i] = 0x7fffffff;
-    best.combo[i] = -1;
-    best.a[i] = 0.f;
-    best.s0[i] = 1.f;
-#pragma unroll
-    for (int d = 0; d < NM; ++d) best.m[i][d] = 0.f;
-  }
+  for (int d = 0; d < NM; ++d) best.m[0][d] = 0.f;
   for (int ps = 0; ps < P.npass; ++ps) {
-    const PassParams& pp = P.pass[ps];
-    const uint32_t* w = words + (size_t)ps * nhalf * plane;
-    if (NPX == 1 || pp.np == 1) {
-      mean_pass<1, FULL8>(P, pp, w, wpitch, sCo, sCo2, sLut, sOff, RO, ci, best);
-    } else if (pp.np == 2) {
-      if constexpr (NPX >= 2) mean_pass<2, FULL8>(P, pp, w, wpitch, sCo, sCo2, sLut, sOff, RO, ci, best);
+    // passes of one patch size come alone, others as three or two
+    if constexpr (L::NPX == 1) {
+      mean_pass<L, 1>(P, ps, vol, G, lane_off, best);
+    } else if (P.pass[ps].np == 2) {
+      mean_pass<L, 2>(P, ps, vol, G, lane_off, best);
     } else {
-      if constexpr (NPX >= 3) mean_pass<3, FULL8>(P, pp, w, wpitch, sCo, sCo2, sLut, sOff, RO, ci, best);
+      mean_pass<L, 3>(P, ps, vol, G, lane_off, best);
     }
   }
-#pragma unroll
-  for (int i = 0; i < PX; ++i) {
-    const int vy = vy0 + y0 + i, vx = vx0 + lane;
-    const int oy = (vy < S.H - 1) ? vy : (vy == S.vH ? S.H - 1 : -1);
-    const int ox = (vx < S.W - 1) ? vx : (vx == S.vW ? S.W - 1 : -1);
-    if (oy < 0 || ox < 0 || vy >= G.vy1) continue;
-    const int o = ci + i * RO;
-    float4 c2 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (FULL8) c2 = sCo2[o];
-    write_pixel<FULL8>(S, (size_t)oy * S.W + ox, sCo[o], c2, i, best);
-  }
+  const int vy = vy0 + warp, vx = vx0 + lane;
+  const int oy = (vy < S.H - 1) ? vy : (vy == S.vH ? S.H - 1 : -1);
+  const int ox = (vx < S.W - 1) ? vx : (vx == S.vW ? S.W - 1 : -1);
+  if (oy < 0 || ox < 0 || vy >= G.vy1) return;
+  const int c = (warp + WSH) * RO + lane + WSH;
+  float4 c2 = make_float4(0.f, 0.f, 0.f, 0.f);
+  if constexpr (L::FULL8) c2 = sCo[L::PLANE + c];
+  write_pixel<L::FULL8>(S, (size_t)oy * S.W + ox, sCo[c], c2, 0, best);
 }
 
 // ---------------------------------------------------------------------------
@@ -530,7 +569,7 @@ int shape_vc(int shape) { return 128 - 8 * ((shape_phm(shape) + 3) / 4); }
 
 template <int PH0, int PH1, int PH2>
 cudaError_t launch_index_t(const FilterParams& F, const SceneDesc* scenes, const SplitSeg* segs, int nseg,
-                           const PassList& passes, int slot, uint32_t* vol, dim3 grid, size_t smem,
+                           const PassList& passes, int slot, char* vol, dim3 grid, size_t smem,
                            cudaStream_t st) {
   static size_t allowed[kMaxDevices];
   const cudaError_t e = allow_dynamic_smem((const void*)nlsar_index_kernel<PH0, PH1, PH2>, smem, allowed);
@@ -539,37 +578,65 @@ cudaError_t launch_index_t(const FilterParams& F, const SceneDesc* scenes, const
   return cudaGetLastError();
 }
 
-template <int NPX, bool FULL8>
+template <int TH, bool FULL8, int NPX>
 cudaError_t launch_mean_t(const FilterParams& F, const SceneDesc* scenes, const SplitSeg* segs, int nseg,
-                          const uint32_t* vol, int tiles, cudaStream_t st) {
+                          const char* vol, int tiles, cudaStream_t st) {
+  using L = MeanL<10, TH, FULL8, NPX>;
   static size_t allowed[kMaxDevices];
-  const size_t smem = mean_smem(F.wsh, NPX, FULL8, F.n_off);
-  const cudaError_t e = allow_dynamic_smem((const void*)nlsar_mean_kernel<NPX, FULL8>, smem, allowed);
+  const cudaError_t e = allow_dynamic_smem((const void*)nlsar_mean_kernel<L>, L::BYTES, allowed);
   if (e != cudaSuccess) return e;
-  nlsar_mean_kernel<NPX, FULL8><<<tiles, MeanL<FULL8>::THREADS, smem, st>>>(F, scenes, segs, nseg, vol);
+  nlsar_mean_kernel<L><<<tiles, L::THREADS, L::BYTES, st>>>(F, scenes, segs, nseg, vol);
   return cudaGetLastError();
 }
+
+// Rows of the tallest mean tile: 32, with 8-plane input 16 (its accumulators
+// want more registers; 24 rows measured 4.39 ms against 4.17 at 1100 x 1203)
+constexpr int tall_tile(bool full8) { return full8 ? 16 : 32; }
+
+template <bool FULL8, int NPX>
+cudaError_t launch_mean_th(int th, const FilterParams& F, const SceneDesc* scenes, const SplitSeg* segs, int nseg,
+                           const char* vol, int tiles, cudaStream_t st) {
+  if (th == 8) return launch_mean_t<8, FULL8, NPX>(F, scenes, segs, nseg, vol, tiles, st);
+  if (th == 16) return launch_mean_t<16, FULL8, NPX>(F, scenes, segs, nseg, vol, tiles, st);
+  return launch_mean_t<tall_tile(FULL8), FULL8, NPX>(F, scenes, segs, nseg, vol, tiles, st);
+}
+
+bool single_patches(const FilterParams& F) {
+  for (int i = 0; i < F.npass; ++i)
+    if (F.pass[i].np > 1) return false;
+  return true;
+}
+
+size_t word_bytes(int np) { return np == 3 ? 4 : np; }
 
 int div_up(int a, int b) { return (a + b - 1) / b; }
 
 }  // namespace
 
-bool split_supported(const FilterParams& F, bool full8) {
-  return F.prec == 0 && !F.withhold_staging && fast_kernel_supported(F, full8);
+bool split_supported(const Plan& pl) {
+  const FilterParams& F = pl.P;
+  if (F.prec != 0 || F.withhold_staging || !pl.fast) return false;
+  for (int i = 0; i < F.npass; ++i)
+    for (int j = 0; j < F.pass[i].np; ++j) {
+      const int c = F.pass[i].combo[j];
+      const float* w = pl.wtab.data() + (size_t)c * kMaxLut;
+      if (F.combo[c].lm1 > 254.0f && std::memcmp(w + 254, w + 255, sizeof(float)) != 0) return false;
+    }
+  return true;
 }
 
 // Cuts the jobs (row ranges of scenes) into segments of at most `budget`
-// words of volume, groups the segments into chunks of at most that size, and
+// bytes of volume, groups the segments into chunks of at most that size, and
 // chooses every chunk's block rows and offset groups.  False where the scene
 // is too wide for one tile row's volume.
 bool split_layout(const Plan& pl, const std::vector<SceneGeom>& geo, const std::vector<SplitJob>& jobs,
                   size_t budget, int sms, SplitLayout& out) {
   const FilterParams& F = pl.P;
-  const int th = pl.full8 ? kSplitTileH8 : kSplitTileH;
+  const int big = tall_tile(pl.full8);  // segments hold whole tiles
   const int nhalf = F.n_off / 2;
   out.segs.clear();
   out.chunks.clear();
-  out.vol_words = 0;
+  out.vol_bytes = 0;
   // the call's pass shapes, in order of first use
   out.nshape = 0;
   for (int i = 0; i < F.npass; ++i) {
@@ -592,11 +659,13 @@ bool split_layout(const Plan& pl, const std::vector<SceneGeom>& geo, const std::
     const int row1 = std::min(j.row1, g.vH + 1);
     if (j.row0 >= row1) continue;
     const int pitch = (g.vW + 1 + 2 * F.wsh + 3) / 4 * 4;
-    const size_t row_words = (size_t)F.npass * nhalf * pitch;
-    const long long fit = (long long)(budget / row_words) - F.wsh;
-    const int most = std::max(th, (int)std::min<long long>(fit, 1 << 20) / th * th);
+    // bytes of one row of one half-window offset, all passes
+    size_t row = 0;
+    for (int p = 0; p < F.npass; ++p) row += (size_t)pitch * word_bytes(F.pass[p].np);
+    const long long fit = (long long)(budget / (row * nhalf)) - F.wsh;
+    const int most = std::max(big, (int)std::min<long long>(fit, 1 << 20) / big * big);
     const int n = row1 - j.row0;
-    const int step = div_up(div_up(n, div_up(n, most)), th) * th;
+    const int step = div_up(div_up(n, div_up(n, most)), big) * big;
     for (int y = j.row0; y < row1; y += step) {
       SplitSeg s{};
       s.scene = j.scene;
@@ -606,29 +675,47 @@ bool split_layout(const Plan& pl, const std::vector<SceneGeom>& geo, const std::
       s.rows = s.vy1 - s.row0;
       s.pitch = pitch;
       s.tiles_x = div_up(g.vW + 1, kTileW);
-      // the mean kernel's offsets inside a pass's volume are 32-bit
-      if ((size_t)nhalf * s.rows * pitch > 0x7fffffff) return false;
-      const size_t words = row_words * s.rows;
-      if (out.chunks.empty() || (used && used + words > budget)) {
+      // the mean kernel's word offsets within a pass are 32-bit
+      if ((size_t)nhalf * s.rows * pitch > 0x3fffffff) return false;
+      size_t bytes = 0;
+      for (int p = 0; p < F.npass; ++p) {
+        s.pass[p] = bytes;
+        bytes += ((size_t)nhalf * s.rows * pitch * word_bytes(F.pass[p].np) + 255) / 256 * 256;
+      }
+      if (out.chunks.empty() || (used && used + bytes > budget)) {
         close_chunk();
         out.chunks.push_back(SplitChunk{});
         out.chunks.back().seg0 = (int)out.segs.size();
       }
       s.vol = used;
-      used += words;
-      out.vol_words = std::max(out.vol_words, used);
+      used += bytes;
+      out.vol_bytes = std::max(out.vol_bytes, used);
       out.segs.push_back(s);
     }
   }
   close_chunk();
   for (SplitChunk& c : out.chunks) {
+    // Rows of the mean tiles: waves of blocks (one per SM) times a block's
+    // time, measured at 1024^2: 182, 94 and 59 us for 32, 16 and 8 rows (few
+    // warps leave latency uncovered), in proportion for other patch sets
+    double best_t = 0.0;
+    for (int th : {big, 16, 8}) {
+      int tiles = 0;
+      for (int i = c.seg0; i < c.seg1; ++i)
+        tiles += out.segs[i].tiles_x * div_up(out.segs[i].vy1 - out.segs[i].vy0, th);
+      const double t = (double)div_up(tiles, sms) * (th > 16 ? 182.0 : (th > 8 ? 94.0 : 59.0));
+      if (best_t == 0.0 || t < 0.98 * best_t) {
+        best_t = t;
+        c.th = th;
+        c.tiles = tiles;
+      }
+    }
     int tiles = 0;
     for (int i = c.seg0; i < c.seg1; ++i) {
       SplitSeg& s = out.segs[i];
       s.tile_begin = tiles;
-      tiles += s.tiles_x * div_up(s.vy1 - s.vy0, th);
+      tiles += s.tiles_x * div_up(s.vy1 - s.vy0, c.th);
     }
-    c.tiles = tiles;
     for (int k = 0; k < out.nshape; ++k) {
       // Block rows R and offset groups Z: the time of a chunk is its waves of
       // blocks (one per SM) times a block's time, staging (about 0.1 us per
@@ -682,7 +769,7 @@ bool split_layout(const Plan& pl, const std::vector<SceneGeom>& geo, const std::
 int split_launches(const SplitLayout& lay) { return (int)lay.chunks.size() * (lay.nshape + 1); }
 
 cudaError_t launch_split(const Plan& pl, const FilterParams& F, const SplitLayout& lay, int chunk,
-                         const SceneDesc* d_scenes, const SplitSeg* d_segs, uint32_t* vol, cudaStream_t st) {
+                         const SceneDesc* d_scenes, const SplitSeg* d_segs, char* vol, cudaStream_t st) {
   const SplitChunk& c = lay.chunks[chunk];
   const SplitSeg* segs = d_segs + c.seg0;
   const int nseg = c.seg1 - c.seg0;
@@ -704,13 +791,12 @@ cudaError_t launch_split(const Plan& pl, const FilterParams& F, const SplitLayou
     }
   }
   if (e != cudaSuccess) return e;
-  int npx = 1;
-  for (int i = 0; i < F.npass; ++i) npx = std::max(npx, F.pass[i].np);
+  const bool single = single_patches(F);
   if (pl.full8)
-    return npx == 1 ? launch_mean_t<1, true>(F, d_scenes, segs, nseg, vol, c.tiles, st)
-                    : launch_mean_t<3, true>(F, d_scenes, segs, nseg, vol, c.tiles, st);
-  return npx == 1 ? launch_mean_t<1, false>(F, d_scenes, segs, nseg, vol, c.tiles, st)
-                  : launch_mean_t<3, false>(F, d_scenes, segs, nseg, vol, c.tiles, st);
+    return single ? launch_mean_th<true, 1>(c.th, F, d_scenes, segs, nseg, vol, c.tiles, st)
+                  : launch_mean_th<true, 3>(c.th, F, d_scenes, segs, nseg, vol, c.tiles, st);
+  return single ? launch_mean_th<false, 1>(c.th, F, d_scenes, segs, nseg, vol, c.tiles, st)
+                : launch_mean_th<false, 3>(c.th, F, d_scenes, segs, nseg, vol, c.tiles, st);
 }
 
 }  // namespace dcl

@@ -12,17 +12,14 @@
 
 namespace dcl {
 
-// Rows of a mean-kernel tile: InSAR input, 8-plane covariance input.
-constexpr int kSplitTileH = 16;
-constexpr int kSplitTileH8 = 24;
 // Volume of weight indices held at a time.
 constexpr size_t kSplitBudgetBytes = size_t(2) << 30;
 constexpr size_t kSplitMinBudgetBytes = size_t(32) << 20;  // below it the fused kernel filters
 constexpr size_t kSplitSmem = 227 * 1024;
 constexpr int kSplitShapes = 2;  // different pass shapes of one call
 
-// A run of virtual rows of one scene with its volume
-// [pass][half-window offset][rows][pitch] of 32-bit words.
+// A run of virtual rows of one scene with its volume: per pass words
+// [half-window offset][rows][pitch] of one byte per patch size (three: four).
 struct SplitSeg {
   int scene;
   int vy0, vy1;        // virtual rows filtered
@@ -30,12 +27,13 @@ struct SplitSeg {
   int pitch;           // words per row; volume column c is virtual column c - wsh
   int tiles_x, tile_begin;                // mean kernel: tiles per row, first tile in the chunk
   int idx_begin[kSplitShapes], idx_bx[kSplitShapes], idx_R[kSplitShapes];  // index kernel: blocks, columns, rows
-  size_t vol;          // first word
+  size_t vol, pass[kMaxPasses];  // first byte, and of each pass from there
 };
 
 // Segments filtered together: one index launch per pass shape, one mean launch.
 struct SplitChunk {
-  int seg0, seg1, tiles;
+  int seg0, seg1;
+  int th, tiles;  // mean kernel: tile rows, tiles
   int idx_blocks[kSplitShapes], idx_z[kSplitShapes];
   size_t idx_smem[kSplitShapes];
 };
@@ -54,25 +52,25 @@ struct SplitJob {
 struct SplitLayout {
   std::vector<SplitSeg> segs;
   std::vector<SplitChunk> chunks;
-  size_t vol_words;
+  size_t vol_bytes;
   int nshape, shape[kSplitShapes];
   PassList passes[kSplitShapes];
 };
 
 // Whether the two-kernel path serves a call (the specialised kernel's shapes
-// in its default arithmetic).
-bool split_supported(const FilterParams& F, bool full8);
+// in its default arithmetic, tables that fit byte codes).
+bool split_supported(const Plan& pl);
 bool split_layout(const Plan& pl, const std::vector<SceneGeom>& geo, const std::vector<SplitJob>& jobs,
-                  size_t budget_words, int sms, SplitLayout& out);
+                  size_t budget, int sms, SplitLayout& out);
 // Kernels a layout launches.
 int split_launches(const SplitLayout& lay);
 // Launches chunk `chunk`: index kernels, then the mean kernel.
 cudaError_t launch_split(const Plan& pl, const FilterParams& F, const SplitLayout& lay, int chunk,
-                         const SceneDesc* d_scenes, const SplitSeg* d_segs, uint32_t* vol, cudaStream_t st);
+                         const SceneDesc* d_scenes, const SplitSeg* d_segs, char* vol, cudaStream_t st);
 
 // All chunks of a layout (nlsar_host.cu), timed as one launch by the profile.
 int launch_split_all(const Plan& pl, const FilterParams& F, const SplitLayout& lay, const SceneDesc* d_scenes,
-                     const SplitSeg* d_segs, uint32_t* vol, cudaStream_t st);
+                     const SplitSeg* d_segs, char* vol, cudaStream_t st);
 int sm_count(int dev);
 
 }  // namespace dcl
