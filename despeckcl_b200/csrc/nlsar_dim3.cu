@@ -44,6 +44,8 @@
 #include "dcl_internal.h"
 #include "nlsar_common.cuh"
 #include "nlsar_plan.h"
+#include "nlsar_split.h"
+#include "nlsar_split3.cuh"
 #include "stats_internal.h"
 
 namespace dcl {
@@ -58,31 +60,7 @@ constexpr int kT3H = kT3Warps;  // output rows per tile
 constexpr int kT3Threads = 32 * kT3Warps;
 constexpr int kNA3 = 23;        // accumulators per patch size
 
-// planes of the nine similarity reals within the 18 covariance planes
-__host__ __device__ constexpr int sim_plane(int k) {
-  return k == 0 ? 0 : k == 1 ? 8 : k == 2 ? 16 : k == 3 ? 2 : k == 4 ? 3 : k == 5 ? 4 : k == 6 ? 5 : k == 7 ? 10 : 11;
-}
-// planes of the diagonal intensities
-__host__ __device__ constexpr int diag_plane(int d) { return 8 * d; }
-
 __device__ __forceinline__ int clamp3(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
-
-// sim_measures.h:78-97 with a = {a00, a11, a22, Re a01, Im a01, Re a02, Im a02, Re a12, Im a12}
-__host__ __device__ __forceinline__ float det3f(const float* a) {
-  return a[0] * a[1] * a[2] - a[0] * (a[7] * a[7] + a[8] * a[8]) - a[1] * (a[5] * a[5] + a[6] * a[6]) -
-         a[2] * (a[3] * a[3] + a[4] * a[4]) +
-         2.0f * (a[3] * a[7] * a[5] - a[4] * a[8] * a[5] + a[3] * a[8] * a[6] + a[4] * a[7] * a[6]);
-}
-
-struct Scene3 {
-  const float* c18;             // [18][Hp][pitch]
-  const float* s9[kMaxScales];  // [9][Hp][pitch] per scale slot
-  const float* ld[kMaxScales];  // [Hp][pitch] per scale slot
-  float* out;                   // [18][H][W]
-  int H, W, vH, vW, pitch, tiles_x;
-  int tile_skip;                // scene tiles before block 0 of the launch (row bands)
-  size_t plane;                 // Hp * pitch
-};
 
 struct Smem3 {
   int rs_w, rs_h, sim_w, sim_h;
@@ -916,8 +894,10 @@ struct Run3 {
   Plan pl;
   Scene3 S;
   size_t smem = 0;
-  int tiles_y = 0, Hp = 0, Wp = 0, used = 0;
+  int tiles_y = 0, Hp = 0, Wp = 0, used = 0, sms = 148;
   char* scratch = nullptr;
+  Split3 split;  // the two-kernel path's segments (rows 0: not used)
+  char* vol = nullptr;
 };
 
 static int plan3(const Plan& pl0, int H, int W, float* cout, Run3& r, cudaStream_t st) {
@@ -958,8 +938,22 @@ static int plan3(const Plan& pl0, int H, int W, float* cout, Run3& r, cudaStream
   for (char u : r.pl.slot_used) r.used += u ? 1 : 0;
   const size_t frame_bytes = S.plane * sizeof(float) * (18 + 10 * (size_t)r.used);
   const size_t wtab_bytes = r.pl.wtab.size() * sizeof(float);
-  cudaError_t e = cudaMallocAsync(&r.scratch, frame_bytes + wtab_bytes + 256, st);
+  // the two-kernel path where it serves the call; a smaller volume where the
+  // device has no room for the usual one, the fused kernel where it has none
+  r.sms = sm_count(dev);
+  size_t budget = kSplitBudgetBytes;
+  if (r.pl.fast && fast3_supported(F) && !F.withhold_staging) r.split = split3_layout(r.pl, S, budget);
+  const size_t fixed = (frame_bytes + 255) / 256 * 256 + (wtab_bytes + 255) / 256 * 256;
+  cudaError_t e = cudaSuccess;
+  for (;;) {
+    e = cudaMallocAsync(&r.scratch, fixed + (r.split.rows ? r.split.vol_bytes : 0), st);
+    if (e != cudaErrorMemoryAllocation || !r.split.rows) break;
+    cudaGetLastError();
+    budget /= 4;
+    r.split = budget >= kSplitMinBudgetBytes ? split3_layout(r.pl, S, budget) : Split3{};
+  }
   if (e != cudaSuccess) return cuda_error(e, "cudaMallocAsync(3x3 scratch)");
+  r.vol = r.scratch + fixed;
   float* p = reinterpret_cast<float*>(r.scratch);
   S.c18 = p;
   p += 18 * S.plane;
@@ -1009,7 +1003,7 @@ static int prep3_rows(const Run3& r, const float* cin, int co0, int co1, int cs0
   return e == cudaSuccess ? DCL_OK : cuda_error(e, "NL-SAR 3x3 prep");
 }
 
-// the fused kernel on tile rows [t0, t1)
+// the filter kernels on tile rows [t0, t1)
 static int launch3_rows(const Run3& r, int t0, int t1, cudaStream_t st) {
   if (t1 <= t0) return DCL_OK;
   Scene3 S = r.S;
@@ -1018,6 +1012,13 @@ static int launch3_rows(const Run3& r, int t0, int t1, cudaStream_t st) {
   const unsigned tiles = (unsigned)((t1 - t0) * S.tiles_x);
   F.total_tiles = (int)tiles;
   cudaError_t e;
+  if (r.split.rows) {
+    const int end = std::min(t1 * kT3H, S.vH + 1);
+    e = cudaSuccess;
+    for (int y = t0 * kT3H; y < end && e == cudaSuccess; y += r.split.rows)
+      e = launch_split3(r.pl, F, S, r.Hp, r.Wp, r.split, r.vol, y, std::min(y + r.split.rows, end), r.sms, st);
+    return e == cudaSuccess ? DCL_OK : cuda_error(e, "NL-SAR 3x3");
+  }
   if (r.pl.fast && fast3_supported(F)) {
     e = launch3_fast(F, S, tiles, st);
   } else {

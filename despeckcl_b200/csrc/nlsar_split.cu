@@ -39,41 +39,14 @@
 #include "dcl_internal.h"
 #include "nlsar_math.cuh"
 #include "nlsar_split.h"
+#include "nlsar_words.cuh"
 
 namespace dcl {
 
 namespace {
 
-// A weight's code: one byte, its table entry, or kZeroCode for weight 0
-// (d > dmax).  Entry 255 is reached only where the scaled sum rounds to
-// exactly 1; it is coded as 254, so a call whose tables have 256 entries needs
-// entries 254 and 255 equal (split_supported).
-constexpr int kZeroCode = 255;
-
-// The codes of a pass of NP patch sizes at one (offset, pixel).
-template <int NP>
-struct WordOf {
-  using T = uint32_t;
-};
-template <>
-struct WordOf<1> {
-  using T = uint8_t;
-};
-template <>
-struct WordOf<2> {
-  using T = uint16_t;
-};
-
 constexpr int kIdxWarps = 16;
 constexpr int kIdxThreads = 32 * kIdxWarps;
-
-template <int PHM>
-struct IdxL {
-  // lanes own four adjacent columns; HL lanes at each end of a warp only
-  // supply the patch halo
-  static constexpr int HL = (PHM + 3) / 4;
-  static constexpr int VC = 128 - 8 * HL;  // columns a warp produces
-};
 
 __host__ __device__ inline int idx_left(int wsh) { return (wsh + 3) / 4 * 4; }  // staged columns left of lane 0
 // float4 slots of a staged row: five per four pixels (see the kernel)
@@ -94,24 +67,16 @@ __host__ __device__ inline size_t idx_smem(int wsh, int phm, int R) {
 // plane with the same indexing holds 1/(4 det) alone for the neighbours
 // (4-byte loads, five words apart: conflict free).
 //
-// A warp walks down the rows for one offset.  Per row a lane evaluates four
-// similarities, gets the patch halo from its neighbour lanes by shuffles,
-// forms the horizontal sums in the nested-ring order of the fused kernel, and
-// keeps, per patch size 2 ph + 1, the 2 ph partial vertical sums in flight
-// (the sum of the last k rows, top down), so a vertical sum costs 2 ph adds,
-// two columns per packed add, and no loads.  A smaller patch is complete
-// PHM - ph rows before the largest, so its field waits in `pend`.
+// A warp walks down the rows for one offset (WordWalk), a lane evaluating the
+// four similarities of its columns per row.
 template <int PH0, int PH1, int PH2>
 __global__ void __launch_bounds__(kIdxThreads, 1)
     nlsar_index_kernel(const __grid_constant__ FilterParams P, const SceneDesc* __restrict__ scenes,
                        const SplitSeg* __restrict__ segs, int nseg, const __grid_constant__ PassList passes,
                        int shape, char* __restrict__ vol) {
-  constexpr int NP = np_of<PH0, PH1, PH2>();
+  using Walk = WordWalk<PH0, PH1, PH2>;
+  constexpr int NP = Walk::NP, PHM = Walk::PHM, HL = Walk::HL, VC = Walk::VC;
   using Word = typename WordOf<NP>::T;
-  constexpr int PHM = cmax(PH0, cmax(PH1, PH2));
-  constexpr int HL = IdxL<PHM>::HL, VC = IdxL<PHM>::VC;
-  constexpr int ND = PHM - PH0;  // rows the first patch's field waits
-  static_assert(PH0 >= 1 && 4 * HL >= PHM, "pass shape");
   extern __shared__ float4 smem4[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int lo = 0, hi = nseg - 1;
@@ -160,18 +125,8 @@ __global__ void __launch_bounds__(kIdxThreads, 1)
       }
     }
   }
-  // patch sums are in log2 units: the lookup scales by ln 2 (nlsar_fast.cu)
-  float inv_span[NP], nbias[NP], lm1[NP], dmax[NP];
-#pragma unroll
-  for (int j = 0; j < NP; ++j) {
-    const ComboParams& cp = P.combo[pp.combo[j]];
-    inv_span[j] = 1.0f / cp.span;
-    nbias[j] = -cp.dmin * inv_span[j];
-    lm1[j] = cp.lm1;
-    dmax[j] = cp.dmax;
-    inv_span[j] *= 0.69314718f;
-    dmax[j] *= 1.44269504f;
-  }
+  Walk walk;
+  walk.set(P, pp, true);  // patch sums in log2 units (nlsar_fast.cu)
   __syncthreads();
 
   const int nhalf = P.n_off / 2;
@@ -191,27 +146,13 @@ __global__ void __launch_bounds__(kIdxThreads, 1)
     Word* out = out0 + (size_t)u * plane;
     const float4* ctr = sC + 5 * (lane + (left >> 2));
     const int n0 = dy * SP + 5 * (lane + (t0 >> 2)) + (t0 & 3);
-    auto walk = [&](auto m_tag) {
-    constexpr int M = decltype(m_tag)::value;
-    const float4* nbr = sC + n0;
-    const float* nld = sL + n0;
-    // partial vertical sums: vs[j][k]: last k + 1 rows of patch j, columns in pairs
-    float2 vs[NP][2 * PHM][2];
-    uint32_t pend[ND > 0 ? ND : 1][4];
-#pragma unroll
-    for (int j = 0; j < NP; ++j)
-#pragma unroll
-      for (int k = 0; k < 2 * PHM; ++k)
-#pragma unroll
-        for (int q = 0; q < 2; ++q) vs[j][k][q] = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int k = 0; k < ND; ++k)
-#pragma unroll
-      for (int o = 0; o < 4; ++o) pend[k][o] = 0;
-    for (int i = 0; i < R + 2 * PHM; ++i) {
-      // ---- similarities of the lane's four columns
-      float s[4 + 2 * PHM];
-      {
+    auto down = [&](auto m_tag) {
+      constexpr int M = decltype(m_tag)::value;
+      const float4* nbr = sC + n0;
+      const float* nld = sL + n0;
+      walk.start();
+      for (int i = 0; i < R + 2 * PHM; ++i) {
+        float s[4 + 2 * PHM];
         const float4 la = ctr[4];
         const float la4[4] = {la.x, la.y, la.z, la.w};
 #pragma unroll
@@ -219,101 +160,22 @@ __global__ void __launch_bounds__(kIdxThreads, 1)
           const int n = j + (M + j >= 4 ? 1 : 0);
           s[PHM + j] = glr_ratio(ctr[j], la4[j], nbr[n], nld[n]);
         }
-      }
-      ctr += SP;
-      nbr += SP;
-      nld += SP;
-#pragma unroll
-      for (int k = 1; k <= PHM; ++k) {
-        s[PHM - k] = __shfl_up_sync(0xffffffffu, s[PHM + 3 - (k - 1) % 4], (k + 3) / 4);
-        s[PHM + 3 + k] = __shfl_down_sync(0xffffffffu, s[PHM + (k - 1) % 4], (k + 3) / 4);
-      }
-      // ---- horizontal sums (nested rings)
-      float hs[NP][4];
-      auto rings = [&] {
-#pragma unroll
-        for (int o = 0; o < 4; ++o) {
-          float ring = s[o + PHM];
-#pragma unroll
-          for (int b = 1; b <= PHM; ++b) {
-            ring += s[o + PHM - b] + s[o + PHM + b];
-#pragma unroll
-            for (int j = 0; j < NP; ++j)
-              if (ph_of<PH0, PH1, PH2>(j) == b) hs[j][o] = ring;
-          }
-        }
-      };
-      rings();
-      // a NaN similarity counts as 0; the largest rings of the first and last
-      // column hold every similarity, so one test finds any NaN
-      if (isnan(hs[NP - 1][0]) || isnan(hs[NP - 1][3])) {
-#pragma unroll
-        for (int k = 0; k < 4 + 2 * PHM; ++k)
-          if (isnan(s[k])) s[k] = 0.0f;
-        rings();
-      }
-      // ---- vertical sums, the weight's table index
-      uint32_t field[NP][4];
-#pragma unroll
-      for (int j = 0; j < NP; ++j) {
-        const int n = 2 * ph_of<PH0, PH1, PH2>(j);
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const float2 h = make_float2(hs[j][2 * q], hs[j][2 * q + 1]);
-          const float2 d2 = __fadd2_rn(vs[j][n - 1][q], h);
-#pragma unroll
-          for (int k = n - 1; k > 0; --k) vs[j][k][q] = __fadd2_rn(vs[j][k - 1][q], h);
-          vs[j][0][q] = h;
-          // saturating FMA (clamps, NaN to 0), round-toward-zero add of 2^23:
-          // the low mantissa bits are the index; d > dmax: weight 0
-          const float2 u2 = make_float2(__saturatef(fmaf(d2.x, inv_span[j], nbias[j])),
-                                        __saturatef(fmaf(d2.y, inv_span[j], nbias[j])));
-          const float2 t2 = __ffma2_rz(u2, make_float2(lm1[j], lm1[j]), make_float2(8388608.0f, 8388608.0f));
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const uint32_t code = min(__float_as_uint(e ? t2.y : t2.x), 0x4B000000u + (kZeroCode - 1));
-            field[j][2 * q + e] = (e ? d2.y : d2.x) > dmax[j] ? (uint32_t)kZeroCode : code;  // the low byte counts
-          }
+        ctr += SP;
+        nbr += SP;
+        nld += SP;
+        uint32_t w[4];
+        walk.template row<true>(s, w);
+        if (i >= 2 * PHM) {
+          if (writes) store_words<NP>(out, w);
+          out += S.pitch;
         }
       }
-      // ---- the words of row i - 2 PHM: byte j is the code of patch j
-      uint32_t w[4];
-#pragma unroll
-      for (int o = 0; o < 4; ++o) {
-        uint32_t next = 0;
-#pragma unroll
-        for (int k = ND; k >= 0; --k) {  // rows waited, the smallest patch first
-          uint32_t v = k < ND ? pend[k][o] : 0u;
-#pragma unroll
-          for (int j = 0; j < NP; ++j)
-            if (PHM - ph_of<PH0, PH1, PH2>(j) == k)
-              v = j == 0 ? field[0][o] : __byte_perm(v, field[j][o], j == 1 ? 0x0040 : 0x0410);
-          if (k < ND) pend[k][o] = next;
-          next = v;
-        }
-        w[o] = next;
-      }
-      if (i >= 2 * PHM) {
-        if (writes) {
-          if constexpr (NP == 3) {
-            *reinterpret_cast<uint4*>(out) = make_uint4(w[0], w[1], w[2], w[3]);
-          } else if constexpr (NP == 2) {
-            *reinterpret_cast<uint2*>(out) =
-                make_uint2(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410));
-          } else {
-            *reinterpret_cast<uint32_t*>(out) =
-                __byte_perm(__byte_perm(w[0], w[1], 0x0040), __byte_perm(w[2], w[3], 0x0040), 0x5410);
-          }
-        }
-        out += S.pitch;
-      }
-    }
     };
     switch (t0 & 3) {
-      case 0: walk(std::integral_constant<int, 0>{}); break;
-      case 1: walk(std::integral_constant<int, 1>{}); break;
-      case 2: walk(std::integral_constant<int, 2>{}); break;
-      default: walk(std::integral_constant<int, 3>{});
+      case 0: down(std::integral_constant<int, 0>{}); break;
+      case 1: down(std::integral_constant<int, 1>{}); break;
+      case 2: down(std::integral_constant<int, 2>{}); break;
+      default: down(std::integral_constant<int, 3>{});
     }
   }
 }
@@ -615,7 +477,11 @@ int div_up(int a, int b) { return (a + b - 1) / b; }
 
 bool split_supported(const Plan& pl) {
   const FilterParams& F = pl.P;
-  if (F.prec != 0 || F.withhold_staging || !pl.fast) return false;
+  return F.prec == 0 && !F.withhold_staging && pl.fast && split_tables_ok(pl);
+}
+
+bool split_tables_ok(const Plan& pl) {
+  const FilterParams& F = pl.P;
   for (int i = 0; i < F.npass; ++i)
     for (int j = 0; j < F.pass[i].np; ++j) {
       const int c = F.pass[i].combo[j];

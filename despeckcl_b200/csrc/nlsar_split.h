@@ -60,6 +60,8 @@ struct SplitLayout {
 // Whether the two-kernel path serves a call (the specialised kernel's shapes
 // in its default arithmetic, tables that fit byte codes).
 bool split_supported(const Plan& pl);
+// Whether the weight tables of a plan's passes fit byte codes.
+bool split_tables_ok(const Plan& pl);
 bool split_layout(const Plan& pl, const std::vector<SceneGeom>& geo, const std::vector<SplitJob>& jobs,
                   size_t budget, int sms, SplitLayout& out);
 // Kernels a layout launches.

@@ -38,3 +38,27 @@ def test_two_kernel_path_equals_fused_kernel(shape, patches, scales):
         for g, w in zip(got, want):
             np.testing.assert_array_equal(g.cpu().numpy(), w.cpu().numpy())
         b.close()
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (1, 33), (12, 18), (13, 32), (25, 107), (49, 131)])
+@pytest.mark.parametrize("patches,scales", [([3, 5, 7], [1, 3]), ([3, 5, 7, 9, 11], [1, 3]), ([5], [1, 3])])
+def test_two_kernel_3x3_path_equals_fused_kernel(shape, patches, scales, monkeypatch):
+    # the staging switch of the timeout tests keeps calls on the fused kernels;
+    # the 3x3 one has no staging copies to withhold
+    def cov(h, w, seed):
+        rng = np.random.default_rng(seed)
+        z = rng.normal(size=(3, 5)) + 1j * rng.normal(size=(3, 5))
+        x = rng.normal(size=(3, h * w)) + 1j * rng.normal(size=(3, h * w))
+        k = (np.linalg.cholesky(z @ z.conj().T) @ x).reshape(3, h, w) * np.linspace(1, 2, w)
+        return (k[:, None] * k[None, :].conj()).astype(np.complex64)
+
+    key = ("3x3", tuple(patches), tuple(scales))
+    if key not in _STATS:
+        _STATS[key] = dcl.nlsar_train(cov(40, 40, 1), patches, scales)
+    c = cov(*shape, 2)
+    for mode in ("argmax_enl", "reference"):
+        monkeypatch.delenv("DESPECKCL_B200_TEST_WITHHOLD_STAGING", raising=False)
+        got = dcl.nlsar(c, 21, patches, scales, _STATS[key], select_mode=mode)
+        monkeypatch.setenv("DESPECKCL_B200_TEST_WITHHOLD_STAGING", "1")
+        want = dcl.nlsar(c, 21, patches, scales, _STATS[key], select_mode=mode)
+        np.testing.assert_array_equal(got.view(np.float32), want.view(np.float32))
