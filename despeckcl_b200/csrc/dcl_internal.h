@@ -18,6 +18,8 @@ constexpr int kMaxDevices = 64;
 // (the limit is a per-device attribute); `cache` holds, per device, the
 // largest size already allowed, so repeated launches skip the call.
 cudaError_t allow_dynamic_smem(const void* func, size_t bytes, size_t* cache);
+// SMs of a device (148 where the query fails).
+int sm_count(int dev);
 // Count `n` kernel launches of the calling thread while dcl_profile_begin is active.
 void profile_count(int n);
 

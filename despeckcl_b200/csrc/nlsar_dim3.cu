@@ -1,8 +1,6 @@
 // NL-SAR on 3x3 (PolSAR) covariance images: despeckcl::nlsar with dim = 3
 // (src/compute/nlsar/nlsar.cpp:171-194 in the reference, the same per-tile
-// pipeline as the 2x2 case, nlsar_filter_sub_image.cpp:146-390) and
-// despeckcl::nlsar_training on such images (training/get_dissims.cpp,
-// training/patches.cpp:43-136).
+// pipeline as the 2x2 case, nlsar_filter_sub_image.cpp:146-390).
 //
 // Differences from the 2x2 path, all following the reference (paths relative
 // to src/compute/nlsar/):
@@ -46,7 +44,6 @@
 #include "nlsar_plan.h"
 #include "nlsar_split.h"
 #include "nlsar_split3.cuh"
-#include "stats_internal.h"
 
 namespace dcl {
 
@@ -811,76 +808,6 @@ cudaError_t launch3_fast(const FilterParams& F, const Scene3& S, unsigned tiles,
 }
 
 
-// ---- training ---------------------------------------------------------------
-
-// rescaled and averaged similarity reals on the valid region (H-s+1) x (W-s+1),
-// [pixel][9] (get_dissims.cpp:84-100 with scale_size_max = s)
-__global__ void train3_avg_kernel(const float* __restrict__ cov, int H, int W, int s, GaussArg ga, float gamma,
-                                  float* __restrict__ out) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int yy = blockIdx.y * blockDim.y + threadIdx.y;
-  const int Ho = H - s + 1, Wo = W - s + 1;
-  if (x >= Wo || yy >= Ho) return;
-  const size_t n = (size_t)H * W;
-  float a[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) a[k] = 0.0f;
-  for (int kx = 0; kx < s; ++kx)
-    for (int ky = 0; ky < s; ++ky) {
-      const size_t q = (size_t)(yy + kx) * W + x + ky;
-      const float g = ga.g[kx * s + ky];
-#pragma unroll
-      for (int k = 0; k < 9; ++k) {
-        const float v = cov[sim_plane(k) * n + q];
-        a[k] = fmaf(g, k >= 3 ? v * gamma : v, a[k]);
-      }
-    }
-#pragma unroll
-  for (int k = 0; k < 9; ++k) out[((size_t)yy * Wo + x) * 9 + k] = a[k];
-}
-
-// patches [n][p*p][9], patch k at ((k / nw) * p, (k % nw) * p), clamp padding
-__global__ void train3_gather_kernel(const float* __restrict__ avg, int Ho, int Wo, int p, int nw, int n,
-                                     float* __restrict__ patches) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int pp = p * p;
-  if (i >= n * pp) return;
-  const int k = i / pp, r = i - k * pp;
-  const int yy = min(Ho - 1, (k / nw) * p + r / p);
-  const int x = min(Wo - 1, (k % nw) * p + r % p);
-#pragma unroll
-  for (int q = 0; q < 9; ++q) patches[(size_t)i * 9 + q] = avg[((size_t)yy * Wo + x) * 9 + q];
-}
-
-// one thread per unordered pair (hi, j), hi > j: the later patch first
-// (combinations.cpp:26-41, patches.cpp:43-69)
-__global__ void train3_pairs_kernel(const float* __restrict__ patches, int pp, long long npairs, float c2d,
-                                    float* __restrict__ out) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= npairs) return;
-  long long hi = (long long)((1.0 + sqrt(1.0 + 8.0 * (double)t)) * 0.5);
-  while (hi * (hi - 1) / 2 > t) --hi;
-  while ((hi + 1) * hi / 2 <= t) ++hi;
-  const long long j = t - hi * (hi - 1) / 2;
-  const float* A = patches + (size_t)hi * pp * 9;
-  const float* B = patches + (size_t)j * pp * 9;
-  float sum = 0.0f;
-  for (int i = 0; i < pp; ++i) {
-    float a[9], b[9], s[9];
-#pragma unroll
-    for (int q = 0; q < 9; ++q) {
-      a[q] = A[i * 9 + q];
-      b[q] = B[i * 9 + q];
-      s[q] = a[q] + b[q];
-    }
-    // sim_measures.h:100-160, nlooks 1
-    float r = -(c2d + logf(det3f(a)) + logf(det3f(b)) - 2.0f * logf(det3f(s)));
-    if (r != r) r = 0.0f;
-    sum += r;
-  }
-  out[t] = sum;
-}
-
 float rescale_gamma_3x3() {
   // covmat_rescale.cl:25-26 with nlooks = 1, dimension = 3
   return std::pow(std::min(1.0f / 3.0f, 1.0f), 0.33333f);
@@ -1129,85 +1056,6 @@ int nlsar_covmat3_host(const Plan& pl, const float* cin, float* cout, int H, int
   const cudaError_t e4 = cudaStreamSynchronize(st);
   if (rc == DCL_OK && e4 != cudaSuccess) rc = cuda_error(e4, "NL-SAR 3x3");
   return rc;
-}
-
-namespace {
-
-struct DevMem {
-  void* p = nullptr;
-  ~DevMem() {
-    if (p) cudaFree(p);
-  }
-};
-
-int train3_one(const float* d_cov, int H, int W, int p, int s, std::vector<float>& sorted) {
-  const int Ho = H - s + 1, Wo = W - s + 1;
-  if (Ho < 1 || Wo < 1)
-    return set_error(DCL_ERR_INVALID_ARGUMENT, "training area %dx%d smaller than scale %d", H, W, s);
-  const int nh = (Ho + p - 1) / p, nw = (Wo + p - 1) / p;
-  const long long n = (long long)nh * nw;
-  if (n < 2) return set_error(DCL_ERR_INVALID_ARGUMENT, "training area holds fewer than two %dx%d patches", p, p);
-  const long long npairs = n * (n - 1) / 2;
-  const int pp = p * p;
-  DevMem avg, pat, dis, dis2;
-  cudaError_t e = cudaMalloc(&avg.p, (size_t)Ho * Wo * 9 * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&pat.p, (size_t)n * pp * 9 * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&dis.p, (size_t)npairs * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&dis2.p, (size_t)npairs * sizeof(float));
-  if (e != cudaSuccess) return cuda_error(e, "training buffers");
-  GaussArg ga;
-  std::memset(&ga, 0, sizeof ga);
-  const std::vector<float> g = gauss_weights(s);
-  std::copy(g.begin(), g.end(), ga.g);
-  dim3 blk(32, 8), grd((Wo + 31) / 32, (Ho + 7) / 8);
-  train3_avg_kernel<<<grd, blk>>>(d_cov, H, W, s, ga, rescale_gamma_3x3(), (float*)avg.p);
-  train3_gather_kernel<<<(unsigned)((n * pp + 255) / 256), 256>>>((const float*)avg.p, Ho, Wo, p, nw, (int)n,
-                                                                  (float*)pat.p);
-  train3_pairs_kernel<<<(unsigned)((npairs + 255) / 256), 256>>>((const float*)pat.p, pp, npairs,
-                                                                2 * 3 * std::log(2.0f), (float*)dis.p);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_error(e, "training kernels");
-  return sort_dissims((float*)dis.p, (float*)dis2.p, npairs, sorted);
-}
-
-}  // namespace
-
-dcl_stats_collection* training_covmat3(const float* cov18, int H, int W, const int* patches, int np,
-                                       const int* scales, int ns) {
-  if (!cov18 || H < 1 || W < 1) {
-    set_error(DCL_ERR_INVALID_ARGUMENT, "null input or empty training area");
-    return nullptr;
-  }
-  if (!patches || !scales || np < 1 || ns < 1) {
-    set_error(DCL_ERR_INVALID_ARGUMENT, "patch_sizes and scale_sizes must not be empty");
-    return nullptr;
-  }
-  const size_t n = (size_t)18 * H * W;
-  DevMem d_cov;
-  cudaError_t e = cudaMalloc(&d_cov.p, n * sizeof(float));
-  if (e == cudaSuccess) e = cudaMemcpy(d_cov.p, cov18, n * sizeof(float), cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) {
-    cuda_error(e, "training setup");
-    return nullptr;
-  }
-  dcl_stats_collection* c = dcl_collection_new();
-  // get_stats.cpp:33-37: patch outer, scale inner; lut_size 256 (:31)
-  for (int pi = 0; pi < np; ++pi)
-    for (int si = 0; si < ns; ++si) {
-      const int p = patches[pi], s = scales[si];
-      if (p < 1 || p % 2 == 0 || s < 1 || s % 2 == 0 || s * s > kMaxGauss) {
-        set_error(DCL_ERR_INVALID_ARGUMENT, "patch and scale sizes must be odd (scale <= 9)");
-        dcl_stats_collection_free(c);
-        return nullptr;
-      }
-      std::vector<float> sorted;
-      if (train3_one((const float*)d_cov.p, H, W, p, s, sorted) != DCL_OK) {
-        dcl_stats_collection_free(c);
-        return nullptr;
-      }
-      dcl_collection_put(c, p, s, stats_from_sorted(sorted, 256));
-    }
-  return c;
 }
 
 }  // namespace dcl

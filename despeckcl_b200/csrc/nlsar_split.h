@@ -73,6 +73,5 @@ cudaError_t launch_split(const Plan& pl, const FilterParams& F, const SplitLayou
 // All chunks of a layout (nlsar_host.cu), timed as one launch by the profile.
 int launch_split_all(const Plan& pl, const FilterParams& F, const SplitLayout& lay, const SceneDesc* d_scenes,
                      const SplitSeg* d_segs, char* vol, cudaStream_t st);
-int sm_count(int dev);
 
 }  // namespace dcl

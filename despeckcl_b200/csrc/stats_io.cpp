@@ -103,11 +103,43 @@ OwnedStats stats_from_sorted(const std::vector<float>& sorted, unsigned L) {
     const auto it = std::lower_bound(sorted.begin(), sorted.end(), d);
     s.quant[i] = ((float)(it - sorted.begin())) / sorted.size();
   }
-  s.chi2.resize(L);
-  const float ystep = 1.0f / L;
-  for (size_t i = 0; i + 1 < L; ++i) s.chi2[i] = (float)chi2_quantile((double)(i * ystep), 49.0);
-  s.chi2[L - 1] = 100000;
+  s.chi2 = chi2_table(L);
   return s;
+}
+
+// Consecutive quantiles are close, so each is found from the one before: a
+// second-order step along the inverse CDF (dx/dF = 1/f, d2x/dF2 = -f'/f^3),
+// then Halley steps on the CDF until they no longer move it (three
+// evaluations of the CDF instead of the ten of chi2_quantile, which also takes
+// over where a step leaves the bracket).
+std::vector<float> chi2_table(unsigned L) {
+  std::vector<float> t(L, 0.0f);
+  const float ystep = 1.0f / L;
+  const double nu = 49.0, k = nu / 2.0, lnorm = -k * std::log(2.0) - std::lgamma(k);
+  auto pdf = [&](double x) { return std::exp((k - 1.0) * std::log(x) - x / 2.0 + lnorm); };
+  double x = 0.0, at = 0.0;
+  for (size_t i = 1; i + 1 < L; ++i) {
+    const double p = (double)(i * ystep), lo = x;
+    bool found = false;
+    if (i > 1) {
+      const double f = pdf(x), d = (k - 1.0) / x - 0.5, u = (p - at) / f;
+      double nx = x + u * (1.0 - 0.5 * d * u);
+      for (int it = 0; it < 6 && nx > lo && !found; ++it) {
+        const double r = (lower_gamma_reg(k, nx / 2.0) - p) / pdf(nx);
+        const double step = r / (1.0 - 0.5 * r * ((k - 1.0) / nx - 0.5));
+        nx -= step;
+        // a Halley step leaves an error of the cube of its size
+        found = std::fabs(step) <= 1e-6 * nx;
+      }
+      if (found && nx > lo) x = nx;
+      else found = false;
+    }
+    if (!found) x = chi2_quantile(p, nu);
+    at = p;
+    t[i] = (float)x;
+  }
+  t[L - 1] = 100000;
+  return t;
 }
 
 }  // namespace dcl
