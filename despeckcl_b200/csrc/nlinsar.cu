@@ -10,20 +10,23 @@
 //
 //  nlinsar_filter_values_kernel  once per call: 0.5 (a1^2 + a2^2) and
 //      a1 a2 e^{-j phi} per pixel (precompute_filter_values.cl);
-//  nlinsar_weights_kernel  one CTA per tile, the tile's six planes in shared
-//      memory; per search-window offset: the pixel similarity and the
-//      Kullback-Leibler divergence of the estimates (sim_measures.h) on the
-//      similarity grid -- with the two pixels swapped in the tile interior for
-//      the first wsh window rows, which the reference copies from the mirrored
-//      offset (precompute_similarities_{1st,2nd}_pass): each lower-row offset
-//      is taken with its mirror, whose interior maps are the lower offset's
-//      shifted, only its border evaluated --, p x p sums rows
+//  nlinsar_weights_kernel  one CTA per tile and group of offsets, the tile's
+//      planes in shared memory; per search-window offset: the pixel similarity
+//      and the Kullback-Leibler divergence of the estimates (sim_measures.h) on
+//      the similarity grid -- with the two pixels swapped in the tile interior
+//      for the first wsh window rows, which the reference copies from the
+//      mirrored offset (precompute_similarities_{1st,2nd}_pass): each lower-row
+//      offset is taken with its mirror, whose interior maps are the lower
+//      offset's shifted, only its border evaluated --, p x p sums rows
 //      first (precompute_patch_similarities.cl), w = exp(S/h + KL/T) with
-//      NaN / inf -> 0 and the centre weight 0 (compute_weights.cl), the looks
-//      (sum w)^2 / sum w^2 accumulated in offset order
-//      (compute_number_of_looks.cl); weights go to a scratch [tile][offset][pixel];
+//      NaN / inf -> 0 and the centre weight 0 (compute_weights.cl); weights go
+//      to a scratch [tile][offset][pixel].  The similarities do not depend on
+//      the estimates: a call of several passes keeps the first one's patch sums
+//      S (in a second scratch of that shape) and evaluates only divergences
+//      after it; divergences from all-zero estimates are zero and skipped;
 //  nlinsar_estimate_kernel  one thread per tile pixel that owns its output:
-//      below lmin looks the lmin largest weights among the window pixels whose
+//      the looks (sum w)^2 / sum w^2 in the order the offsets are taken
+//      (compute_number_of_looks.cl); below lmin looks the lmin largest weights among the window pixels whose
 //      master amplitude is below twice the centre's become their mean, chosen
 //      with the reference's std::priority_queue (smoothing.cpp:65-117, a binary
 //      heap replayed exactly); then the weighted means (compute_insar.cl),
@@ -45,10 +48,13 @@ namespace dcl {
 namespace {
 
 constexpr int kTile = 80;        // nlinsar.cpp:84, tile_dims {80, 80}
-constexpr int kThreads = 1024;   // weights kernel (32 warps: the one CTA an SM holds)
-constexpr int kMaxPixPerThread = 6;
+// Threads of the weights kernel: with the similarity maps one CTA fills an
+// SM's shared memory; the divergence maps alone leave room for two, whose
+// barriers then cover each other.
+__host__ __device__ constexpr int weights_threads(bool sim) { return sim ? 1024 : 512; }
 constexpr int kMaxLmin = 64;
 constexpr int kEstThreads = 128;
+constexpr size_t kWeightsBytes = size_t(4) << 30;  // weights held at a time
 
 struct NlGeom {
   int H, W, sws, wsh, p, psh, ov;
@@ -98,175 +104,232 @@ __global__ void nlinsar_filter_values_kernel(const float* __restrict__ a1, const
   fi[i] = x1 * x2 * sinf(-d);
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+// Sizes of a tile's maps: compile-time for the usual search windows and patch
+// sizes (the maps' index divisions become multiplications), else from the call.
+template <int SWS_, int P_>
+struct NlSizes {
+  static constexpr bool FIXED = SWS_ > 0;
+  const NlGeom& g;
+  __device__ __forceinline__ int sws() const { return FIXED ? SWS_ : g.sws; }
+  __device__ __forceinline__ int wsh() const { return FIXED ? (SWS_ - 1) / 2 : g.wsh; }
+  __device__ __forceinline__ int p() const { return FIXED ? P_ : g.p; }
+  __device__ __forceinline__ int hsim() const { return FIXED ? kTile - SWS_ + 1 : g.hsim; }
+  __device__ __forceinline__ int hori() const { return FIXED ? kTile - (SWS_ - 1) - (P_ - 1) : g.hori; }
+  __device__ __forceinline__ int nborder() const {
+    return FIXED ? wsh() * hsim() + (hsim() - wsh()) * 2 * wsh() : g.nborder;
+  }
+};
+
+// Work of a tile in units, in the order the looks sum their weights: with
+// mirrored maps the offsets of the centre window row, then every lower-row
+// offset with its mirror; else every offset.
+constexpr float kPairCost = 1.6f;  // a pair of mirrored offsets, in single offsets
+
+__host__ __device__ inline int nl_units(const NlGeom& g) { return g.mirror ? g.sws + g.wsh * g.sws : g.sws * g.sws; }
+// first unit of group z of Z groups of about equal cost
+__host__ __device__ inline int nl_group(const NlGeom& g, int z, int Z) {
+  if (!g.mirror) return (int)((long long)nl_units(g) * z / Z);
+  const float at = (g.sws + kPairCost * (g.wsh * g.sws)) * z / Z;
+  const int u = at <= g.sws ? (int)at : g.sws + (int)((at - g.sws) / kPairCost);
+  return z == Z ? nl_units(g) : (u < nl_units(g) ? u : nl_units(g));
+}
+
+// SIM: evaluate similarities (else their patch sums, over h, are read from
+// `sums`).
+template <class Z_, bool SIM>
+__global__ void __launch_bounds__(weights_threads(SIM), SIM ? 1 : 2)
     nlinsar_weights_kernel(const float* __restrict__ a1, const float* __restrict__ a2, const float* __restrict__ dp,
                            const float* __restrict__ rf, const float* __restrict__ pf, const float* __restrict__ cf,
-                           NlGeom g, int tile0, float* __restrict__ wout, float* __restrict__ nols) {
+                           const __grid_constant__ NlGeom g, int tile0, const int* __restrict__ nonzero,
+                           float* __restrict__ sums, float* __restrict__ wout) {
   extern __shared__ float sm[];
+  constexpr int kThreads = weights_threads(SIM);
+  const Z_ z{g};
   constexpr int n2 = kTile * kTile;
-  float* sA1 = sm;
-  float* sA2 = sA1 + n2;
-  float* sDp = sA2 + n2;
-  float* sRf = sDp + n2;
+  float* sRf = sm;
   float* sPf = sRf + n2;
   float* sCf = sPf + n2;
-  float* sS = sCf + n2;               // [hsim][hsim]
-  float* sK = sS + g.hsim * g.hsim;
-  float* sRS = sK + g.hsim * g.hsim;  // [hsim][hori] row sums
-  float* sRK = sRS + g.hsim * g.hori;
+  float* sA1 = sCf + n2;  // SIM only: the amplitudes and the phase
+  float* sA2 = sA1 + n2;
+  float* sDp = sA2 + n2;
+  const int nsim = z.hsim() * z.hsim(), npix = z.hori() * z.hori(), nrow = z.hsim() * z.hori();
+  const int nborder = g.mirror ? z.nborder() : 0;
+  float* sK = sm + (SIM ? 6 : 3) * n2;  // [hsim][hsim]
+  float* sRK = sK + nsim;               // [hsim][hori] row sums
+  float* sBK = sRK + nrow;              // mirror's border
+  float* sS = sBK + nborder;            // SIM only: the same three maps of the similarity
+  float* sRS = sS + nsim;
+  float* sBS = sRS + nrow;
   const int tile = tile0 + blockIdx.x;
   const int ti = tile / g.ntx, tj = tile - ti * g.ntx;
   const int h0 = -g.ov + ti * g.step, w0 = -g.ov + tj * g.step;
   const int tid = threadIdx.x;
+  // divergences from estimates that are all zero are zero (pixel_kl's r2 = 0)
+  const bool kl_on = *nonzero != 0;
   for (int i = tid; i < n2; i += kThreads) {
     const int y = i / kTile, x = i - y * kTile;
     const size_t o = (size_t)clampn(h0 + y, 0, g.H - 1) * g.W + clampn(w0 + x, 0, g.W - 1);
-    sA1[i] = a1[o];
-    sA2[i] = a2[o];
-    sDp[i] = dp[o];
-    sRf[i] = rf[o];
-    sPf[i] = pf[o];
-    sCf[i] = cf[o];
+    if (kl_on) {
+      sRf[i] = rf[o];
+      sPf[i] = pf[o];
+      sCf[i] = cf[o];
+    }
+    if (SIM) {
+      sA1[i] = a1[o];
+      sA2[i] = a2[o];
+      sDp[i] = dp[o];
+    }
   }
-  const int npix = g.hori * g.hori, nsim = g.hsim * g.hsim, nrow = g.hsim * g.hori;
-  float s1[kMaxPixPerThread], s2[kMaxPixPerThread];
-#pragma unroll
-  for (int q = 0; q < kMaxPixPerThread; ++q) s1[q] = s2[q] = 0.0f;
-  const int no = g.sws * g.sws, kc = g.wsh * g.sws + g.wsh;
-  float* wt = wout + (size_t)blockIdx.x * no * npix;
+  const int kc = z.wsh() * z.sws() + z.wsh();
+  const size_t base = (size_t)blockIdx.x * z.sws() * z.sws() * npix;
+  float* wt = wout + base;
+  float* st = sums ? sums + base : nullptr;
   __syncthreads();
+  // similarity and divergence of grid position i's pixel pair (c, q)
+  auto evaluate = [&](int c, int q, float* s, float* k, int i) {
+    if (SIM) s[i] = pixel_sim(sA1[c], sA2[c], sDp[c], sA1[q], sA2[q], sDp[q]);
+    if (kl_on) k[i] = pixel_kl(sRf[c], sPf[c], sCf[c], sRf[q], sPf[q], sCf[q]);
+  };
   // similarities and divergences of offset (hh, ww) on the whole grid, with
   // the two pixels swapped in the interior for the first wsh window rows (the
   // values the reference copies from the mirrored offset)
-  auto sims_direct = [&](int hh, int ww) {
+  auto direct = [&](int hh, int ww) {
     for (int it = tid; it < nsim; it += kThreads) {
-      const int h = it / g.hsim, w = it - h * g.hsim;
-      const bool interior = h >= g.wsh && w >= g.wsh && w < g.hsim - g.wsh;
-      int c = (h + g.wsh) * kTile + (w + g.wsh), q = (h + hh) * kTile + (w + ww);
-      if (interior && hh < g.wsh) {
-        const int t = c;
-        c = q;
-        q = t;
-      }
-      sS[it] = pixel_sim(sA1[c], sA2[c], sDp[c], sA1[q], sA2[q], sDp[q]);
-      sK[it] = pixel_kl(sRf[c], sPf[c], sCf[c], sRf[q], sPf[q], sCf[q]);
+      const int h = it / z.hsim(), w = it - h * z.hsim();
+      const bool interior = h >= z.wsh() && w >= z.wsh() && w < z.hsim() - z.wsh();
+      const int c = (h + z.wsh()) * kTile + (w + z.wsh()), q = (h + hh) * kTile + (w + ww);
+      const bool swap = interior && hh < z.wsh();
+      evaluate(swap ? q : c, swap ? c : q, sS, sK, it);
     }
   };
-  // p-wide row sums of a map given by `val(h, w)` (similarity, divergence)
-  auto row_sums = [&](auto val) {
-    for (int it = tid; it < nrow; it += kThreads) {
-      const int r = it / g.hori, col = it - r * g.hori;
-      float rs = 0.0f, rk = 0.0f;
-      for (int ky = 0; ky < g.p; ++ky) {
-        const float2 v = val(r, col + ky);
-        rs += v.x;
-        rk += v.y;
-      }
-      sRS[it] = rs;
-      sRK[it] = rk;
-    }
-  };
-  auto direct_val = [&](int h, int w) { return make_float2(sS[h * g.hsim + w], sK[h * g.hsim + w]); };
-  // p-wide column sums, weights and looks of offset k
-  auto weights_of = [&](int k) {
+  // p-wide row sums of the maps; `at(h, w)` gives a map's value.  An item is
+  // three adjacent sums from one load of their p + 2 values, each added left
+  // to right.
+  const int third = (z.hori() + 2) / 3;
+  auto row_sums = [&](auto at) {
+    for (int it = tid; it < z.hsim() * third; it += kThreads) {
+      const int r = it / third, col = 3 * (it - r * third);
+      float rs[3] = {0.0f, 0.0f, 0.0f}, rk[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
-    for (int q = 0; q < kMaxPixPerThread; ++q) {
-      const int pix = tid + q * kThreads;
-      if (pix < npix) {
-        const int x = pix / g.hori, y = pix - x * g.hori;
-        float s = sRS[x * g.hori + y], kl = sRK[x * g.hori + y];
-        for (int kx = 1; kx < g.p; ++kx) {
-          s += sRS[(x + kx) * g.hori + y];
-          kl += sRK[(x + kx) * g.hori + y];
+      for (int ky = 0; ky < z.p() + 2; ++ky) {
+        if (col + ky >= z.hsim()) break;
+        const float vs = SIM ? at(sS, sBS, r, col + ky) : 0.0f, vk = kl_on ? at(sK, sBK, r, col + ky) : 0.0f;
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+          if (ky >= e && ky < z.p() + e) {
+            if (SIM) rs[e] += vs;
+            rk[e] += vk;
+          }
+      }
+#pragma unroll
+      for (int e = 0; e < 3; ++e)
+        if (col + e < z.hori()) {
+          if (SIM) sRS[r * z.hori() + col + e] = rs[e];
+          if (kl_on) sRK[r * z.hori() + col + e] = rk[e];
         }
-        float wv = expf(s / g.h + kl / g.T);
+    }
+  };
+  auto direct_at = [&](const float* m, const float*, int h, int w) { return m[h * z.hsim() + w]; };
+  // p-wide column sums and weights of offset k; an item is three rows of a
+  // column, each sum added top down
+  auto weights_of = [&](int k) {
+    for (int it = tid; it < z.hori() * third; it += kThreads) {
+      const int x3 = it / z.hori(), y = it - x3 * z.hori(), x = 3 * x3;
+      float s[3], kl[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int kx = 0; kx < z.p() + 2; ++kx) {
+        if (x + kx >= z.hsim()) break;
+        const float vs = SIM ? sRS[(x + kx) * z.hori() + y] : 0.0f, vk = kl_on ? sRK[(x + kx) * z.hori() + y] : 0.0f;
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+          if (SIM && kx == e) s[e] = vs;
+          if (SIM && kx > e && kx < z.p() + e) s[e] += vs;
+          if (kx == e) kl[e] = vk;
+          if (kx > e && kx < z.p() + e) kl[e] += vk;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        if (x + e >= z.hori()) break;
+        const size_t at = (size_t)k * npix + (x + e) * z.hori() + y;
+        float t;
+        if (SIM) {
+          t = s[e] / g.h;
+          if (st) st[at] = t;
+        } else {
+          t = st[at];
+        }
+        if (kl_on) t += kl[e] / g.T;
+        float wv = expf(t);
         if (isnan(wv) || isinf(wv)) wv = 0.0f;
         if (k == kc) wv = 0.0f;
-        wt[(size_t)k * npix + pix] = wv;
-        s1[q] += wv;
-        s2[q] += wv * wv;
+        wt[at] = wv;
       }
     }
   };
-  if (!g.mirror) {
-    for (int hh = 0; hh < g.sws; ++hh)
-      for (int ww = 0; ww < g.sws; ++ww) {
-        sims_direct(hh, ww);
-        __syncthreads();
-        row_sums(direct_val);
-        __syncthreads();
-        weights_of(hh * g.sws + ww);
-        __syncthreads();
-      }
-  } else {
-    // the centre window row, computed as the reference computes it
-    for (int ww = 0; ww < g.sws; ++ww) {
-      sims_direct(g.wsh, ww);
+  const int u0 = nl_group(g, blockIdx.y, gridDim.y), u1 = nl_group(g, blockIdx.y + 1, gridDim.y);
+  for (int u = u0; u < u1; ++u) {
+    if (!g.mirror || u < z.sws()) {
+      // an offset of the centre window row (or any one, without mirrors),
+      // computed as the reference computes it
+      const int hh = g.mirror ? z.wsh() : u / z.sws(), ww = g.mirror ? u : u - hh * z.sws();
+      direct(hh, ww);
       __syncthreads();
-      row_sums(direct_val);
+      row_sums(direct_at);
       __syncthreads();
-      weights_of(g.wsh * g.sws + ww);
+      weights_of(hh * z.sws() + ww);
       __syncthreads();
+      continue;
     }
-    // every lower-row offset with its mirror: the mirror's interior values are
-    // the lower offset's maps shifted by the mirror's offset (the very values
-    // the reference copies), its border values are computed here
-    float* sBS = sRK + nrow;  // mirror's border: similarity, divergence
-    float* sBK = sBS + g.nborder;
-    const int top = g.wsh * g.hsim, band = 2 * g.wsh;
-    for (int hl = g.wsh + 1; hl < g.sws; ++hl)
-      for (int wl = 0; wl < g.sws; ++wl) {
-        const int hu = 2 * g.wsh - hl, wu = 2 * g.wsh - wl;
-        for (int it = tid; it < nsim + g.nborder; it += kThreads) {
-          int c, q;
-          if (it < nsim) {
-            const int h = it / g.hsim, w = it - h * g.hsim;
-            c = (h + g.wsh) * kTile + (w + g.wsh);
-            q = (h + hl) * kTile + (w + wl);
-            sS[it] = pixel_sim(sA1[c], sA2[c], sDp[c], sA1[q], sA2[q], sDp[q]);
-            sK[it] = pixel_kl(sRf[c], sPf[c], sCf[c], sRf[q], sPf[q], sCf[q]);
-          } else {
-            const int ib = it - nsim;
-            int h, w;
-            if (ib < top) {
-              h = ib / g.hsim;
-              w = ib - h * g.hsim;
-            } else {
-              const int j = ib - top;
-              h = g.wsh + j / band;
-              const int m = j - (j / band) * band;
-              w = m < g.wsh ? m : g.hsim - band + m;
-            }
-            c = (h + g.wsh) * kTile + (w + g.wsh);
-            q = (h + hu) * kTile + (w + wu);
-            sBS[ib] = pixel_sim(sA1[c], sA2[c], sDp[c], sA1[q], sA2[q], sDp[q]);
-            sBK[ib] = pixel_kl(sRf[c], sPf[c], sCf[c], sRf[q], sPf[q], sCf[q]);
-          }
+    // a lower-row offset with its mirror: the mirror's interior values are the
+    // lower offset's maps shifted by the mirror's offset (the very values the
+    // reference copies), its border values are computed here
+    const int v = u - z.sws();
+    const int hl = z.wsh() + 1 + v / z.sws(), wl = v % z.sws();
+    const int hu = 2 * z.wsh() - hl, wu = 2 * z.wsh() - wl;
+    const int top = z.wsh() * z.hsim(), band = 2 * z.wsh();
+    for (int it = tid; it < nsim + nborder; it += kThreads) {
+      if (it < nsim) {
+        const int h = it / z.hsim(), w = it - h * z.hsim();
+        evaluate((h + z.wsh()) * kTile + (w + z.wsh()), (h + hl) * kTile + (w + wl), sS, sK, it);
+      } else {
+        const int ib = it - nsim;
+        int h, w;
+        if (ib < top) {
+          h = ib / z.hsim();
+          w = ib - h * z.hsim();
+        } else {
+          const int j = ib - top;
+          h = z.wsh() + j / band;
+          const int m = j - (j / band) * band;
+          w = m < z.wsh() ? m : z.hsim() - band + m;
         }
-        __syncthreads();
-        row_sums(direct_val);
-        __syncthreads();
-        weights_of(hl * g.sws + wl);
-        __syncthreads();
-        const int dh = hu - g.wsh, dw = wu - g.wsh;
-        row_sums([&](int h, int w) {
-          if (h >= g.wsh && w >= g.wsh && w < g.hsim - g.wsh) {
-            const int i = (h + dh) * g.hsim + (w + dw);
-            return make_float2(sS[i], sK[i]);
-          }
-          const int ib = h < g.wsh ? h * g.hsim + w : top + (h - g.wsh) * band + (w < g.wsh ? w : w - g.hsim + band);
-          return make_float2(sBS[ib], sBK[ib]);
-        });
-        __syncthreads();
-        weights_of(hu * g.sws + wu);
-        __syncthreads();
+        evaluate((h + z.wsh()) * kTile + (w + z.wsh()), (h + hu) * kTile + (w + wu), sBS, sBK, ib);
       }
+    }
+    __syncthreads();
+    row_sums(direct_at);
+    __syncthreads();
+    weights_of(hl * z.sws() + wl);
+    __syncthreads();
+    const int dh = hu - z.wsh(), dw = wu - z.wsh();
+    row_sums([&](const float* m, const float* border, int h, int w) {
+      if (h >= z.wsh() && w >= z.wsh() && w < z.hsim() - z.wsh()) return m[(h + dh) * z.hsim() + (w + dw)];
+      return border[h < z.wsh() ? h * z.hsim() + w
+                                : top + (h - z.wsh()) * band + (w < z.wsh() ? w : w - z.hsim() + band)];
+    });
+    __syncthreads();
+    weights_of(hu * z.sws() + wu);
+    __syncthreads();
   }
-#pragma unroll
-  for (int q = 0; q < kMaxPixPerThread; ++q) {
-    const int pix = tid + q * kThreads;
-    if (pix < npix) nols[(size_t)blockIdx.x * npix + pix] = s1[q] * s1[q] / s2[q];
-  }
+}
+
+// whether any reflectivity estimate is not zero
+__global__ void nlinsar_nonzero_kernel(const float* __restrict__ rf, size_t n, int* __restrict__ nonzero) {
+  bool any = false;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    any = any || !(rf[i] == 0.0f);
+  if (__syncthreads_or(any) && threadIdx.x == 0) *nonzero = 1;
 }
 
 // std::priority_queue<weight_el> of smoothing.cpp: a binary heap whose top is
@@ -320,7 +383,7 @@ __global__ void __launch_bounds__(kEstThreads)
                             const float* __restrict__ fi, const float* __restrict__ prf,
                             const float* __restrict__ ppf, const float* __restrict__ pcf, float* __restrict__ orf,
                             float* __restrict__ opf, float* __restrict__ ocf, NlGeom g, int tile0,
-                            const float* __restrict__ wts, const float* __restrict__ nols) {
+                            const float* __restrict__ wts) {
   const int npix = g.hori * g.hori;
   const int pix = blockIdx.x * kEstThreads + threadIdx.x;
   if (pix >= npix) return;
@@ -339,11 +402,30 @@ __global__ void __launch_bounds__(kEstThreads)
   else return;
   const int no = g.sws * g.sws;
   const float* wp = wts + (size_t)blockIdx.y * no * npix + pix;
+  // looks, the weights in the order of the weights kernel's units
+  float s1 = 0.0f, s2 = 0.0f;
+  auto look = [&](int k) {
+    const float wv = wp[(size_t)k * npix];
+    s1 += wv;
+    s2 += wv * wv;
+  };
+  if (!g.mirror) {
+#pragma unroll 4
+    for (int k = 0; k < no; ++k) look(k);
+  } else {
+#pragma unroll 4
+    for (int ww = 0; ww < g.sws; ++ww) look(g.wsh * g.sws + ww);
+#pragma unroll 4
+    for (int k = (g.wsh + 1) * g.sws; k < no; ++k) {
+      look(k);
+      look(no - 1 - k);  // the mirror
+    }
+  }
   // smoothing (smoothing.cpp:65-117)
   int sel[kMaxLmin];
   int nsel = 0;
   float wmean = 0.0f;
-  if (nols[(size_t)blockIdx.y * npix + pix] < (float)g.lmin) {
+  if (s1 * s1 / s2 < (float)g.lmin) {
     DevHeap hp;
     const double as = a1[(size_t)clampn(h0 + x + g.ov, 0, g.H - 1) * g.W + clampn(w0 + y + g.ov, 0, g.W - 1)];
     for (int hh = 0; hh < g.sws; ++hh) {
@@ -413,10 +495,9 @@ __global__ void __launch_bounds__(kEstThreads)
   ocf[o] = valid(coh) ? fminf(1.0f, fmaxf(0.0f, coh)) : pcf[o];
 }
 
-size_t weights_smem(const NlGeom& g) {
-  return ((size_t)6 * kTile * kTile + 2 * (size_t)g.hsim * g.hsim + 2 * (size_t)g.hsim * g.hori +
-          (g.mirror ? 2 * (size_t)g.nborder : 0)) *
-         sizeof(float);
+size_t weights_smem(const NlGeom& g, bool sim) {
+  const size_t maps = (size_t)g.hsim * g.hsim + (size_t)g.hsim * g.hori + (g.mirror ? (size_t)g.nborder : 0);
+  return ((sim ? 6 : 3) * (size_t)kTile * kTile + (sim ? 2 : 1) * maps) * sizeof(float);
 }
 
 int nlinsar_geom(int H, int W, int sws, int p, int lmin, NlGeom& g) {
@@ -442,9 +523,9 @@ int nlinsar_geom(int H, int W, int sws, int p, int lmin, NlGeom& g) {
   // and room for the mirror's border values
   g.nborder = g.wsh * g.hsim + (g.hsim - g.wsh) * 2 * g.wsh;
   g.mirror = 2 * g.wsh < g.hsim ? 1 : 0;
-  if (g.mirror && weights_smem(g) > 227 * 1024) g.mirror = 0;
+  if (g.mirror && weights_smem(g, true) > 227 * 1024) g.mirror = 0;
   if (g.hori < 1) return set_error(DCL_ERR_UNSUPPORTED, "search window and patch too large for the 80 x 80 tiles");
-  if ((g.hori * g.hori + kThreads - 1) / kThreads > kMaxPixPerThread || weights_smem(g) > 227 * 1024)
+  if (g.hori * g.hori > 6 * 1024 || weights_smem(g, true) > 227 * 1024)
     return set_error(DCL_ERR_UNSUPPORTED, "search window %d with patch %d: tile state exceeds shared memory", sws, p);
   g.step = kTile - 2 * g.ov;
   g.nty = 0;
@@ -459,6 +540,42 @@ int nlinsar_geom(int H, int W, int sws, int p, int lmin, NlGeom& g) {
   return DCL_OK;
 }
 
+template <class Z, bool SIM>
+cudaError_t launch_weights_t(const float* a1, const float* a2, const float* dp, float* const* est, const NlGeom& g,
+                             int tile0, int tiles, int groups, const int* nonzero, float* sums, float* wts,
+                             cudaStream_t st) {
+  static size_t allowed[kMaxDevices];
+  const size_t smem = weights_smem(g, SIM);
+  const cudaError_t e = allow_dynamic_smem((const void*)nlinsar_weights_kernel<Z, SIM>, smem, allowed);
+  if (e != cudaSuccess) return e;
+  nlinsar_weights_kernel<Z, SIM><<<dim3(tiles, groups), weights_threads(SIM), smem, st>>>(a1, a2, dp, est[0], est[1], est[2], g,
+                                                                            tile0, nonzero, sums, wts);
+  return cudaGetLastError();
+}
+
+template <bool SIM>
+cudaError_t launch_weights(const float* a1, const float* a2, const float* dp, float* const* est, const NlGeom& g,
+                           int tile0, int tiles, const int* nonzero, float* sums, float* wts, int sms,
+                           cudaStream_t st) {
+  // Groups of offsets per tile: waves of blocks (one or two per SM) times a block's
+  // time, its share of a tile's work (about 4 ms) and staging (about 8 us).
+  // One block per tile left 168 tiles of a 600 x 700 scene in two waves.
+  int groups = 1;
+  double best = 0.0;
+  for (int z = 1; z <= std::min(64, nl_units(g)); ++z) {
+    const int at_once = sms * (SIM ? 1 : 2);
+    const double t = (double)(((long long)tiles * z + at_once - 1) / at_once) * (4000.0 / z + 8.0);
+    if (best == 0.0 || t < best) {
+      best = t;
+      groups = z;
+    }
+  }
+  auto go = [&](auto launch) { return launch(a1, a2, dp, est, g, tile0, tiles, groups, nonzero, sums, wts, st); };
+  if (g.sws == 21 && g.p == 7) return go(launch_weights_t<NlSizes<21, 7>, SIM>);
+  if (g.sws == 21 && g.p == 3) return go(launch_weights_t<NlSizes<21, 3>, SIM>);
+  return go(launch_weights_t<NlSizes<0, 0>, SIM>);
+}
+
 }  // namespace
 
 int nlinsar_check(int H, int W, int sws, int p, int lmin) {
@@ -471,11 +588,9 @@ int nlinsar_device(const float* a1, const float* a2, const float* dp, float* ref
                    int W, int sws, int p, int niter, int lmin, cudaStream_t st) {
   if (!a1 || !a2 || !dp || !ref || !phase || !coh) return set_error(DCL_ERR_INVALID_ARGUMENT, "null pointer");
   if (niter < 0) return set_error(DCL_ERR_INVALID_ARGUMENT, "niter must be >= 0");
-  {
-    int dev = 0;
-    const int rc0 = ensure_device_ready(dev);
-    if (rc0) return rc0;
-  }
+  int dev = 0;
+  const int rc0 = ensure_device_ready(dev);
+  if (rc0) return rc0;
   NlGeom g;
   int rc = nlinsar_geom(H, W, sws, p, lmin, g);
   if (rc) return rc;
@@ -483,32 +598,47 @@ int nlinsar_device(const float* a1, const float* a2, const float* dp, float* ref
   const size_t n = (size_t)H * W;
   const int ntiles = g.ntx * g.nty;
   const size_t npix = (size_t)g.hori * g.hori, no = (size_t)sws * sws;
-  const size_t per_tile = (no * npix + npix) * sizeof(float);
-  const int chunk = (int)std::max<size_t>(1, std::min<size_t>(ntiles, ((size_t)4 << 30) / per_tile));
-  float* buf = nullptr;
-  cudaError_t e = cudaMallocAsync(&buf, (6 * n) * sizeof(float) + (size_t)chunk * per_tile, st);
+  const size_t per_tile = no * npix * sizeof(float);
+  const int chunk = (int)std::max<size_t>(1, std::min<size_t>(ntiles, kWeightsBytes / per_tile));
+  // the first pass's patch sums of the similarities, where the later passes
+  // can keep them (a second scratch of at most the weights' size)
+  const size_t sum_bytes = niter > 1 && chunk == ntiles ? (size_t)ntiles * per_tile : 0;
+  char* buf = nullptr;
+  const size_t fixed = 6 * n * sizeof(float) + 256 + (size_t)chunk * per_tile;
+  cudaError_t e = cudaMallocAsync(&buf, fixed + sum_bytes, st);
+  bool keep = sum_bytes > 0;
+  if (e == cudaErrorMemoryAllocation && keep) {
+    cudaGetLastError();
+    keep = false;
+    e = cudaMallocAsync(&buf, fixed, st);
+  }
   if (e != cudaSuccess) return cuda_error(e, "cudaMallocAsync(NL-InSAR)");
-  float *fa = buf, *fr = fa + n, *fi = fr + n, *tr = fi + n, *tp = tr + n, *tc = tp + n;
+  int* nonzero = reinterpret_cast<int*>(buf);
+  float* fa = reinterpret_cast<float*>(buf + 256);
+  float *fr = fa + n, *fi = fr + n, *tr = fi + n, *tp = tr + n, *tc = tp + n;
   float* wts = tc + n;
-  float* nols = wts + (size_t)chunk * no * npix;
-  const size_t smem = weights_smem(g);
-  e = cudaFuncSetAttribute(nlinsar_weights_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  float* sums = keep ? wts + (size_t)chunk * no * npix : nullptr;
+  e = cudaMemsetAsync(nonzero, 0, sizeof(int), st);
   if (e == cudaSuccess) {
+    const int sms = sm_count(dev);
     nlinsar_filter_values_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a1, a2, dp, fa, fr, fi, n);
     profile_count(1);
     // estimates ping-pong between the caller's planes and tr/tp/tc; an odd
     // number of passes ends in tr/tp/tc and is copied back
     float* cur[3] = {ref, phase, coh};
     float* nxt[3] = {tr, tp, tc};
-    for (int it = 0; it < niter; ++it) {
-      for (int t0 = 0; t0 < ntiles; t0 += chunk) {
+    for (int it = 0; it < niter && e == cudaSuccess; ++it) {
+      nlinsar_nonzero_kernel<<<(unsigned)std::min<size_t>((n + 1023) / 1024, 8 * sms), 256, 0, st>>>(cur[0], n, nonzero);
+      for (int t0 = 0; t0 < ntiles && e == cudaSuccess; t0 += chunk) {
         const int nt = std::min(chunk, ntiles - t0);
-        nlinsar_weights_kernel<<<nt, kThreads, smem, st>>>(a1, a2, dp, cur[0], cur[1], cur[2], g, t0, wts, nols);
+        e = keep && it > 0 ? launch_weights<false>(a1, a2, dp, cur, g, t0, nt, nonzero, sums, wts, sms, st)
+                           : launch_weights<true>(a1, a2, dp, cur, g, t0, nt, nonzero, sums, wts, sms, st);
         dim3 grid((unsigned)((npix + kEstThreads - 1) / kEstThreads), nt);
         nlinsar_estimate_kernel<<<grid, kEstThreads, 0, st>>>(a1, fa, fr, fi, cur[0], cur[1], cur[2], nxt[0], nxt[1],
-                                                              nxt[2], g, t0, wts, nols);
+                                                              nxt[2], g, t0, wts);
         profile_count(2);
       }
+      profile_count(1);
       std::swap(cur, nxt);
     }
     if (cur[0] != ref)

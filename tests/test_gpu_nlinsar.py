@@ -78,3 +78,18 @@ def test_host_entry_point_equals_device_entry_point():
     dev = _gpu(a1, a2, ph, 2, 10)
     for h, d in zip(host, dev):
         assert np.array_equal(h, d)
+
+
+@pytest.mark.parametrize("shape,sws,patch", [((54, 54), 21, 7), ((55, 109), 21, 7), ((70, 60), 21, 3), ((64, 75), 15, 7),
+                                             ((60, 61), 31, 3), ((40, 50), 41, 7)])
+def test_passes_of_one_call_equal_single_pass_calls(shape, sws, patch):
+    # a call of several passes keeps the first pass's similarity sums and skips
+    # the divergences of zero estimates; single-pass calls evaluate all of them
+    t = [torch.from_numpy(x).cuda() for x in synthetic.insar_scene(*shape, 31)]
+    whole = dcl.nlinsar_device(*t, sws, patch, 3, 10)
+    est = None
+    for _ in range(3):
+        est = dcl.nlinsar_device(*t, sws, patch, 1, 10, estimates=est)
+    torch.cuda.synchronize()
+    for a, b in zip(whole, est):
+        np.testing.assert_array_equal(a.cpu().numpy(), b.cpu().numpy())
