@@ -18,6 +18,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <utility>
 #include <vector>
 
@@ -639,14 +640,18 @@ int host_pipe(int dev, size_t nev, HostPipe*& out) {
   return DCL_OK;
 }
 
-constexpr int kMaxBands = 8;   // row bands of a host-pointer call
-constexpr int kBandWaves = 8;  // fewest waves of tiles (one CTA per SM) per band: each band's launch
-                               // ends in a partly filled wave, so small scenes stay in one band
+constexpr int kMaxBands = 8;  // row bands of a host-pointer call
+// Fewest waves of tiles (one CTA per SM) per band: each band's launch ends in
+// a partly filled wave, so small scenes stay in one band.  Pageable planes of
+// kStageBytes in all or more go through pinned slots, which leaves more time
+// to hide behind smaller bands.
+constexpr int kStagedWaves = 4;
+constexpr size_t kStageBytes = size_t(8) << 20;
 
-int band_count(int dev, long long tiles, int tile_rows) {
+int band_count(int dev, long long tiles, int tile_rows, int waves) {
   const int sms = sm_count(dev);
   int nb = (int)std::max(1LL, std::min<long long>(std::min(kMaxBands, tile_rows),
-                                                  tiles / ((long long)kBandWaves * sms)));
+                                                  tiles / ((long long)waves * sms)));
   // DESPECKCL_B200_BANDS=n forces n bands (at most one per tile row): the
   // tests use it to cut small scenes
   if (const char* fb = std::getenv("DESPECKCL_B200_BANDS")) {
@@ -686,10 +691,22 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
   pl.P.K = K;
   const SceneGeom g = scene_geom(pl, H, W);
   if ((long long)g.tiles_x * g.tiles_y > 0x7fffffff) return set_error(DCL_ERR_INVALID_ARGUMENT, "scene too large");
-  const int nb = band_count(dev, (long long)g.tiles_x * g.tiles_y, g.tiles_y);
+  // pageable planes: the driver's own staging copies them one after another
+  // on the calling thread (about 10 GB/s, and page faults of fresh outputs
+  // with it); large ones go through pinned slots, copied by several threads
+  bool staged = (size_t)(nin + nout) * H * W * sizeof(float) >= kStageBytes;
+  for (int i = 0; i < nin && staged; ++i) staged = is_pageable(hin[i]);
+  for (int i = 0; i < nout && staged; ++i) staged = is_pageable(hout[i]);
   HostPipe* hp = nullptr;
+  rc = host_pipe(dev, 2 * (size_t)kMaxBands + 2, hp);
+  if (rc) return rc;
+  staged = staged && hp->in.ready() && hp->out.ready();
+  const int nb = band_count(dev, (long long)g.tiles_x * g.tiles_y, g.tiles_y, staged ? kStagedWaves : 8);
   rc = host_pipe(dev, 2 * (size_t)nb + 2, hp);
   if (rc) return rc;
+  // 3 to 7 helpers measured alike, more slower (1531 x 1999: 5.6 - 6.2 ms,
+  // with 15 7.3 - 7.7; 10.3 ms through the driver's staging)
+  CopyCrew crew(staged ? std::max(1, std::min(4, (int)std::thread::hardware_concurrency() - 1)) : 0);
   cudaEvent_t* ev_in = hp->ev.data();       // band inputs uploaded
   cudaEvent_t* ev_out = hp->ev.data() + nb;  // band results written
   cudaEvent_t ev_alloc = hp->ev[2 * nb], ev_done = hp->ev[2 * nb + 1];
@@ -777,7 +794,7 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
   pl.P.timeouts = d_timeouts;
 
   const int TH = pl.P.tile_h, G = pl.P.G;
-  int in_done = 0, co_done = 0, cs_done = 0;
+  int in_done = 0, co_done = 0, cs_done = 0, slot = 0;
   for (int i = 0; i < nb && rc == DCL_OK; ++i) {
     const bool last = i == nb - 1;
     // frame rows the band's tiles read (scaled covariance: tile + patch and
@@ -788,8 +805,22 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
     const int in_need = last ? H : std::max(1, std::min(H, co_need - G));
     if (in_need > in_done) {
       const size_t off = (size_t)in_done * W, cnt = (size_t)(in_need - in_done) * W * sizeof(float);
-      for (int p = 0; p < nin && e == cudaSuccess; ++p)
-        e = cudaMemcpyAsync(buf + p * n + off, hin[p] + off, cnt, cudaMemcpyHostToDevice, hp->h2d);
+      for (int p = 0; p < nin && e == cudaSuccess; ++p) {
+        if (!staged) {
+          e = cudaMemcpyAsync(buf + p * n + off, hin[p] + off, cnt, cudaMemcpyHostToDevice, hp->h2d);
+          continue;
+        }
+        for (size_t at = 0; at < cnt && e == cudaSuccess; at += PinnedSlots::kSlotBytes, ++slot) {
+          const size_t len = std::min(PinnedSlots::kSlotBytes, cnt - at);
+          cudaEvent_t free_ev = hp->in.ev[slot % PinnedSlots::kSlots];
+          if (slot >= PinnedSlots::kSlots) e = cudaEventSynchronize(free_ev);
+          if (e != cudaSuccess) break;
+          crew.copy(hp->in.slot(slot), reinterpret_cast<const char*>(hin[p] + off) + at, len);
+          e = cudaMemcpyAsync(reinterpret_cast<char*>(buf + p * n + off) + at, hp->in.slot(slot), len,
+                              cudaMemcpyHostToDevice, hp->h2d);
+          if (e == cudaSuccess) e = cudaEventRecord(free_ev, hp->h2d);
+        }
+      }
       in_done = in_need;
     }
     if (e == cudaSuccess) e = cudaEventRecord(ev_in[i], hp->h2d);
@@ -815,15 +846,44 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
   }
   // results: band b holds output rows [tb[b] * TH, tb[b+1] * TH) below row
   // H-1; row H-1 comes from the last tile row (virtual row H-1+overlap)
+  struct Down {
+    char* to;
+    size_t bytes;
+  };
+  std::vector<Down> down;  // staged: the pieces in the slots, oldest first
+  size_t landed = 0;
+  auto land = [&](size_t upto) {
+    for (; landed < upto && e == cudaSuccess; ++landed) {
+      e = cudaEventSynchronize(hp->out.ev[landed % PinnedSlots::kSlots]);
+      if (e == cudaSuccess) crew.copy(down[landed].to, hp->out.slot((int)landed), down[landed].bytes);
+    }
+  };
   for (int i = 0; i < nb && rc == DCL_OK; ++i) {
     const int r0 = std::min(tb[i] * TH, H - 1);
     const int r1 = i == nb - 1 ? H : std::min(tb[i + 1] * TH, H - 1);
     e = cudaStreamWaitEvent(hp->d2h, ev_out[i], 0);
     if (r1 > r0) {
       const size_t off = (size_t)r0 * W, cnt = (size_t)(r1 - r0) * W * sizeof(float);
-      for (int p = 0; p < nout && e == cudaSuccess; ++p)
-        e = cudaMemcpyAsync(hout[p] + off, dout + p * n + off, cnt, cudaMemcpyDeviceToHost, hp->d2h);
+      for (int p = 0; p < nout && e == cudaSuccess; ++p) {
+        if (!staged) {
+          e = cudaMemcpyAsync(hout[p] + off, dout + p * n + off, cnt, cudaMemcpyDeviceToHost, hp->d2h);
+          continue;
+        }
+        for (size_t at = 0; at < cnt && e == cudaSuccess; at += PinnedSlots::kSlotBytes) {
+          const size_t len = std::min(PinnedSlots::kSlotBytes, cnt - at), k = down.size();
+          if (k >= PinnedSlots::kSlots) land(k - PinnedSlots::kSlots + 1);
+          if (e != cudaSuccess) break;
+          down.push_back({reinterpret_cast<char*>(hout[p] + off) + at, len});
+          e = cudaMemcpyAsync(hp->out.slot((int)k), reinterpret_cast<const char*>(dout + p * n + off) + at, len,
+                              cudaMemcpyDeviceToHost, hp->d2h);
+          if (e == cudaSuccess) e = cudaEventRecord(hp->out.ev[k % PinnedSlots::kSlots], hp->d2h);
+        }
+      }
     }
+    if (e != cudaSuccess) rc = cuda_error(e, "cudaMemcpyAsync(D2H)");
+  }
+  if (rc == DCL_OK) {
+    land(down.size());
     if (e != cudaSuccess) rc = cuda_error(e, "cudaMemcpyAsync(D2H)");
   }
   // the buffers are freed in stream order after every copy that uses them

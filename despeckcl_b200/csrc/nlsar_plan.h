@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../include/despeckcl_b200.h"
+#include "host_copy.h"
 #include "nlsar_common.cuh"
 
 namespace dcl {
@@ -52,11 +53,12 @@ struct HostPipe {
   cudaStream_t h2d = nullptr, d2h = nullptr;
   std::vector<cudaEvent_t> ev;
   int* h_timeouts = nullptr;  // pinned: the last call's staging-timeout count
+  PinnedSlots in, out;        // staging of pageable planes
 };
 int host_pipe(int dev, size_t nev, HostPipe*& out);
 // Row bands of a host-pointer call over `tiles` tiles in `tile_rows` rows
-// (DESPECKCL_B200_BANDS overrides).
-int band_count(int dev, long long tiles, int tile_rows);
+// (DESPECKCL_B200_BANDS overrides), of at least `waves` waves of tiles each.
+int band_count(int dev, long long tiles, int tile_rows, int waves = 8);
 // NL-SAR of a 3x3 covariance scene [18][H][W] (nlsar_dim3.cu): device
 // pointers on `st`, or host pointers (copied in and out, synchronous)
 int nlsar_covmat3_device(const Plan& pl, const float* cin, float* cout, int H, int W, cudaStream_t st);
