@@ -6,7 +6,9 @@
 // One pass over HBM: each CTA stages its output tile plus a (w-1)/2 halo of
 // (I, Re, Im) = ((a1^2+a2^2)/2, a1 a2 cos phi, a1 a2 sin phi) in shared memory,
 // forms horizontal window sums, then vertical sums, and writes
-// ref = mean I, phase = atan2(Im, Re), coh = |sum Re + j Im| / sum I.
+// ref = mean I, phase = atan2(Im, Re), coh = |sum Re + j Im| / sum I.  On large
+// scenes with windows up to 7 x 7 warps walk down the scene instead, the sums
+// in registers (boxcar_walk_kernel).
 //
 // Like NL-SAR, the reference's clamped tile write-back puts the result of
 // virtual row H-1+(w-1)/2 of the clamp-extended image into output row H-1
@@ -91,6 +93,14 @@ __global__ void __launch_bounds__(kBoxThreads)
     phase[o] = atan2_fast(sj, sr);
     coh[o] = sqrtf(sr * sr + sj * sj) / si;
   }
+}
+
+// |sum| / sum I from 2 I sums, with the hardware square root and the fast
+// division (a few ulps, against the 1e-4 relative tolerance of the coherence)
+__device__ __forceinline__ float boxcar_coherence(float sr, float sj, float si) {
+  float m;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(m) : "f"(__fmaf_rn(sr, sr, __fmul_rn(sj, sj))));
+  return __fdividef(2.0f * m, si);
 }
 
 // Packed and scalar adds for the window sums: (Re, Im) pairs are summed two
@@ -325,11 +335,7 @@ __global__ void __launch_bounds__(kBoxThreads)
       const float sr = sZc[e][q].x, sj = sZc[e][q].y;
       o_r[e] = si * inv_2n;
       o_p[e] = atan2_fast(sj, sr);
-      // |sum| / sum I with the hardware square root and the fast division
-      // (a few ulps, against the 1e-4 relative tolerance of the coherence)
-      float m;
-      asm("sqrt.approx.f32 %0, %1;" : "=f"(m) : "f"(sr * sr + sj * sj));
-      o_c[e] = __fdividef(2.0f * m, si);
+      o_c[e] = boxcar_coherence(sr, sj, si);
     }
     const size_t rowo = (size_t)oy * W;
     if (cols_plain && vec_out) {
@@ -348,6 +354,247 @@ __global__ void __launch_bounds__(kBoxThreads)
       }
     }
   }
+}
+
+// Window radius 1 <= R <= 3 on large scenes: a warp walks down a strip of 128
+// columns, each lane owning four adjacent ones.  The pixels of a row come by
+// asynchronous copies, one 16-byte vector per lane and plane, into the warp's
+// ring in shared memory a few rows ahead; the R columns on either side come
+// from the neighbour lanes by shuffles (the strip's outer lanes only supply
+// them); the horizontal sums of the last 2 R rows stay in registers, and each
+// row of windows is written as soon as its last row has come in.  The sums are
+// those of boxcar_r_kernel in the same order (its items are four columns of I,
+// two of (Re, Im) and four rows, from the same origins), so the results are
+// the same bits.
+//
+// VEC: all planes and rows are 16-byte aligned.  Otherwise, and at the scene's
+// edges, the copies are single values, 32 adjacent columns at a time, and the
+// results reach memory the same way through shared memory.
+//
+// 8192 x 8192, 7 x 7: the tiled kernel takes 438 us, bound by shared memory
+// (79 %) and issue (137 thread instructions per pixel); this one takes
+// 312 us (5.1 TB/s of the six planes) at 98 instructions per pixel.  Registers
+// set its pace: 158 of them and twelve warps per SM.  Held to 128 for sixteen
+// warps it spills and takes 530 us or more; with all rows of a group summed
+// before the first output it needs 218 and takes 425 us.  A ring of eight rows
+// takes 330 us, walks of 128 rows 334 us, of 32 rows 325 us.
+constexpr int kWalkWarps = 4;
+constexpr int kWalkCols = 120;  // columns a warp outputs
+constexpr int kWalkRing = 4;   // rows in flight per warp
+constexpr int kWalkBlocks = 3;  // per SM
+constexpr int kWalkGroups = 16;  // groups of four rows a warp outputs at most
+
+template <int R, bool VEC>
+__global__ void __launch_bounds__(32 * kWalkWarps, kWalkBlocks)
+    boxcar_walk_kernel(const float* __restrict__ a1, const float* __restrict__ a2, const float* __restrict__ phi,
+                       float* __restrict__ ref, float* __restrict__ phase, float* __restrict__ coh, int H, int W,
+                       int groups) {
+  static_assert(R >= 1 && R <= 3, "registers; the halo comes from one neighbour lane");
+  constexpr int w = 2 * R + 1;
+  const int lane = threadIdx.x & 31;
+  const int xs = (int)(blockIdx.x * kWalkWarps + (threadIdx.x >> 5)) * kWalkCols - 4;  // the strip's first column
+  const int x0 = xs + 4 * lane;
+  const int vW = W - 1 + R, vH = H - 1 + R;
+  if (xs + 4 > vW) return;  // whole warp
+  const int y0 = (int)blockIdx.y * groups * 4;
+  const bool inside = xs >= 0 && xs + 128 <= W;
+  const bool plain = xs + 124 < W;  // all output columns map to themselves
+  const bool writes = lane >= 1 && lane <= 30;
+  const float inv_2n = 0.5f / (float)(w * w);
+
+  __shared__ __align__(16) float ring_s[kWalkWarps][kWalkRing][3][128];
+  __shared__ __align__(16) float out_s[VEC ? 1 : kWalkWarps][3][128];
+  float(*ring)[3][128] = ring_s[threadIdx.x >> 5];
+  int slot = 0;
+  int y = y0 - R;  // of the row to fetch next
+  auto fetch = [&] {
+    const size_t row = (size_t)clampi_b(y, 0, H - 1) * W;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      const float* src = (p == 0 ? a1 : p == 1 ? a2 : phi) + row;
+      const uint32_t d = (uint32_t)__cvta_generic_to_shared(&ring[slot][p][0]);
+      if (VEC && inside) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * lane), "l"(src + x0) : "memory");
+      } else if (inside) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 4 * lane + 128 * k),
+                       "l"(src + xs + lane + 32 * k)
+                       : "memory");
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 4 * lane + 128 * k),
+                       "l"(src + clampi_b(xs + lane + 32 * k, 0, W - 1))
+                       : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    ++y;
+    slot = slot + 1 == kWalkRing ? 0 : slot + 1;
+  };
+  struct Row {
+    float2 I[2];  // horizontal sums of 2 I, columns in pairs
+    float2 Z[4];  // and of (Re, Im)
+  };
+  // the horizontal sums of the next row, whose place takes the row kWalkRing
+  // further
+  auto next_row = [&](Row& h) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kWalkRing - 1) : "memory");
+    __syncwarp();  // every lane's copies
+    const float4 m4 = reinterpret_cast<const float4*>(ring[slot][0])[lane],
+                 s4 = reinterpret_cast<const float4*>(ring[slot][1])[lane],
+                 p4 = reinterpret_cast<const float4*>(ring[slot][2])[lane];
+    const float am[4] = {m4.x, m4.y, m4.z, m4.w};
+    const float as[4] = {s4.x, s4.y, s4.z, s4.w};
+    const float ph[4] = {p4.x, p4.y, p4.z, p4.w};
+    float v[4 + 2 * R];
+    float2 z[4 + 2 * R];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float sn, cs;
+      __sincosf(ph[c], &sn, &cs);
+      const float aa = am[c] * as[c];
+      // twice the intensity: the halving is folded into the output
+      v[R + c] = am[c] * am[c] + as[c] * as[c];
+      z[R + c] = make_float2(aa * cs, aa * sn);
+    }
+    __syncwarp();  // the row is read
+    fetch();
+#pragma unroll
+    for (int b = 1; b <= R; ++b) {
+      v[R - b] = __shfl_up_sync(0xffffffffu, v[R + 4 - b], 1);
+      v[R + 3 + b] = __shfl_down_sync(0xffffffffu, v[R + b - 1], 1);
+      z[R - b].x = __shfl_up_sync(0xffffffffu, z[R + 4 - b].x, 1);
+      z[R - b].y = __shfl_up_sync(0xffffffffu, z[R + 4 - b].y, 1);
+      z[R + 3 + b].x = __shfl_down_sync(0xffffffffu, z[R + b - 1].x, 1);
+      z[R + 3 + b].y = __shfl_down_sync(0xffffffffu, z[R + b - 1].y, 1);
+    }
+    float o[4];
+    window4<R>(v, o);
+    h.I[0] = make_float2(o[0], o[1]);
+    h.I[1] = make_float2(o[2], o[3]);
+    window2<R>(z, h.Z[0], h.Z[1]);
+    window2<R>(z + 2, h.Z[2], h.Z[3]);
+  };
+  auto add = [](const Row& a, const Row& b) {
+    Row r;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) r.I[c] = wadd(a.I[c], b.I[c]);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) r.Z[c] = wadd(a.Z[c], b.Z[c]);
+    return r;
+  };
+  auto write = [&](const Row& s, int vy) {
+    const int oy = (vy < H - 1) ? vy : (vy == vH ? H - 1 : -1);
+    if (oy < 0) return;
+    float o_r[4], o_p[4], o_c[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float si = c & 1 ? s.I[c / 2].y : s.I[c / 2].x;
+      o_r[c] = si * inv_2n;
+      o_p[c] = atan2_fast(s.Z[c].y, s.Z[c].x);
+      o_c[c] = boxcar_coherence(s.Z[c].x, s.Z[c].y, si);
+    }
+    const size_t rowo = (size_t)oy * W;
+    if (VEC && plain) {
+      if (!writes) return;
+      *reinterpret_cast<float4*>(ref + rowo + x0) = make_float4(o_r[0], o_r[1], o_r[2], o_r[3]);
+      *reinterpret_cast<float4*>(phase + rowo + x0) = make_float4(o_p[0], o_p[1], o_p[2], o_p[3]);
+      *reinterpret_cast<float4*>(coh + rowo + x0) = make_float4(o_c[0], o_c[1], o_c[2], o_c[3]);
+      return;
+    }
+    if (!VEC && plain) {
+      // rows of any alignment: through shared memory, so that a store covers
+      // 32 adjacent columns
+      float(*o)[128] = out_s[threadIdx.x >> 5];
+      __syncwarp();  // the row before is written
+      reinterpret_cast<float4*>(o[0])[lane] = make_float4(o_r[0], o_r[1], o_r[2], o_r[3]);
+      reinterpret_cast<float4*>(o[1])[lane] = make_float4(o_p[0], o_p[1], o_p[2], o_p[3]);
+      reinterpret_cast<float4*>(o[2])[lane] = make_float4(o_c[0], o_c[1], o_c[2], o_c[3]);
+      __syncwarp();
+      const size_t at = rowo + xs + 4 + lane;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (k == 3 && lane >= kWalkCols - 96) break;
+        ref[at + 32 * k] = o[0][4 + lane + 32 * k];
+        phase[at + 32 * k] = o[1][4 + lane + 32 * k];
+        coh[at + 32 * k] = o[2][4 + lane + 32 * k];
+      }
+      return;
+    }
+    if (!writes) return;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int x = x0 + c;
+      const int ox = (x < W - 1) ? x : (x == vW ? W - 1 : -1);
+      if (ox < 0) continue;
+      ref[rowo + ox] = o_r[c];
+      phase[rowo + ox] = o_p[c];
+      coh[rowo + ox] = o_c[c];
+    }
+  };
+
+#pragma unroll
+  for (int b = 0; b < kWalkRing; ++b) fetch();
+  Row v[2 * R + 4];  // rows of a group of four windows; the first 2 R stay for the next
+#pragma unroll
+  for (int b = 0; b < 2 * R; ++b) next_row(v[b]);
+  for (int g = 0; g < groups; ++g) {
+    const int vy = y0 + 4 * g;
+    if (vy > vH) break;
+    // window4's sums, each output as soon as its last row is there
+    if (R == 1) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        next_row(v[q + 2]);
+        write(add(add(v[q], v[q + 1]), v[q + 2]), vy + q);
+      }
+    } else {
+      next_row(v[w - 1]);
+      Row c = v[3];
+#pragma unroll
+      for (int k = 4; k < w; ++k) c = add(c, v[k]);
+      const Row l1 = add(v[1], v[2]);
+      write(add(add(v[0], l1), c), vy);
+      const Row t1 = add(l1, c), t2 = add(v[2], c);
+      next_row(v[w]);
+      write(add(t1, v[w]), vy + 1);
+      next_row(v[w + 1]);
+      const Row r2 = add(v[w], v[w + 1]);
+      write(add(t2, r2), vy + 2);
+      next_row(v[w + 2]);
+      write(add(c, add(r2, v[w + 2])), vy + 3);
+    }
+#pragma unroll
+    for (int b = 0; b < 2 * R; ++b) v[b] = v[b + 4];
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+template <int R>
+cudaError_t launch_boxcar_walk(const float* a1, const float* a2, const float* phi, float* ref, float* phase,
+                               float* coh, int H, int W, int sms, cudaStream_t st) {
+  auto vec = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+  const bool all = W % 4 == 0 && vec(a1) && vec(a2) && vec(phi) && vec(ref) && vec(phase) && vec(coh);
+  const int gx = ((W - 1 + R) / kWalkCols + kWalkWarps) / kWalkWarps, rows4 = (H - 1 + R) / 4 + 1;
+  // every walk sums 2 R rows before its first output: long ones where the
+  // scene has several waves of them, else the length with the shortest sum of
+  // waves
+  const long long slots = (long long)kWalkBlocks * sms;
+  int groups = kWalkGroups;
+  long long best = 0;
+  for (int g = kWalkGroups; g >= 1; --g) {
+    const long long waves = ((long long)gx * ((rows4 + g - 1) / g) + slots - 1) / slots;
+    const long long cost = waves * (4 * g + 2 * R + 4);
+    if (best == 0 || cost < best) best = cost, groups = g;
+  }
+  const dim3 grid(gx, (rows4 + groups - 1) / groups);
+  if (all)
+    boxcar_walk_kernel<R, true><<<grid, 32 * kWalkWarps, 0, st>>>(a1, a2, phi, ref, phase, coh, H, W, groups);
+  else
+    boxcar_walk_kernel<R, false><<<grid, 32 * kWalkWarps, 0, st>>>(a1, a2, phi, ref, phase, coh, H, W, groups);
+  return cudaGetLastError();
 }
 
 template <int R>
@@ -381,12 +628,24 @@ int boxcar_device(const float* a1, const float* a2, const float* phi, float* ref
     const cudaError_t e = allow_dynamic_smem((const void*)boxcar_kernel, smem, allowed);
     if (e != cudaSuccess) return cuda_error(e, "boxcar shared-memory limit");
   }
+  // The walk wins once the scene gives every SM its twelve warps: 3 x 3 and
+  // 7 x 7 take 41 and 47 us at 2500 x 2503 (tiled 49 and 50), 31 and 38 at
+  // 2100 x 2203 (36 and 37), 12.4 and 14.5 at 1024 x 1024 (9.6 and 10.8).  At
+  // 9 x 9 its registers leave eight warps: 110 us at 4096 x 4096 (114), 96 at
+  // 3000 x 4001 (92).
+  const bool walk = (long long)H * W >= 5LL << 20;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const int sms = sm_count(dev);
   cudaError_t e = cudaSuccess;
   switch (r) {
     case 0: e = launch_boxcar_r<0>(a1, a2, phi, ref, phase, coh, H, W, grid, st); break;
-    case 1: e = launch_boxcar_r<1>(a1, a2, phi, ref, phase, coh, H, W, grid, st); break;
-    case 2: e = launch_boxcar_r<2>(a1, a2, phi, ref, phase, coh, H, W, grid, st); break;
-    case 3: e = launch_boxcar_r<3>(a1, a2, phi, ref, phase, coh, H, W, grid, st); break;
+    case 1: e = walk ? launch_boxcar_walk<1>(a1, a2, phi, ref, phase, coh, H, W, sms, st)
+                       : launch_boxcar_r<1>(a1, a2, phi, ref, phase, coh, H, W, grid, st); break;
+    case 2: e = walk ? launch_boxcar_walk<2>(a1, a2, phi, ref, phase, coh, H, W, sms, st)
+                       : launch_boxcar_r<2>(a1, a2, phi, ref, phase, coh, H, W, grid, st); break;
+    case 3: e = walk ? launch_boxcar_walk<3>(a1, a2, phi, ref, phase, coh, H, W, sms, st)
+                       : launch_boxcar_r<3>(a1, a2, phi, ref, phase, coh, H, W, grid, st); break;
     case 4: e = launch_boxcar_r<4>(a1, a2, phi, ref, phase, coh, H, W, grid, st); break;
     case 5: e = launch_boxcar_r<5>(a1, a2, phi, ref, phase, coh, H, W, grid, st); break;
     case 6: e = launch_boxcar_r<6>(a1, a2, phi, ref, phase, coh, H, W, grid, st); break;
