@@ -22,8 +22,10 @@
 //     lane's registers, shared memory for the transposes), multiplies by
 //     |Z|^alpha (weighted_multiply.cl), transforms back with the 1/p^2 scale
 //     of the reference's clFFT plan (goldstein_patch_ft_test.cpp) and stores the
-//     patch;
-//  goldstein_pack_kernel   one thread per 4 output pixels of a row: the raw interferogram
+//     patch, as it lies in shared memory, by one bulk copy (four patches a block,
+//     24 warps per SM; 183 us on 4099 x 5003, issue 65 %, against 190 us with
+//     the rows read back and stored by the lanes);
+//  goldstein_pack_kernel   one thread per column of a few output rows: the raw interferogram
 //     plus the weighted contributions of the (up to four) patches covering the
 //     pixel, added in the order of the reference's four parity launches, which
 //     accumulate onto the buffer that still holds the raw interferogram
@@ -34,8 +36,8 @@
 // DESPECKCL_B200_GOLDSTEIN_FUSED=1 selects goldstein_fused_kernel instead, the
 // same arithmetic in one warp-specialised launch per tile with the patches
 // kept in shared memory (described above the kernel).  Both give the same
-// bits.  On B200 the two kernels are faster at every measured size (8192^2:
-// 1.09 ms against 1.56 ms): the fused kernel's ring of patch rows (205 KB)
+// bits.  On B200 the two kernels are faster at every measured size (4096^2:
+// 0.25 ms against 0.46 ms): the fused kernel's ring of patch rows (205 KB)
 // leaves one CTA of 16 warps per SM, half of them FFTs and half latency-bound
 // overlap-add, while the patch kernel runs 24 warps per SM and the pack kernel
 // up to 64, and the patches' round trip through HBM (~28 B per output pixel)
@@ -45,6 +47,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdint>
 #include <cstdlib>
 #include <vector>
 
@@ -65,6 +68,8 @@ const bool g_goldstein_fused = [] {
 constexpr int kP = 32;           // patch side (the FFT length)
 constexpr int kWarps = 4;        // patches per CTA (34 KB of transpose buffers)
 constexpr int kPitch = kP + 1;   // float2 row pitch of a warp's transpose buffer
+constexpr int kPatch = kP * kPitch;  // float2 of a filtered patch, in the buffer and in memory
+static_assert(kPatch * sizeof(float2) % 16 == 0, "whole patches by bulk copies");
 
 // W_32^m = exp(-2 pi i m / 32), m = 0..15
 __constant__ float2 c_tw32[16] = {
@@ -172,14 +177,19 @@ struct GoldsteinTile {
   int x_lo, x_hi;      // output columns likewise
 };
 
-// Z = 0.5 (a1 + a2) e^{j phi} at flat index i (raw_interferogram.cl)
-__device__ __forceinline__ float2 raw_z(const float* __restrict__ a1, const float* __restrict__ a2,
-                                        const float* __restrict__ phi, size_t i) {
-  const float amp = __fmul_rn(0.5f, __fadd_rn(a1[i], a2[i]));
+// Z = 0.5 (a1 + a2) e^{j phi} (raw_interferogram.cl)
+__device__ __forceinline__ float2 raw_z(float a1, float a2, float phi) {
+  const float amp = __fmul_rn(0.5f, __fadd_rn(a1, a2));
   float sn, cs;
-  __sincosf(phi[i], &sn, &cs);
+  __sincosf(phi, &sn, &cs);
   return make_float2(__fmul_rn(amp, cs), __fmul_rn(amp, sn));
 }
+__device__ __forceinline__ float2 raw_z(const float* __restrict__ a1, const float* __restrict__ a2,
+                                        const float* __restrict__ phi, size_t i) {
+  return raw_z(a1[i], a2[i], phi[i]);
+}
+
+constexpr int kGather = 8;  // rows of a patch loaded before any is used
 
 // Filters patch (py, px) of the tile whose position (0, 0) is image pixel
 // (o0y, o0x) into buf[r * kPitch + c] (row r, column c), one warp: gathers the
@@ -192,11 +202,36 @@ __device__ __forceinline__ void filter_patch(const float* __restrict__ a1, const
   {
     const int tx = clampg(px * g.s + lane - g.ov, 0, g.sub - 1);
     const int ix = clampg(o0x + tx, 0, g.W - 1);
-#pragma unroll 4
-    for (int r = 0; r < kP; ++r) {
-      const int ty = clampg(py * g.s + r - g.ov, 0, g.sub - 1);
-      const int iy = clampg(o0y + ty, 0, g.H - 1);
-      buf[r * kPitch + lane] = raw_z(a1, a2, phi, (size_t)iy * g.W + ix);
+    // patches whose rows all lie inside the tile and the scene read without
+    // clamping, kGather rows of loads in flight
+    const int ty0 = py * g.s - g.ov, iy0 = o0y + ty0;
+    const bool inside = ty0 >= 0 && ty0 + kP <= g.sub && iy0 >= 0 && iy0 + kP <= g.H;
+    const size_t at = (size_t)(inside ? iy0 : 0) * g.W + ix;
+#pragma unroll 1
+    for (int r0 = 0; r0 < kP; r0 += kGather) {
+      float m[kGather], s[kGather], p[kGather];
+      if (inside) {
+        const float* b1 = a1 + at + (size_t)r0 * g.W;
+        const float* b2 = a2 + at + (size_t)r0 * g.W;
+        const float* bp = phi + at + (size_t)r0 * g.W;
+#pragma unroll
+        for (int r = 0; r < kGather; ++r) {
+          m[r] = __ldg(b1 + (size_t)r * g.W);
+          s[r] = __ldg(b2 + (size_t)r * g.W);
+          p[r] = __ldg(bp + (size_t)r * g.W);
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < kGather; ++r) {
+          const int ty = clampg(ty0 + r0 + r, 0, g.sub - 1);
+          const size_t i = (size_t)clampg(o0y + ty, 0, g.H - 1) * g.W + ix;
+          m[r] = __ldg(a1 + i);
+          s[r] = __ldg(a2 + i);
+          p[r] = __ldg(phi + i);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < kGather; ++r) buf[(r0 + r) * kPitch + lane] = raw_z(m[r], s[r], p[r]);
     }
   }
   __syncwarp();
@@ -236,16 +271,23 @@ __device__ __forceinline__ void filter_patch(const float* __restrict__ a1, const
 __global__ void __launch_bounds__(32 * kWarps)
     goldstein_patch_kernel(const float* __restrict__ a1, const float* __restrict__ a2, const float* __restrict__ phi,
                            float2* __restrict__ patches, GoldsteinGeom g, GoldsteinTile t, float alpha) {
-  __shared__ float2 sbuf[kWarps][kP * kPitch];
+  __shared__ __align__(16) float2 sbuf[kWarps][kPatch];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int pid = blockIdx.x * kWarps + warp;
   if (pid >= t.n_py * t.n_px) return;  // whole warp leaves together
   float2* buf = sbuf[warp];
   filter_patch(a1, a2, phi, buf, g, t.h0, t.w0, t.py_lo + pid / t.n_px, t.px_lo + pid % t.n_px, alpha, lane);
+  // the buffer as it is, padding included, in one bulk copy
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncwarp();
-  float2* out = patches + (size_t)pid * kP * kP;
-#pragma unroll 4
-  for (int r = 0; r < kP; ++r) out[r * kP + lane] = buf[r * kPitch + lane];
+  if (lane == 0) {
+    asm volatile(
+        "cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\t"
+        "cp.async.bulk.commit_group;\n\t"
+        "cp.async.bulk.wait_group 0;" ::"l"(patches + (size_t)pid * kPatch),
+        "r"((uint32_t)__cvta_generic_to_shared(buf)), "n"(kPatch * (int)sizeof(float2))
+        : "memory");
+  }
 }
 
 // weight of a patch sample in the overlap-add (patches_pack.cl:50-63)
@@ -272,69 +314,112 @@ __device__ __forceinline__ void write_polar(float* __restrict__ ref, float* __re
   phase[o] = atan2_fast(v.y, v.x);
 }
 
-constexpr int kPackX = 4;  // output columns per thread (32 apart: coalesced per warp); 2 and 8 measured slower
+// The covering patches along one axis of tile position t: q = (t + ov) / s at
+// offset t + ov - q s, and q - 1 at offset + s when that is still inside the
+// patch (one of each parity); index 0 is the even patch, 1 the odd one.
+// Patches lo .. lo + n - 1 are filtered.
+struct PackCover {
+  int q[2];    // patch minus lo
+  int o[2];    // offset in it
+  float f[2];  // weight; 0: it does not cover t
+};
 
-__global__ void __launch_bounds__(256)
+__device__ __forceinline__ PackCover pack_cover(int t, int lo, int n, const GoldsteinGeom& g) {
+  const int q = div_s(t + g.ov, g), o = t + g.ov - q * g.s;
+  const bool in0 = q >= lo && q < lo + n;
+  const bool in1 = q - 1 >= lo && q - 1 < lo + n && o + g.s < kP;
+  const bool odd = q & 1;
+  PackCover c;
+  c.q[0] = (odd ? q - 1 : q) - lo;
+  c.q[1] = (odd ? q : q - 1) - lo;
+  c.o[0] = odd ? o + g.s : o;
+  c.o[1] = odd ? o : o + g.s;
+  c.f[0] = (odd ? in1 : in0) ? pack_factor(c.o[0], t, g.ov, g.sub) : 0.0f;
+  c.f[1] = (odd ? in0 : in1) ? pack_factor(c.o[1], t, g.ov, g.sub) : 0.0f;
+  return c;
+}
+
+constexpr int kPackBatch = 2;   // rows whose samples a thread loads before it uses any
+constexpr int kPackBlocks = 5;  // per SM, for registers without spills
+
+// A block takes kPackRows rows of 256 columns, a thread one column of them:
+// what depends on the column (patches, offsets, weights) is worked out once
+// per thread, what depends on the row once per block, in shared memory.  With
+// both worked out per pixel the kernel spent 209 thread instructions on each,
+// most of them integer, and took 157 us on 4099 x 5003 (117 us now).  Two rows
+// of loads in flight at five blocks per SM are faster than three or four at
+// four and three (122 and 120 us); a batch of four held to 64 registers spills
+// (134 us and more).
+template <int kPackRows>
+__global__ void __launch_bounds__(256, kPackBlocks)
     goldstein_pack_kernel(const float* __restrict__ a1, const float* __restrict__ a2, const float* __restrict__ phi,
                           const float2* __restrict__ patches, float* __restrict__ ref, float* __restrict__ phase,
                           GoldsteinGeom g, GoldsteinTile t) {
-  const int y = t.y_lo + blockIdx.y * 8 + (threadIdx.x >> 5);
-  if (y > t.y_hi) return;
-  // tile position whose result lands here (the clamped write-back keeps the
-  // last one; only the last tile row / column reaches row H-1 / column W-1)
-  const int ty = (y == g.H - 1) ? g.sub - g.ov - 1 : y - t.h0;
-  const size_t irow = (size_t)clampg(t.h0 + ty, 0, g.H - 1) * g.W;
-  // covering patches per axis: q = (t + ov) / s at offset t + ov - q s, and
-  // q - 1 at offset + s when that is still inside the patch (one of each
-  // parity); index 0 of the arrays below is the even patch, 1 the odd one
-  const int qy = div_s(ty + g.ov, g), ry = ty + g.ov - qy * g.s;
-  const bool vy0 = qy >= t.py_lo && qy < t.py_lo + t.n_py;
-  const bool vy1 = qy - 1 >= t.py_lo && qy - 1 < t.py_lo + t.n_py && ry + g.s < kP;
-  const bool ye1 = qy & 1;
-  int py_[2], ry_[2];
-  bool vy_[2];
-  float fy_[2];
-  py_[0] = ye1 ? qy - 1 : qy;
-  py_[1] = ye1 ? qy : qy - 1;
-  ry_[0] = ye1 ? ry + g.s : ry;
-  ry_[1] = ye1 ? ry : ry + g.s;
-  vy_[0] = ye1 ? vy1 : vy0;
-  vy_[1] = ye1 ? vy0 : vy1;
+  __shared__ size_t s_in[kPackRows];  // flat index of the raw interferogram's row
+  // the covering patches, even row first: their row at column 0 of the tile's
+  // patches, and their weights (0: none)
+  __shared__ const float2* s_patch[kPackRows][2];
+  __shared__ float s_f[kPackRows][2];
+  const int y0 = t.y_lo + (int)blockIdx.y * kPackRows, rows = min(kPackRows, t.y_hi + 1 - y0);
+  // tile position whose result lands on an output (the clamped write-back
+  // keeps the last one; only the last tile row / column reaches row H-1 /
+  // column W-1)
+  if ((int)threadIdx.x < kPackRows) {
+    const int y = min(y0 + (int)threadIdx.x, t.y_hi);
+    const int ty = (y == g.H - 1) ? g.sub - g.ov - 1 : y - t.h0;
+    const PackCover c = pack_cover(ty, t.py_lo, t.n_py, g);
+    s_in[threadIdx.x] = (size_t)clampg(t.h0 + ty, 0, g.H - 1) * g.W;
+    const float2* r0 = patches + (ptrdiff_t)c.q[0] * t.n_px * kPatch + c.o[0] * kPitch;
+    const float2* r1 = patches + (ptrdiff_t)c.q[1] * t.n_px * kPatch + c.o[1] * kPitch;
+    const bool even = c.f[0] != 0.0f;
+    s_patch[threadIdx.x][0] = even ? r0 : r1;
+    s_patch[threadIdx.x][1] = r1;
+    s_f[threadIdx.x][0] = even ? c.f[0] : c.f[1];
+    s_f[threadIdx.x][1] = even ? c.f[1] : 0.0f;
+  }
+  __syncthreads();
+  const int x = t.x_lo + (int)blockIdx.x * 256 + (int)threadIdx.x;
+  if (x > t.x_hi) return;
+  const int tx = (x == g.W - 1) ? g.sub - g.ov - 1 : x - t.w0;
+  const int ix = clampg(t.w0 + tx, 0, g.W - 1);
+  const PackCover c = pack_cover(tx, t.px_lo, t.n_px, g);
+  const int at[2] = {c.q[0] * kPatch + c.o[0], c.q[1] * kPatch + c.o[1]};
+  const bool in[2] = {c.f[0] != 0.0f, c.f[1] != 0.0f};
+  size_t out = (size_t)y0 * g.W + x;
+#pragma unroll 1
+  for (int k0 = 0; k0 < rows; k0 += kPackBatch) {
+    float m[kPackBatch], s[kPackBatch], p[kPackBatch];
+    float2 q[kPackBatch][2][2];  // [x parity][first, second patch row]
 #pragma unroll
-  for (int b = 0; b < 2; ++b) fy_[b] = pack_factor(ry_[b], ty, g.ov, g.sub);
-  const int x0 = t.x_lo + blockIdx.x * (32 * kPackX) + (threadIdx.x & 31);
+    for (int k = 0; k < kPackBatch; ++k) {
+      const size_t i = s_in[k0 + k] + ix;
+      m[k] = __ldg(a1 + i);
+      s[k] = __ldg(a2 + i);
+      p[k] = __ldg(phi + i);
 #pragma unroll
-  for (int m = 0; m < kPackX; ++m) {
-    const int x = x0 + 32 * m;
-    if (x > t.x_hi) break;
-    const int tx = (x == g.W - 1) ? g.sub - g.ov - 1 : x - t.w0;
-    float2 v = raw_z(a1, a2, phi, irow + clampg(t.w0 + tx, 0, g.W - 1));
-    const int qx = div_s(tx + g.ov, g), cx = tx + g.ov - qx * g.s;
-    const bool vx0 = qx >= t.px_lo && qx < t.px_lo + t.n_px;
-    const bool vx1 = qx - 1 >= t.px_lo && qx - 1 < t.px_lo + t.n_px && cx + g.s < kP;
-    const bool xe1 = qx & 1;
-    int px_[2], cx_[2];
-    bool vx_[2];
-    float fx_[2];
-    px_[0] = xe1 ? qx - 1 : qx;
-    px_[1] = xe1 ? qx : qx - 1;
-    cx_[0] = xe1 ? cx + g.s : cx;
-    cx_[1] = xe1 ? cx : cx + g.s;
-    vx_[0] = xe1 ? vx1 : vx0;
-    vx_[1] = xe1 ? vx0 : vx1;
+      for (int b = 0; b < 2; ++b) {
+        if (s_f[k0 + k][b] == 0.0f) continue;
+        const float2* r = s_patch[k0 + k][b];
 #pragma unroll
-    for (int a = 0; a < 2; ++a) fx_[a] = pack_factor(cx_[a], tx, g.ov, g.sub);
-    // the reference's four parity launches in order: (x, y) parity (0,0), (0,1), (1,0), (1,1)
-#pragma unroll
-    for (int xpar = 0; xpar < 2; ++xpar)
-#pragma unroll
-      for (int ypar = 0; ypar < 2; ++ypar) {
-        if (!vx_[xpar] || !vy_[ypar]) continue;
-        add_sample(v, fx_[xpar], fy_[ypar],
-                   patches[((size_t)(py_[ypar] - t.py_lo) * t.n_px + (px_[xpar] - t.px_lo)) * kP * kP +
-                           ry_[ypar] * kP + cx_[xpar]]);
+        for (int a = 0; a < 2; ++a)
+          if (in[a]) q[k][a][b] = __ldg(r + at[a]);
       }
-    write_polar(ref, phase, (size_t)y * g.W + x, v);
+    }
+#pragma unroll
+    for (int k = 0; k < kPackBatch; ++k) {
+      if (k0 + k >= rows) break;
+      float2 v = raw_z(m[k], s[k], p[k]);
+      // the reference's four parity launches in order: (x, y) parity (0,0), (0,1), (1,0), (1,1)
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          const float f = s_f[k0 + k][b];
+          if (f != 0.0f && in[a]) add_sample(v, c.f[a], f, q[k][a][b]);
+        }
+      write_polar(ref, phase, out, v);
+      out += g.W;
+    }
   }
 }
 
@@ -671,7 +756,7 @@ int goldstein_device(const float* a1, const float* a2, const float* phi, float* 
   size_t np = 0;
   for (const GoldsteinTile& t : tiles) np = std::max(np, (size_t)t.n_py * t.n_px);
   float2* patches = nullptr;
-  cudaError_t e = cudaMallocAsync(&patches, np * kP * kP * sizeof(float2), st);
+  cudaError_t e = cudaMallocAsync(&patches, np * kPatch * sizeof(float2), st);
   if (e != cudaSuccess) return cuda_error(e, "cudaMallocAsync(Goldstein patches)");
   // tiles in the reference's order; each pack writes only the pixels its tile
   // owns, so one patch buffer serves the tiles in turn
@@ -679,8 +764,14 @@ int goldstein_device(const float* a1, const float* a2, const float* phi, float* 
     const size_t n = (size_t)t.n_py * t.n_px;
     goldstein_patch_kernel<<<(unsigned)((n + kWarps - 1) / kWarps), 32 * kWarps, 0, st>>>(a1, a2, phi, patches, g, t,
                                                                                          alpha);
-    dim3 grid((t.x_hi - t.x_lo + 32 * kPackX) / (32 * kPackX), (t.y_hi - t.y_lo + 8) / 8);
-    goldstein_pack_kernel<<<grid, 256, 0, st>>>(a1, a2, phi, patches, ref, phase, g, t);
+    // eight rows per block while they fill the GPU a few times over: 4099 x
+    // 5003 takes 117 us (four rows: 129), 512 x 512 4.7 us (3.6)
+    const unsigned nx = (unsigned)((t.x_hi - t.x_lo + 256) / 256);
+    const int n_rows = t.y_hi - t.y_lo + 1;
+    if ((long long)nx * (n_rows / 8) >= 4LL * kPackBlocks * sm_count(dev))
+      goldstein_pack_kernel<8><<<dim3(nx, (n_rows + 7) / 8), 256, 0, st>>>(a1, a2, phi, patches, ref, phase, g, t);
+    else
+      goldstein_pack_kernel<4><<<dim3(nx, (n_rows + 3) / 4), 256, 0, st>>>(a1, a2, phi, patches, ref, phase, g, t);
     profile_count(2);
   }
   e = cudaGetLastError();

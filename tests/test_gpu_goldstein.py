@@ -108,3 +108,26 @@ def test_fused_kernel_equals_two_pass_path_bit_for_bit(tmp_path):
         res.append([z[k] for k in sorted(z.files, key=lambda s: int(s.split("_")[1]))])
     for a, b in zip(*res):
         assert np.array_equal(a, b, equal_nan=True)
+
+
+@pytest.mark.parametrize("shape,ov", [((1999, 3073), 4), ((24001, 100), 7), ((2005, 3000), 1)])
+def test_blocks_of_eight_rows_equal_fused_kernel(tmp_path, shape, ov):
+    # scenes large enough for the overlap-add's blocks of eight rows, with a
+    # last block of one column or of one to seven rows
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    head, rest = FUSED_VS_TWO_PASS.split("in [")
+    code = head + f"in [({shape[0]}, {shape[1]}, {ov}, 0.5, 3)]:" + rest.split("]:", 1)[1]
+    res = []
+    for fused in ("1", "0"):
+        out = str(tmp_path / f"{fused}.npz")
+        env = dict(os.environ, DCL_ROOT=root, DCL_OUT=out, DESPECKCL_B200_GOLDSTEIN_FUSED=fused)
+        r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0, r.stderr[-3000:]
+        z = np.load(out)
+        res.append([z[k] for k in sorted(z.files)])
+    for a, b in zip(*res):
+        assert np.array_equal(a, b, equal_nan=True)
