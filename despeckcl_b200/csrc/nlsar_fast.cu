@@ -2,7 +2,11 @@
 // half size and the patch half sizes of the passes (the common
 // configurations: one pass shape, or two such as {3,5,7} and {9,11} with the
 // tile staged for the largest patch), for sm_100a.  Same semantics as the
-// generic kernel in nlsar_kernels.cu.
+// generic kernel in nlsar_kernels.cu.  It filters where nlsar_split.cu has no
+// memory for its volume of weight codes (allocation-free entry point, request
+// server, a full device), tables the codes cannot hold, explicit batch variants
+// and the arithmetic variants; elsewhere the two kernels there take about half
+// its time (40.7 ms against 77.0 at 4096 x 4096) for the same bits.
 //
 // Per CTA: a 32 x 32 output tile (32 x 24 for 8-plane covariance input), each
 // thread owning 2 (16 warps) or 4 (8 warps) vertically consecutive pixels of
@@ -174,7 +178,7 @@ template <class L, int PH0, int PH1, int PH2, int PV>
 __device__ __forceinline__ void fast_pass(const FilterParams& P, const PassParams& pp, float* smem,
                                           Best<L::PX, L::NM>& best) {
   constexpr int WSH = L::WSH, K = L::K, RS = L::RS, RO = L::RO, TW = L::TW, PX = L::PX;
-  constexpr int NT = L::THREADS, NW = L::WARPS, NA = L::NA, NM = L::NM;
+  constexpr int NT = L::THREADS, NW = L::WARPS, NA = L::NA;
   constexpr bool FULL8 = L::FULL8;
   constexpr int NP = np_of<PH0, PH1, PH2>();
   constexpr int PHM = cmax(PH0, cmax(PH1, PH2));

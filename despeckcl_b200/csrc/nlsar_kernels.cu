@@ -5,7 +5,9 @@
 //                  "virtual plane" arrays in HBM: the un-rescaled covariance
 //                  and, per scale, the rescaled Gaussian-averaged covariance
 //                  plus its log-determinant.
-//   fused kernel   one CTA per 32-column output tile: stages the tile and its
+//   filter         the two kernels of nlsar_split.cu for the common shapes; for
+//                  all others the kernel of this file,
+//                  one CTA per 32-column output tile: stages the tile and its
 //                  halo in shared memory, loops over every search-window
 //                  offset computing GLR pixel similarities, box sums for up to
 //                  three patch sizes, LUT weights and register accumulators,

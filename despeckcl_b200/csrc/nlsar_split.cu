@@ -9,8 +9,9 @@
 //
 //  nlsar_index_kernel  for the lower half window (dy > 0, or dy = 0 and
 //      dx > 0), every scale and patch size: GLR similarity, patch sums and
-//      the index of the composite weight (compute_weights.cl:40-51); up to
-//      three patch sizes of a pass share one 32-bit word per (offset, pixel).
+//      the index of the composite weight (compute_weights.cl:40-51), one byte
+//      per patch size; three patch sizes share a 32-bit word per (offset,
+//      pixel).
 //  nlsar_mean_kernel   per output pixel: for all offsets in the reference's
 //      row-major order (compute_nl_statistics.cl:77-78) the word of o at x
 //      (lower half) or at x + q for q = -o (upper half), the weights from the
@@ -24,8 +25,8 @@
 // kernel has no accumulators, so it can hold the vertical sums of a column in
 // registers: one warp walks down 128 columns for one offset with no barrier.
 //
-// The volume of one pass is (sws^2 - 1) / 2 words per pixel (880 B at search
-// 21), so a scene is filtered in segments of rows whose volume fits a budget
+// The volume of one pass is (sws^2 - 1) / 2 words of 1, 2 or 4 bytes per pixel
+// (220 to 880 B at search 21), so a scene is filtered in segments of rows whose volume fits a budget
 // (kSplitBudgetBytes), index kernel and mean kernel in turn.
 
 #include <cuda_runtime.h>

@@ -25,8 +25,11 @@
  *   dcl_stats_entry          nlsar::params + nlsar::stats                include/compute/nlsar/parameters.h:26-57,
  *                                                                          include/compute/nlsar/stats.h:28-55
  *
- * Staging timeouts.  The specialised NL-SAR kernel stages each tile with TMA
- * copies and waits for them with a bounded wait.  A thread block whose wait
+ * Staging timeouts.  The fused NL-SAR kernel (request server, allocation-free
+ * entry point, batches of an explicit variant, calls for whose weight codes
+ * there is no memory) stages each tile with TMA copies and waits for them with
+ * a bounded wait; the two kernels that filter all other calls have no such
+ * wait.  A thread block whose wait
  * runs out stops and leaves its remaining tiles unwritten (the reference has no
  * such case: it terminates the process on any OpenCL error,
  * src/compute/nlsar/nlsar_filter_sub_image.cpp:74-78).  It is reported:
@@ -93,12 +96,13 @@ int dcl_take_stage_timeouts(int* count);
 /* Timing of this library's kernels on the calling thread (no reference
  * counterpart; the reference's timed_run, src/clcfg/clcfg.h:97-119, measures
  * host wall clock).  Between begin and end, CUDA events are recorded on the
- * launching stream around every fused NL-SAR launch; end waits for them and
- * returns the summed fused-kernel time, the number of fused launches and the
- * number of all kernels the library launched. */
+ * launching stream around the filter launches of every NL-SAR call or band (the
+ * fused kernel, or the kernels around a volume of weight codes); end waits for
+ * them and returns their summed time, the number of such groups and the number
+ * of all kernels the library launched. */
 void dcl_profile_begin(void);
 /* Measured FP32 FMA throughput of the current device in TFLOP/s (FMA = 2
- * flops): the roofline denominator for the fused NL-SAR kernel.  No
+ * flops): the roofline denominator for the NL-SAR kernels.  No
  * reference counterpart. */
 int dcl_measure_fp32_tflops(double* tflops);
 int dcl_profile_end(double* fused_ms, long* fused_launches, long* all_launches);
@@ -159,7 +163,7 @@ int dcl_nlsar_covmat_device(const float* covmat_raw, float* covmat_filt, int hei
                             float h_param, float c_param, int select_mode, void* stream);
 
 /* Batched NL-SAR: n_scenes InSAR pairs of possibly different sizes, all
- * filtered with the same parameters in one persistent launch.  Each array
+ * filtered with the same parameters in shared launches.  Each array
  * holds n_scenes device pointers / sizes; a staging timeout is counted in the
  * device ledger (dcl_take_stage_timeouts).  The batched counterpart of
  * despeckcl::nlsar (include/despeckcl.h:45-59). */
@@ -172,11 +176,11 @@ int dcl_nlsar_insar_batch_device(int n_scenes, const float* const* ampl_master, 
 
 /* Prepared batches.  A batch binds n_scenes device input/output pointer sets
  * and the filter parameters once: the scratch, the scene descriptors and the
- * weight tables are set up at creation, every run filters all scenes with one
- * fused launch.  Flags: DCL_BATCH_GRAPH captures the launch sequence in a CUDA
- * graph (each run is one graph launch); DCL_BATCH_AUTOTUNE times the
- * specialised kernel's instantiations on the batch at creation and keeps the
- * fastest (cached per device and configuration; DESPECKCL_B200_TUNE_CACHE names
+ * weight tables are set up at creation, every run filters all scenes in shared
+ * launches.  Flags: DCL_BATCH_GRAPH captures the launch sequence in a CUDA
+ * graph (each run is one graph launch); DCL_BATCH_AUTOTUNE, where the batch runs
+ * on the fused kernel (see "Staging timeouts" above), times its
+ * instantiations on the batch at creation and keeps the fastest (cached per device and configuration; DESPECKCL_B200_TUNE_CACHE names
  * a file that keeps the choices across processes).  The autotuner times up to
  * three tile shapes: 32 x 32 tiles with 2 or 4 pixels per thread (variants 0
  * and 1) and, for patches {3,5,7}, 32 x 16 tiles with 2 pixels per thread
@@ -199,7 +203,7 @@ int dcl_nlsar_batch_run(dcl_nlsar_batch* batch, void* stream);
 /* The kernel instantiation in use (0: 32 x 32 tiles, 2 pixels per thread;
  * 1: 32 x 32, 4 pixels per thread; 2: 32 x 16, 2 pixels per thread). */
 int dcl_nlsar_batch_variant(const dcl_nlsar_batch* batch);
-/* Kernels one run launches (prep kernels per scene plus the fused launch). */
+/* Kernels one run launches (prep kernels per scene plus the filter launches). */
 int dcl_nlsar_batch_launches(const dcl_nlsar_batch* batch);
 void dcl_nlsar_batch_destroy(dcl_nlsar_batch* batch);
 
