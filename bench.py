@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""NL-SAR benchmark: Mpix/s of the fused B200 path on one 4096x4096 InSAR scene.
+"""NL-SAR benchmark: Mpix/s of the B200 path on one 4096x4096 InSAR scene.
 
 Workload: the plain NL-SAR configuration on a single 4096 x 4096 float32
 synthetic scene (search window 21, patches {3,5,7}, scales {1,3}, h 15, c 49,
@@ -7,7 +7,7 @@ per-pixel selection by the largest bias-reduced ENL), statistics trained on a
 separate seeded 128 x 128 homogeneous area (reflectivity 1, coherence 0.6).
 Seeded synthetic data stands in for real interferograms.
 
-A step is one full filter of the scene (prep kernels + the fused kernel) with
+A step is one full filter of the scene (prep kernels + filter kernels) with
 inputs resident in HBM (201 MB of inputs, larger than the 126 MB L2, so every
 step streams them from HBM).  `e2e` is the same metric through the public host
 API with pinned host buffers, copies included.  Under torchrun each rank
@@ -190,9 +190,9 @@ def cpu_oracle_rate(a1, a2, ph, stats, side, mode, threads):
 
 
 def traffic_from_profiles(size):
-    """DRAM bytes per fused launch from the committed ncu summary, scaled to
-    `size`, or None."""
-    path = os.path.join(ROOT, "profiles", "nlsar_fast_kernel.md")
+    """DRAM bytes of a step's filter kernels from the committed ncu summary,
+    scaled to `size`, or None."""
+    path = os.path.join(ROOT, "profiles", "nlsar_split_kernels.md")
     try:
         for line in open(path):
             if line.startswith("dram_bytes_per_pixel:"):
@@ -365,7 +365,7 @@ def run_ours(args):
                     "d2h_bytes_per_step": 3 * S * S * 4, "ms_per_step": e2e_ms},
             "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
                          "frac": achieved / peak.value, "traffic": traffic,
-                         "kernel": "nlsar_fast_kernel (specialised fused NL-SAR)", "kernel_ms": kern_ms,
+                         "kernel": "nlsar_index_kernel + nlsar_mean_kernel", "kernel_ms": kern_ms,
                          "flop_per_pixel": flop_per_pixel(args.mode),
                          "peak_source": "measured in-process FP32 FMA probe (dcl_measure_fp32_tflops)"},
             "gpu_launches": int(all_n.value),
