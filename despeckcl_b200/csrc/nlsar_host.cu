@@ -249,6 +249,7 @@ int make_plan(int sws, const int* patches, int np, const int* scales, int ns, co
   F.G = F.wsh + F.phm + pl.shm;
   // the specialised kernel serves the common settings, in 32 x 32 tiles for
   // InSAR input and 32 x 24 tiles for 8-plane covariance input
+  pl.generic_only = g_force_generic;
   pl.fast = !g_force_generic && fast_kernel_supported(F, full8);
   if (pl.fast && full8) F.tile_h = kFastTileH8;
   return DCL_OK;

@@ -5,8 +5,9 @@
 //                  "virtual plane" arrays in HBM: the un-rescaled covariance
 //                  and, per scale, the rescaled Gaussian-averaged covariance
 //                  plus its log-determinant.
-//   filter         the two kernels of nlsar_split.cu for the common shapes; for
-//                  all others the kernel of this file,
+//   filter         the two kernels of nlsar_split.cu for the patch sizes they
+//                  have; for all others, and where there is no memory for
+//                  their volume, the kernel of this file,
 //                  one CTA per 32-column output tile: stages the tile and its
 //                  halo in shared memory, loops over every search-window
 //                  offset computing GLR pixel similarities, box sums for up to

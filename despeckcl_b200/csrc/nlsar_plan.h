@@ -22,6 +22,7 @@ struct Plan {
   int shm = 0;                   // largest scale half among used slots
   bool full8 = false;
   bool fast = false;  // served by the specialised kernel (nlsar_fast.cu)
+  bool generic_only = false;  // the kernel of nlsar_kernels.cu was asked for
   int px = 4;
 };
 

@@ -25,6 +25,10 @@
 // kernel has no accumulators, so it can hold the vertical sums of a column in
 // registers: one warp walks down 128 columns for one offset with no barrier.
 //
+// Settings without a specialised fused kernel (other windows, patches {3,5})
+// take the same way with the arithmetic and summation order of nlsar_kernels.cu
+// (EXACT, nlsar_exact_mean_kernel), whose results they give bit for bit.
+//
 // The volume of one pass is (sws^2 - 1) / 2 words of 1, 2 or 4 bytes per pixel
 // (220 to 880 B at search 21), so a scene is filtered in segments of rows whose volume fits a budget
 // (kSplitBudgetBytes), index kernel and mean kernel in turn.
@@ -56,6 +60,14 @@ __host__ __device__ inline size_t idx_smem(int wsh, int phm, int R) {
   return (size_t)(R + 2 * phm + wsh) * idx_row_slots(wsh) * 20;
 }
 
+// The similarity of a lower-half offset as nlsar_kernels.cu evaluates it
+// (neighbour first, copy_symm_weights.cl:66-74; a NaN counts as 0 in WordWalk)
+__device__ __forceinline__ float glr_lower(float c2d, const float4 a, float la, const float4 b, float lb) {
+  const float s00 = a.x + b.x, s11 = a.y + b.y, sre = a.z + b.z, sim = a.w + b.w;
+  const float det = (s00 * s11) - (sre * sre + sim * sim);
+  return -(((c2d + lb) + la) - 2.0f * logf(det));
+}
+
 // One block: a rectangle of R rows x VC columns of one segment's volume, one
 // pass, the offsets u = 16 z + warp, 16 (z + Z) + warp, ...
 //
@@ -70,12 +82,16 @@ __host__ __device__ inline size_t idx_smem(int wsh, int phm, int R) {
 //
 // A warp walks down the rows for one offset (WordWalk), a lane evaluating the
 // four similarities of its columns per row.
-template <int PH0, int PH1, int PH2>
+//
+// EXACT: the arithmetic of nlsar_kernels.cu for the settings that it serves:
+// the staged term is ln det from the frame, the similarity takes the rounded
+// logarithm, the index a rounded division.
+template <int PH0, int PH1, int PH2, bool EXACT>
 __global__ void __launch_bounds__(kIdxThreads, 1)
     nlsar_index_kernel(const __grid_constant__ FilterParams P, const SceneDesc* __restrict__ scenes,
                        const SplitSeg* __restrict__ segs, int nseg, const __grid_constant__ PassList passes,
                        int shape, char* __restrict__ vol) {
-  using Walk = WordWalk<PH0, PH1, PH2>;
+  using Walk = WordWalk<PH0, PH1, PH2, EXACT>;
   constexpr int NP = Walk::NP, PHM = Walk::PHM, HL = Walk::HL, VC = Walk::VC;
   using Word = typename WordOf<NP>::T;
   extern __shared__ float4 smem4[];
@@ -106,19 +122,25 @@ __global__ void __launch_bounds__(kIdxThreads, 1)
     const int fx0 = VC * bx - 4 * HL - wsh - left + P.G, fy0 = S.row0 + r0 - PHM + P.G;
     const int ncol = left + 128 + wsh;
     const float4* cs = D.cs[pp.scale_slot];
+    const float* ld = D.ld[pp.scale_slot];
     constexpr int U = 6;  // 32 U >= ncol for search windows up to 41
     for (int r = warp; r < nrow; r += kIdxWarps) {
-      const float4* row = cs + (size_t)min(max(fy0 + r, 0), Hp - 1) * D.pitch;
+      const size_t row = (size_t)min(max(fy0 + r, 0), Hp - 1) * D.pitch;
       float4 v[U];
+      float term[U];
 #pragma unroll
       for (int k = 0; k < U; ++k)
-        if (lane + 32 * k < ncol) v[k] = row[min(max(fx0 + lane + 32 * k, 0), Wp - 1)];
+        if (lane + 32 * k < ncol) {
+          const size_t g = row + min(max(fx0 + lane + 32 * k, 0), Wp - 1);
+          v[k] = cs[g];
+          if (EXACT) term[k] = ld[g];
+        }
 #pragma unroll
       for (int k = 0; k < U; ++k) {
         const int p = lane + 32 * k;
         if (p < ncol) {
           const int slot = r * SP + p + (p >> 2);
-          const float t = pixel_term<kPrecRatio>(v[k]);
+          const float t = EXACT ? term[k] : pixel_term<kPrecRatio>(v[k]);
           sC[slot] = v[k];
           sL[slot] = t;
           reinterpret_cast<float*>(sC + r * SP + 5 * (p >> 2) + 4)[p & 3] = t;
@@ -127,7 +149,7 @@ __global__ void __launch_bounds__(kIdxThreads, 1)
     }
   }
   Walk walk;
-  walk.set(P, pp, true);  // patch sums in log2 units (nlsar_fast.cu)
+  walk.set(P, pp, !EXACT);  // patch sums in log2 units (nlsar_fast.cu)
   __syncthreads();
 
   const int nhalf = P.n_off / 2;
@@ -159,7 +181,7 @@ __global__ void __launch_bounds__(kIdxThreads, 1)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int n = j + (M + j >= 4 ? 1 : 0);
-          s[PHM + j] = glr_ratio(ctr[j], la4[j], nbr[n], nld[n]);
+          s[PHM + j] = EXACT ? glr_lower(P.c2d, ctr[j], la4[j], nbr[n], nld[n]) : glr_ratio(ctr[j], la4[j], nbr[n], nld[n]);
         }
         ctr += SP;
         nbr += SP;
@@ -415,29 +437,261 @@ __global__ void __launch_bounds__(L::THREADS, 1)
   write_pixel<L::FULL8>(S, (size_t)oy * S.W + ox, sCo[c], c2, 0, best);
 }
 
+// Means as nlsar_kernels.cu sums them, any window: the offsets in pairs, the
+// upper half's first and its mirror after it, the centre last.  One block: a
+// 32 x TH tile, one pixel per thread, the window at run time.  Every setting
+// measured gains over the kernel there, which computes every weight twice, a
+// pixel's similarities, sums and weights behind three block barriers per few
+// offsets: 400 x 450 with patches {3,5,7} and search 15 6.69 -> 0.88 ms, with
+// {3,5} and search 21 9.56 -> 1.20 ms, search 3 0.32 -> 0.14 ms; 64 x 64 with
+// one patch size and search 3 0.11 -> 0.07 ms.
+constexpr int kPairs = 7;  // offset pairs whose words are in flight
+
+__host__ __device__ constexpr int exact_tables(int npx) { return (npx + 1) / 2 * 65536; }
+__host__ __device__ inline size_t exact_smem(int wsh, int th, bool full8, int npx) {
+  return exact_tables(npx) + (size_t)(full8 ? 2 : 1) * (32 + 2 * wsh) * (th + 2 * wsh) * 16;
+}
+
+template <int TH, bool FULL8, int NPX>
+struct ExactL {
+  static constexpr int THREADS = 32 * TH;
+  static constexpr int NA = FULL8 ? 12 : 8, NM = FULL8 ? 8 : 4;
+};
+
+template <int TH, bool FULL8, int NPX, int NP>
+__device__ __forceinline__ void exact_pass(const FilterParams& P, int ps, const char* __restrict__ vol,
+                                           const SplitSeg& G, uint32_t lane_off, int RO, int extra, float& best_e,
+                                           float& best_a, float& best_s0, int& best_rank, int& best_combo,
+                                           float* best_m) {
+  using Word = typename WordOf<NP>::T;
+  using L = ExactL<TH, FULL8, NPX>;
+  constexpr int NA = L::NA;
+  extern __shared__ float4 smem4[];
+  char* sm = reinterpret_cast<char*>(smem4);
+  const PassParams& pp = P.pass[ps];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wsh = P.wsh;
+  __syncthreads();  // the previous pass's tables are no longer read
+  for (int i = tid; i < NP * 256 * 8; i += L::THREADS) {
+    const int m = i >> 11, e = (i >> 3) & 255;
+    const float w = e == kZeroCode ? 0.0f : P.wtab[pp.combo[m] * kMaxLut + e];
+    *reinterpret_cast<float4*>(sm + (m >> 1) * 65536 + e * 256 + (m & 1) * 128 + (i & 7) * 16) =
+        make_float4(w, w, w, w);
+  }
+  __syncthreads();
+  float A[NP][NA];
+#pragma unroll
+  for (int j = 0; j < NP; ++j)
+#pragma unroll
+    for (int a = 0; a < NA; ++a) A[j][a] = 0.0f;
+  const uint32_t lane4 = 4u * lane;
+  const float4* ctr = reinterpret_cast<const float4*>(sm + exact_tables(NPX)) + (warp + wsh) * RO + lane + wsh;
+  auto accumulate = [&](uint32_t word, const float4* v) {
+    const float4 c = v[0];
+    float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (FULL8) e = v[extra];
+    const float q0 = __fmul_rn(c.x, c.x), q1 = __fmul_rn(c.y, c.y);
+#pragma unroll
+    for (int j = 0; j < NP; ++j) {
+      const float w = *reinterpret_cast<const float*>(sm + (j >> 1) * 65536 + (j & 1) * 128 +
+                                                      __byte_perm(word, lane4, 0x5504 | (j << 4)));
+      A[j][0] = __fadd_rn(A[j][0], w);
+      A[j][1] = __fmaf_rn(w, w, A[j][1]);
+      A[j][2] = __fmaf_rn(w, c.x, A[j][2]);
+      A[j][3] = __fmaf_rn(w, c.y, A[j][3]);
+      A[j][4] = __fmaf_rn(w, q0, A[j][4]);
+      A[j][5] = __fmaf_rn(w, q1, A[j][5]);
+      A[j][6] = __fmaf_rn(w, c.z, A[j][6]);
+      A[j][7] = __fmaf_rn(w, c.w, A[j][7]);
+      if constexpr (FULL8) {
+        A[j][8] = __fmaf_rn(w, e.x, A[j][8]);
+        A[j][9] = __fmaf_rn(w, e.y, A[j][9]);
+        A[j][10] = __fmaf_rn(w, e.z, A[j][10]);
+        A[j][11] = __fmaf_rn(w, e.w, A[j][11]);
+      }
+    }
+  };
+  // pair i (offset o = (dy, dx) of the lower half, word i) from the last to
+  // the first: the weight of -o is word i at x - o, of o word i at x
+  const uint32_t plane = (uint32_t)G.rows * G.pitch;
+  const Word* words = reinterpret_cast<const Word*>(vol + G.vol + G.pass[ps]);
+  const int nhalf = P.n_off / 2;
+  uint32_t up[kPairs], down[kPairs];
+  int li = nhalf - 1, ldy = wsh, ldx = wsh;  // next pair to load
+  auto load = [&](int k) {
+    if (li >= 0) {
+      const uint32_t off = lane_off + (uint32_t)li * plane;
+      down[k] = __ldcg(words + off);
+      up[k] = __ldcg(words + (off - (uint32_t)(ldy * G.pitch + ldx)));
+      --li;
+      if (--ldx < -wsh) ldx = wsh, --ldy;
+    }
+  };
+#pragma unroll
+  for (int k = 0; k < kPairs; ++k) load(k);
+  int d = wsh * RO + wsh, dx = wsh;  // place of x + o after x
+  for (int i = nhalf - 1; i >= 0; i -= kPairs) {
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k) {
+      if (i - k < 0) break;
+      const uint32_t wu = up[k], wd = down[k];
+      load(k);
+      accumulate(wu, ctr - d);
+      accumulate(wd, ctr + d);
+      --d;
+      if (--dx < -wsh) dx = wsh, d -= RO - 2 * wsh - 1;
+    }
+  }
+  // centre weight 1, statistics, alpha, ENL', selection (nlsar_kernels.cu)
+  const float4 c = ctr[0];
+  float4 c2 = make_float4(0.f, 0.f, 0.f, 0.f);
+  if constexpr (FULL8) c2 = ctr[extra];
+#pragma unroll
+  for (int j = 0; j < NP; ++j) {
+    const float s0 = A[j][0] + 1.0f, s1 = A[j][1] + 1.0f;
+    const float s2 = A[j][2] + c.x, s3 = A[j][3] + c.y;
+    // rounded as there, where the products are shared by the patch sizes
+    const float s4 = __fadd_rn(A[j][4], __fmul_rn(c.x, c.x)), s5 = __fadd_rn(A[j][5], __fmul_rn(c.y, c.y));
+    const float s6 = A[j][6] + c.z, s7 = A[j][7] + c.w;
+    const float enl = s0 * s0 / s1;
+    const float i0 = s2 / s0, i1 = s3 / s0;
+    const float v0 = s4 / s0 - i0 * i0, v1 = s5 / s0 - i1 * i1;
+    float alpha = 0.0f;
+    alpha = fmaxf(alpha, fmaxf(0.0f, (v0 - i0 * i0) / v0));
+    alpha = fmaxf(alpha, fmaxf(0.0f, (v1 - i1 * i1) / v1));
+    if (P.alpha_zero) alpha = 0.0f;
+    const float oma = 1.0f - alpha;
+    const float enb = enl / (oma * oma + (alpha * alpha + 2.0f * alpha * (1.0f - alpha) / s0) * enl);
+    const int combo = pp.combo[j];
+    const int rank = P.combo[combo].rank;
+    const bool take = P.select_mode == 0 || enb > best_e || (enb == best_e && rank < best_rank);
+    const bool take_fb = !take && best_combo < 0 && combo == P.fallback_combo;
+    if (take) {
+      best_e = enb;
+      best_rank = rank;
+    }
+    if (take || take_fb) {
+      best_combo = combo;
+      best_a = alpha;
+      best_s0 = s0;
+      best_m[0] = s2;
+      best_m[1] = s3;
+      best_m[2] = s6;
+      best_m[3] = s7;
+      if constexpr (FULL8) {
+        best_m[4] = A[j][8] + c2.x;
+        best_m[5] = A[j][9] + c2.y;
+        best_m[6] = A[j][10] + c2.z;
+        best_m[7] = A[j][11] + c2.w;
+      }
+    }
+  }
+}
+
+template <int TH, bool FULL8, int NPX>
+__global__ void __launch_bounds__(32 * TH, 1)
+    nlsar_exact_mean_kernel(const __grid_constant__ FilterParams P, const SceneDesc* __restrict__ scenes,
+                            const SplitSeg* __restrict__ segs, int nseg, const char* __restrict__ vol) {
+  using L = ExactL<TH, FULL8, NPX>;
+  extern __shared__ float4 smem4[];
+  char* sm = reinterpret_cast<char*>(smem4);
+  float4* sCo = reinterpret_cast<float4*>(sm + exact_tables(NPX));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wsh = P.wsh;
+  const int RO = 32 + 2 * wsh, ROH = TH + 2 * wsh, extra = RO * ROH;
+  int lo = 0, hi = nseg - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (segs[mid].tile_begin <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
+  }
+  const SplitSeg& G = segs[lo];
+  const SceneDesc& S = scenes[G.scene];
+  const int lt = (int)blockIdx.x - G.tile_begin;
+  const int ty = lt / G.tiles_x, tx = lt - ty * G.tiles_x;
+  const int vy0 = G.vy0 + ty * TH, vx0 = tx * kTileW;
+  {
+    const int Hp = S.tiles_y * P.tile_h + 2 * P.G;
+    for (int r = warp; r < ROH; r += TH) {
+      const size_t row = (size_t)min(vy0 - wsh + P.G + r, Hp - 1) * S.pitch + (vx0 - wsh + P.G);
+      for (int c = lane; c < RO; c += 32) {
+        sCo[r * RO + c] = S.cori[row + c];
+        if constexpr (FULL8) sCo[extra + r * RO + c] = S.cori2[row + c];
+      }
+    }
+  }
+  // pixels past the last virtual row and column repeat it: their words exist
+  const uint32_t lane_off = (uint32_t)(min(vy0 + warp, G.vy1 - 1) - G.row0) * G.pitch + min(vx0 + lane, S.vW) + wsh;
+  float best_e = -1.0f, alpha = 0.f, s0 = 1.f, m[L::NM];
+  int best_rank = 0x7fffffff, combo = -1;
+#pragma unroll
+  for (int d = 0; d < L::NM; ++d) m[d] = 0.f;
+  for (int ps = 0; ps < P.npass; ++ps) {
+    auto pass = [&](auto np) {
+      exact_pass<TH, FULL8, NPX, decltype(np)::value>(P, ps, vol, G, lane_off, RO, extra, best_e, alpha, s0, best_rank,
+                                                      combo, m);
+    };
+    if constexpr (NPX == 1) {
+      pass(std::integral_constant<int, 1>{});
+    } else if (P.pass[ps].np == 2) {
+      pass(std::integral_constant<int, 2>{});
+    } else {
+      pass(std::integral_constant<int, 3>{});
+    }
+  }
+  const int vy = vy0 + warp, vx = vx0 + lane;
+  const int oy = (vy < S.H - 1) ? vy : (vy == S.vH ? S.H - 1 : -1);
+  const int ox = (vx < S.W - 1) ? vx : (vx == S.vW ? S.W - 1 : -1);
+  if (oy < 0 || ox < 0 || vy >= G.vy1) return;
+  const float4 c = sCo[(warp + wsh) * RO + lane + wsh];
+  const float oma = 1.0f - alpha;
+  const float c00 = oma * m[0] / s0 + alpha * c.x;
+  const float c11 = oma * m[1] / s0 + alpha * c.y;
+  const float cre = oma * m[2] / s0 + alpha * c.z;
+  const float cim = oma * m[3] / s0 + alpha * c.w;
+  const size_t o = (size_t)oy * S.W + ox;
+  if constexpr (FULL8) {
+    const float4 c2 = sCo[extra + (warp + wsh) * RO + lane + wsh];
+    const size_t n = (size_t)S.H * S.W;
+    S.cov_out[o] = c00;
+    S.cov_out[n + o] = oma * m[4] / s0 + alpha * c2.x;
+    S.cov_out[2 * n + o] = cre;
+    S.cov_out[3 * n + o] = cim;
+    S.cov_out[4 * n + o] = oma * m[5] / s0 + alpha * c2.y;
+    S.cov_out[5 * n + o] = oma * m[6] / s0 + alpha * c2.z;
+    S.cov_out[6 * n + o] = c11;
+    S.cov_out[7 * n + o] = oma * m[7] / s0 + alpha * c2.w;
+  } else {
+    const float am = sqrtf(c00), as = sqrtf(c11);
+    const float r = 0.5f * (am + as);
+    S.ref[o] = r * r;
+    S.phase[o] = atan2f(cim, cre);
+    S.coh[o] = sqrtf(cim * cim + cre * cre) / (am * as);
+  }
+  if (S.sel_out) S.sel_out[o] = combo;
+}
+
 // ---------------------------------------------------------------------------
 // host
 // ---------------------------------------------------------------------------
 
 // pass shapes with an index kernel: 0 {1,2,3}, 1 {4,5}, 2..6 the single
-// halves 1..5; -1 none
+// halves 1..5, 7 {1,2}; -1 none
 int pass_shape(const PassParams& p) {
   if (p.np == 3 && p.ph[0] == 1 && p.ph[1] == 2 && p.ph[2] == 3) return 0;
   if (p.np == 2 && p.ph[0] == 4 && p.ph[1] == 5) return 1;
   if (p.np == 1 && p.ph[0] >= 1 && p.ph[0] <= 5) return 1 + p.ph[0];
+  if (p.np == 2 && p.ph[0] == 1 && p.ph[1] == 2) return 7;
   return -1;
 }
-int shape_phm(int shape) { return shape == 0 ? 3 : (shape == 1 ? 5 : shape - 1); }
+int shape_phm(int shape) { return shape == 0 ? 3 : (shape == 1 ? 5 : (shape == 7 ? 2 : shape - 1)); }
 int shape_vc(int shape) { return 128 - 8 * ((shape_phm(shape) + 3) / 4); }
 
-template <int PH0, int PH1, int PH2>
+template <int PH0, int PH1, int PH2, bool EXACT>
 cudaError_t launch_index_t(const FilterParams& F, const SceneDesc* scenes, const SplitSeg* segs, int nseg,
                            const PassList& passes, int slot, char* vol, dim3 grid, size_t smem,
                            cudaStream_t st) {
   static size_t allowed[kMaxDevices];
-  const cudaError_t e = allow_dynamic_smem((const void*)nlsar_index_kernel<PH0, PH1, PH2>, smem, allowed);
+  const cudaError_t e = allow_dynamic_smem((const void*)nlsar_index_kernel<PH0, PH1, PH2, EXACT>, smem, allowed);
   if (e != cudaSuccess) return e;
-  nlsar_index_kernel<PH0, PH1, PH2><<<grid, kIdxThreads, smem, st>>>(F, scenes, segs, nseg, passes, slot, vol);
+  nlsar_index_kernel<PH0, PH1, PH2, EXACT><<<grid, kIdxThreads, smem, st>>>(F, scenes, segs, nseg, passes, slot, vol);
   return cudaGetLastError();
 }
 
@@ -464,6 +718,26 @@ cudaError_t launch_mean_th(int th, const FilterParams& F, const SceneDesc* scene
   return launch_mean_t<tall_tile(FULL8), FULL8, NPX>(F, scenes, segs, nseg, vol, tiles, st);
 }
 
+template <int TH, bool FULL8, int NPX>
+cudaError_t launch_exact_t(const FilterParams& F, const SceneDesc* scenes, const SplitSeg* segs, int nseg,
+                           const char* vol, int tiles, cudaStream_t st) {
+  const size_t smem = exact_smem(F.wsh, TH, FULL8, NPX);
+  static size_t allowed[kMaxDevices];
+  const cudaError_t e =
+      allow_dynamic_smem((const void*)nlsar_exact_mean_kernel<TH, FULL8, NPX>, kSplitSmem, allowed);
+  if (e != cudaSuccess) return e;
+  nlsar_exact_mean_kernel<TH, FULL8, NPX><<<tiles, 32 * TH, smem, st>>>(F, scenes, segs, nseg, vol);
+  return cudaGetLastError();
+}
+
+template <bool FULL8, int NPX>
+cudaError_t launch_exact_th(int th, const FilterParams& F, const SceneDesc* scenes, const SplitSeg* segs, int nseg,
+                            const char* vol, int tiles, cudaStream_t st) {
+  if (th == 8) return launch_exact_t<8, FULL8, NPX>(F, scenes, segs, nseg, vol, tiles, st);
+  if (th == 16) return launch_exact_t<16, FULL8, NPX>(F, scenes, segs, nseg, vol, tiles, st);
+  return launch_exact_t<tall_tile(FULL8), FULL8, NPX>(F, scenes, segs, nseg, vol, tiles, st);
+}
+
 bool single_patches(const FilterParams& F) {
   for (int i = 0; i < F.npass; ++i)
     if (F.pass[i].np > 1) return false;
@@ -478,7 +752,26 @@ int div_up(int a, int b) { return (a + b - 1) / b; }
 
 bool split_supported(const Plan& pl) {
   const FilterParams& F = pl.P;
-  return F.prec == 0 && !F.withhold_staging && pl.fast && split_tables_ok(pl);
+  if (F.prec != 0 || F.withhold_staging || !split_tables_ok(pl)) return false;
+  if (pl.fast) return true;
+  // settings of the kernel in nlsar_kernels.cu: passes that the index kernel
+  // has (their sizes in any scale), and a window whose staged planes fit
+  if (pl.generic_only || F.npass < 1) return false;
+  int shapes = 0, seen[kMaxPasses];
+  for (int i = 0; i < F.npass; ++i) {
+    const int s = pass_shape(F.pass[i]);
+    if (s < 0) return false;
+    int k = 0;
+    while (k < shapes && seen[k] != s) ++k;
+    if (k == shapes) seen[shapes++] = s;
+    if (idx_smem(F.wsh, shape_phm(s), 8) > kSplitSmem) return false;
+  }
+  const int npx = single_patches(F) ? 1 : 3;
+  if (npx == 3)
+    for (int i = 0; i < F.npass; ++i)
+      if (F.pass[i].np == 1) return false;  // the mean kernels take passes of one size alone
+  return shapes <= kSplitShapes && F.wsh >= 1 && idx_left(F.wsh) + 128 + F.wsh <= 32 * 6 &&
+         exact_smem(F.wsh, tall_tile(pl.full8), pl.full8, npx) <= kSplitSmem;
 }
 
 bool split_tables_ok(const Plan& pl) {
@@ -542,13 +835,16 @@ bool split_layout(const Plan& pl, const std::vector<SceneGeom>& geo, const std::
       s.rows = s.vy1 - s.row0;
       s.pitch = pitch;
       s.tiles_x = div_up(g.vW + 1, kTileW);
-      // the mean kernel's word offsets within a pass are 32-bit
+      // (a large window's volume of one tile row can exceed the budget: the
+      // kernel of nlsar_kernels.cu needs none)
+      // the mean kernels' word offsets within a pass are 32-bit
       if ((size_t)nhalf * s.rows * pitch > 0x3fffffff) return false;
       size_t bytes = 0;
       for (int p = 0; p < F.npass; ++p) {
         s.pass[p] = bytes;
         bytes += ((size_t)nhalf * s.rows * pitch * word_bytes(F.pass[p].np) + 255) / 256 * 256;
       }
+      if (!pl.fast && bytes > kSplitBudgetBytes) return false;
       if (out.chunks.empty() || (used && used + bytes > budget)) {
         close_chunk();
         out.chunks.push_back(SplitChunk{});
@@ -646,24 +942,34 @@ cudaError_t launch_split(const Plan& pl, const FilterParams& F, const SplitLayou
     auto go = [&](auto launch) {
       return launch(F, d_scenes, segs, nseg, lay.passes[k], k, vol, grid, c.idx_smem[k], st);
     };
-    switch (lay.shape[k]) {
-      case 0: e = go(launch_index_t<1, 2, 3>); break;
-      case 1: e = go(launch_index_t<4, 5, -1>); break;
-      case 2: e = go(launch_index_t<1, -1, -1>); break;
-      case 3: e = go(launch_index_t<2, -1, -1>); break;
-      case 4: e = go(launch_index_t<3, -1, -1>); break;
-      case 5: e = go(launch_index_t<4, -1, -1>); break;
-      case 6: e = go(launch_index_t<5, -1, -1>); break;
-      default: e = cudaErrorInvalidValue;
-    }
+    auto index = [&](auto exact) {
+      constexpr bool EXACT = decltype(exact)::value;
+      switch (lay.shape[k]) {
+        case 0: return go(launch_index_t<1, 2, 3, EXACT>);
+        case 1: return go(launch_index_t<4, 5, -1, EXACT>);
+        case 2: return go(launch_index_t<1, -1, -1, EXACT>);
+        case 3: return go(launch_index_t<2, -1, -1, EXACT>);
+        case 4: return go(launch_index_t<3, -1, -1, EXACT>);
+        case 5: return go(launch_index_t<4, -1, -1, EXACT>);
+        case 6: return go(launch_index_t<5, -1, -1, EXACT>);
+        case 7: return EXACT ? go(launch_index_t<1, 2, -1, true>) : cudaErrorInvalidValue;
+        default: return cudaErrorInvalidValue;
+      }
+    };
+    e = pl.fast ? index(std::false_type{}) : index(std::true_type{});
   }
   if (e != cudaSuccess) return e;
   const bool single = single_patches(F);
-  if (pl.full8)
-    return single ? launch_mean_th<true, 1>(c.th, F, d_scenes, segs, nseg, vol, c.tiles, st)
-                  : launch_mean_th<true, 3>(c.th, F, d_scenes, segs, nseg, vol, c.tiles, st);
-  return single ? launch_mean_th<false, 1>(c.th, F, d_scenes, segs, nseg, vol, c.tiles, st)
-                : launch_mean_th<false, 3>(c.th, F, d_scenes, segs, nseg, vol, c.tiles, st);
+  auto mean = [&](auto full8, auto npx) {
+    constexpr bool FULL8 = decltype(full8)::value;
+    constexpr int NPX = decltype(npx)::value;
+    return pl.fast ? launch_mean_th<FULL8, NPX>(c.th, F, d_scenes, segs, nseg, vol, c.tiles, st)
+                   : launch_exact_th<FULL8, NPX>(c.th, F, d_scenes, segs, nseg, vol, c.tiles, st);
+  };
+  using one = std::integral_constant<int, 1>;
+  using three = std::integral_constant<int, 3>;
+  if (pl.full8) return single ? mean(std::true_type{}, one{}) : mean(std::true_type{}, three{});
+  return single ? mean(std::false_type{}, one{}) : mean(std::false_type{}, three{});
 }
 
 }  // namespace dcl

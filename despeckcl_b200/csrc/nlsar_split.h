@@ -57,8 +57,9 @@ struct SplitLayout {
   PassList passes[kSplitShapes];
 };
 
-// Whether the two-kernel path serves a call (the specialised kernel's shapes
-// in its default arithmetic, tables that fit byte codes).
+// Whether the two-kernel path serves a call: the specialised kernel's shapes
+// in its default arithmetic, or other windows with passes of the same patch
+// sizes or {3,5}; tables that fit byte codes.
 bool split_supported(const Plan& pl);
 // Whether the weight tables of a plan's passes fit byte codes.
 bool split_tables_ok(const Plan& pl);

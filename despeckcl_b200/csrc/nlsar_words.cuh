@@ -53,7 +53,8 @@ __device__ __forceinline__ void store_words(typename WordOf<NP>::T* out, const u
 // k rows, top down), so a vertical sum costs 2 ph adds, two columns per packed
 // add, and no loads.  A smaller patch is complete PHM - ph rows before the
 // largest, so its code waits in `pend`.
-template <int PH0, int PH1, int PH2>
+// EXACT: the table index as nlsar_kernels.cu takes it, by a rounded division.
+template <int PH0, int PH1, int PH2, bool EXACT = false>
 struct WordWalk {
   static constexpr int NP = np_of<PH0, PH1, PH2>();
   static constexpr int PHM = cmax(PH0, cmax(PH1, PH2));
@@ -62,7 +63,7 @@ struct WordWalk {
   static constexpr int ND = PHM - PH0;         // rows the first patch's code waits
   static_assert(PH0 >= 1 && 4 * HL >= PHM, "pass shape");
 
-  float inv_span[NP], nbias[NP], lm1[NP], dmax[NP];
+  float inv_span[NP], nbias[NP], lm1[NP], dmax[NP];  // EXACT: the span, the lower end
   float2 vs[NP][2 * PHM][2];  // vs[j][k]: last k + 1 rows of patch j, columns in pairs
   uint32_t pend[ND > 0 ? ND : 1][4];
 
@@ -71,8 +72,8 @@ struct WordWalk {
 #pragma unroll
     for (int j = 0; j < NP; ++j) {
       const ComboParams& cp = P.combo[pp.combo[j]];
-      inv_span[j] = 1.0f / cp.span;
-      nbias[j] = -cp.dmin * inv_span[j];
+      inv_span[j] = EXACT ? cp.span : 1.0f / cp.span;
+      nbias[j] = EXACT ? cp.dmin : -cp.dmin * inv_span[j];
       lm1[j] = cp.lm1;
       dmax[j] = cp.dmax;
       if (log2_units) {
@@ -140,6 +141,16 @@ struct WordWalk {
 #pragma unroll
         for (int k = n - 1; k > 0; --k) vs[j][k][q] = __fadd2_rn(vs[j][k - 1][q], h);
         vs[j][0][q] = h;
+        if constexpr (EXACT) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float d = e ? d2.y : d2.x;
+            const float dc = fminf(fmaxf(d, nbias[j]), dmax[j]);
+            const uint32_t code = (uint32_t)__fmul_rn(__fdiv_rn(__fsub_rn(dc, nbias[j]), inv_span[j]), lm1[j]);
+            field[j][2 * q + e] = d > dmax[j] ? (uint32_t)kZeroCode : min(code, (uint32_t)kZeroCode - 1);
+          }
+          continue;
+        }
         // saturating FMA (clamps, NaN to 0), round-toward-zero add of 2^23:
         // the low mantissa bits are the index; d > dmax: weight 0
         const float2 u2 = make_float2(__saturatef(fmaf(d2.x, inv_span[j], nbias[j])),

@@ -62,3 +62,57 @@ def test_two_kernel_3x3_path_equals_fused_kernel(shape, patches, scales, monkeyp
         monkeypatch.setenv("DESPECKCL_B200_TEST_WITHHOLD_STAGING", "1")
         want = dcl.nlsar(c, 21, patches, scales, _STATS[key], select_mode=mode)
         np.testing.assert_array_equal(got.view(np.float32), want.view(np.float32))
+
+
+# settings without a specialised fused kernel: other windows, patches {3,5};
+# the staging switch keeps them on the general kernel, which has no staging
+# copies to withhold.  Statistics of a larger patch than the call's make the
+# reference's selection fall back to its first combination with alpha 0.
+@pytest.mark.parametrize("search", [3, 5, 15, 21, 23, 39])
+@pytest.mark.parametrize("patches,scales,trained", [([3, 5], [1, 3], [3, 5]), ([3, 5, 7], [1, 3], [3, 5, 7]),
+                                                    ([5], [1, 3], [5]), ([3, 5, 7, 9, 11], [3], [3, 5, 7, 9, 11]),
+                                                    ([3, 5], [3], [3, 5, 7]), ([9], [1], [9]), ([11], [3], [11])])
+def test_other_settings_equal_general_kernel(search, patches, scales, trained, monkeypatch):
+    st = _stats(trained, scales)
+    shapes = [(1, 1), (2, 40), (33, 17), (71, 131)]
+    scenes = [synthetic.insar_scene(*s, 5) for s in shapes]
+    scenes[2][0][3:9, 2:12] = 0
+    scenes[2][1][3:9, 2:12] = 0
+    scenes[3][0][20, 30] = np.inf
+    scenes[3][1][50, 100] = np.nan
+    dev = [tuple(torch.from_numpy(x).cuda() for x in s) for s in scenes]
+    covs = []
+    for a1, a2, ph in scenes:
+        z = a1 * a2 * np.exp(1j * ph)
+        covs.append(np.array([[a1 * a1, z], [z.conj(), a2 * a2]]).astype(np.complex64))
+    for mode in ("argmax_enl", "reference"):
+        if search == 21 and (patches != [3, 5] or mode == "reference"):
+            continue  # the specialised kernel's
+
+        def attempt(call):
+            try:
+                return [np.asarray(o.cpu() if hasattr(o, "cpu") else o) for o in call()]
+            except dcl.DespeckclError as e:  # the largest windows and patches have no room, either way
+                assert "too large for shared memory" in str(e)
+                return [np.zeros(0)]
+
+        def run():
+            args = (search, patches, scales, st)
+            out = []
+            for a in dev:
+                out += attempt(lambda: dcl.nlsar_insar_device(*a, *args, select_mode=mode))
+            out += attempt(lambda: [o for scene in dcl.nlsar_insar_batch_device(dev, *args, select_mode=mode)
+                                    for o in scene])
+            for s in scenes:
+                out += attempt(lambda: dcl.nlsar_insar(*s, *args, select_mode=mode))
+            for c in covs:
+                out += attempt(lambda: [dcl.nlsar(c, *args, select_mode=mode).view(np.float32)])
+            return out
+
+        monkeypatch.delenv("DESPECKCL_B200_TEST_WITHHOLD_STAGING", raising=False)
+        got = run()
+        monkeypatch.setenv("DESPECKCL_B200_TEST_WITHHOLD_STAGING", "1")
+        want = run()
+        assert len(got) == len(want)
+        for g, w in zip(got, want):
+            np.testing.assert_array_equal(g, w)
