@@ -822,7 +822,9 @@ bool split_layout(const Plan& pl, const std::vector<SceneGeom>& geo, const std::
     // bytes of one row of one half-window offset, all passes
     size_t row = 0;
     for (int p = 0; p < F.npass; ++p) row += (size_t)pitch * word_bytes(F.pass[p].np);
-    const long long fit = (long long)(budget / (row * nhalf)) - F.wsh;
+    // the mean kernels' word offsets within a pass are 32-bit
+    const long long words = 0x3fffffffLL / ((long long)nhalf * pitch);
+    const long long fit = std::min((long long)(budget / (row * nhalf)), words) - F.wsh;
     const int most = std::max(big, (int)std::min<long long>(fit, 1 << 20) / big * big);
     const int n = row1 - j.row0;
     const int step = div_up(div_up(n, div_up(n, most)), big) * big;
@@ -835,15 +837,15 @@ bool split_layout(const Plan& pl, const std::vector<SceneGeom>& geo, const std::
       s.rows = s.vy1 - s.row0;
       s.pitch = pitch;
       s.tiles_x = div_up(g.vW + 1, kTileW);
-      // (a large window's volume of one tile row can exceed the budget: the
-      // kernel of nlsar_kernels.cu needs none)
-      // the mean kernels' word offsets within a pass are 32-bit
+      // a tile row's words do not fit
       if ((size_t)nhalf * s.rows * pitch > 0x3fffffff) return false;
       size_t bytes = 0;
       for (int p = 0; p < F.npass; ++p) {
         s.pass[p] = bytes;
         bytes += ((size_t)nhalf * s.rows * pitch * word_bytes(F.pass[p].np) + 255) / 256 * 256;
       }
+      // (a large window's volume of one tile row can exceed the budget: the
+      // kernel of nlsar_kernels.cu needs none)
       if (!pl.fast && bytes > kSplitBudgetBytes) return false;
       if (out.chunks.empty() || (used && used + bytes > budget)) {
         close_chunk();

@@ -64,6 +64,22 @@ def test_two_kernel_3x3_path_equals_fused_kernel(shape, patches, scales, monkeyp
         np.testing.assert_array_equal(got.view(np.float32), want.view(np.float32))
 
 
+# one byte per weight: more than 2^30 of them in 2 GiB, so segments are cut by
+# the 32-bit word offsets instead
+@pytest.mark.parametrize("shape", [(2300, 2301), (5003, 1100)])
+def test_segments_cut_by_word_offsets(shape):
+    st = _stats([3, 5, 7], [1, 3])
+    a = [torch.from_numpy(x).cuda() for x in synthetic.insar_scene(*shape, 78)]
+    got = dcl.nlsar_insar_device(*a, 21, [3, 5, 7], [1, 3], st, select_mode="reference")
+    b = dcl.NlsarBatch([tuple(a)], 21, [3, 5, 7], [1, 3], st, select_mode="reference", graph=False, autotune=False,
+                       variant=1)
+    want = b.run()[0]
+    torch.cuda.synchronize()
+    for g, w in zip(got, want):
+        np.testing.assert_array_equal(g.cpu().numpy(), w.cpu().numpy())
+    b.close()
+
+
 # settings without a specialised fused kernel: other windows, patches {3,5};
 # the staging switch keeps them on the general kernel, which has no staging
 # copies to withhold.  Statistics of a larger patch than the call's make the
