@@ -27,9 +27,9 @@
 // (sum w, w^2, w I_d^2 for d = 0..2, and w times each of the 18 planes, read
 // through the L1 cache); the epilogue derives ENL, alpha and ENL', selects and
 // blends with the centre pixel.  Search 21 with patches {3,5,7} (or one of
-// them) runs nlsar3_fast_kernel instead (where nlsar_split3.cu has no memory for its
-// volumes, else the three kernels there), which splits each pixel's
-// accumulators over two threads.
+// them) runs nlsar3_fast_kernel instead, which splits each pixel's
+// accumulators over two threads.  Both filter only where nlsar_split3.cu does
+// not: no memory for its volumes, tables or patch sizes it has no codes for.
 
 #include <cuda_runtime.h>
 
@@ -795,7 +795,11 @@ int fast3_shape(const FilterParams& F) {
 }
 
 // whether the specialised 3x3 kernel has the call's pass shapes
+}  // namespace
+
 bool fast3_supported(const FilterParams& F) { return fast3_shape(F) != 0; }
+
+namespace {
 
 // the specialised 3x3 kernel, for the plans fast3_supported() accepts
 cudaError_t launch3_fast(const FilterParams& F, const Scene3& S, unsigned tiles, cudaStream_t st) {
@@ -870,7 +874,7 @@ static int plan3(const Plan& pl0, int H, int W, float* cout, Run3& r, cudaStream
   // device has no room for the usual one, the fused kernel where it has none
   r.sms = sm_count(dev);
   size_t budget = kSplitBudgetBytes;
-  if (r.pl.fast && fast3_supported(F) && !F.withhold_staging) r.split = split3_layout(r.pl, S, budget);
+  if (!F.withhold_staging) r.split = split3_layout(r.pl, S, budget);
   const size_t fixed = (frame_bytes + 255) / 256 * 256 + (wtab_bytes + 255) / 256 * 256;
   cudaError_t e = cudaSuccess;
   for (;;) {

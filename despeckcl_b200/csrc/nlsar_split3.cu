@@ -14,11 +14,18 @@
 //
 // The fused kernel spent 4.57 ms on 509 x 512 with patches {3,5,7} and scales
 // {1,3}.
+//
+// Settings of the general kernel (nlsar3_kernel: other windows, patches {3,5},
+// 9 or 11 alone) take the same three steps with its arithmetic and summation
+// order, for its bits (EXACT, exact3_mean_kernel): 280 x 290 with {3,5,7} and
+// search 15 3.72 -> 0.82 ms, search 23 8.60 -> 1.72 ms, {3,5} and search 21
+// 5.30 -> 1.23 ms.
 
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "dcl_internal.h"
 #include "nlsar_split.h"
@@ -40,6 +47,8 @@ __host__ __device__ inline size_t sim3_smem(int wsh) { return (size_t)(kSimTH + 
 // One block: 32 x 16 pixels of the volume, two per thread (8 rows apart), the
 // offsets z, z + Z, ..  The nine reals and ln det of a staged pixel are two
 // float4 and one float2 plane; lanes read consecutive pixels.
+// EXACT: with the arithmetic of nlsar3_kernel (nlsar_dim3.cu).
+template <bool EXACT>
 __global__ void __launch_bounds__(kSimThreads, 3)
     sim3_kernel(const float* __restrict__ s9, const float* __restrict__ ld, int Hp, int Wp, int pitch, size_t plane,
                 int wsh, float c2d, int fy0, int fx0, float* __restrict__ sims, int srows, int spitch) {
@@ -89,8 +98,13 @@ __global__ void __launch_bounds__(kSimThreads, 3)
       const float2 nc = sC[ni + 8 * p * RW];
       const float sum[9] = {a[p].x + na.x, a[p].y + na.y, a[p].z + na.z, a[p].w + na.w, b[p].x + nb.x,
                             b[p].y + nb.y, b[p].z + nb.z, b[p].w + nb.w, c[p].x + nc.x};
-      const float t = (c[p].y + nc.y) + c2d;
-      float sim = fmaf(2.0f * 0.69314718f, __log2f(det3f(sum)), -t);
+      float sim;
+      if (EXACT) {  // a lower-half offset: neighbour first (copy_symm_weights.cl:66-74)
+        sim = -(((c2d + nc.y) + c[p].y) - 2.0f * logf(det3f(sum)));
+      } else {
+        const float t = (c[p].y + nc.y) + c2d;
+        sim = fmaf(2.0f * 0.69314718f, __log2f(det3f(sum)), -t);
+      }
       if (sim != sim) sim = 0.0f;
       if (in_c && r0 + warp + 8 * p < srows) out[u * splane + (size_t)(8 * p) * spitch] = sim;
     }
@@ -104,11 +118,11 @@ constexpr int kWordsWarps = 8;
 // One warp: a strip of VC columns x R rows of a pass's words for one offset.
 // Similarity row 0 is the words' row 0 less the call's largest patch half
 // `halo`.
-template <int PH0, int PH1, int PH2>
+template <int PH0, int PH1, int PH2, bool EXACT>
 __global__ void __launch_bounds__(32 * kWordsWarps, 2)
     words3_kernel(const __grid_constant__ FilterParams P, int ps, const float* __restrict__ sims, int srows, int spitch,
                   int halo, char* __restrict__ words, int rows, int pitch, int R, int nbx, int items) {
-  using Walk = WordWalk<PH0, PH1, PH2>;
+  using Walk = WordWalk<PH0, PH1, PH2, EXACT>;
   using Word = typename WordOf<Walk::NP>::T;
   constexpr int PHM = Walk::PHM;
   const int lane = threadIdx.x & 31;
@@ -384,6 +398,202 @@ __global__ void __launch_bounds__(L::THREADS, 1)
   }
 }
 
+// Means as nlsar3_kernel sums them, any window: the offsets in pairs, the upper
+// half's first and its mirror after it, the centre last.  Tile, tables and
+// staged planes as above, the window at run time.
+__host__ __device__ constexpr int exact3_tables(int npx) { return 256 * 256 + (npx > 2 ? 256 * 128 : 0); }
+inline size_t exact3_smem(int wsh, int th, int npx) {
+  return exact3_tables(npx) + (size_t)(32 + 2 * wsh) * (th + 2 * wsh) * 72;
+}
+constexpr int kPairs3 = 4;  // offset pairs whose words are in flight
+
+template <int TH, int NPX, int NP>
+__device__ __forceinline__ void exact3_pass(const FilterParams& P, int ps, const char* __restrict__ pass_words,
+                                            int rows, int wpitch, uint32_t lane_off, int RO, int PLANE,
+                                            Best3x& best) {
+  using Word = typename WordOf<NP>::T;
+  extern __shared__ float4 smem4[];
+  char* sm = reinterpret_cast<char*>(smem4);
+  const PassParams& pp = P.pass[ps];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wsh = P.wsh;
+  __syncthreads();  // the previous pass's tables are no longer read
+  for (int i = tid; i < NP * 256 * 8; i += 32 * TH) {
+    const int j = i >> 11, e = (i >> 3) & 255;
+    const float w = e == kZeroCode ? 0.0f : P.wtab[pp.combo[j] * kMaxLut + e];
+    const int at = j < 2 ? e * 256 + j * 128 : 65536 + e * 128;
+    *reinterpret_cast<float4*>(sm + at + (i & 7) * 16) = make_float4(w, w, w, w);
+  }
+  __syncthreads();
+  float A[NP][5], m[NP][18];  // sum w, w^2, w I_d^2; of w times the planes
+#pragma unroll
+  for (int j = 0; j < NP; ++j) {
+#pragma unroll
+    for (int a = 0; a < 5; ++a) A[j][a] = 0.0f;
+#pragma unroll
+    for (int a = 0; a < 18; ++a) m[j][a] = 0.0f;
+  }
+  const uint32_t lane4 = 4u * lane;
+  const float4* tile = reinterpret_cast<const float4*>(sm + exact3_tables(NPX));
+  const float2* tile2 = reinterpret_cast<const float2*>(tile + 4 * PLANE);
+  auto planes = [&](int i, float (&v)[18]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float4 t = tile[q * PLANE + i];
+      v[4 * q] = t.x;
+      v[4 * q + 1] = t.y;
+      v[4 * q + 2] = t.z;
+      v[4 * q + 3] = t.w;
+    }
+    const float2 t = tile2[i];
+    v[16] = t.x;
+    v[17] = t.y;
+  };
+  auto accumulate = [&](uint32_t word, int i) {
+    float v[18], i2[3];
+    planes(i, v);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) i2[d] = __fmul_rn(v[diag_plane(d)], v[diag_plane(d)]);
+#pragma unroll
+    for (int j = 0; j < NP; ++j) {
+      const int at = j == 2 ? 65536 + (int)(((word >> 9) & 0x7F80u) | lane4)
+                            : j * 128 + (int)__byte_perm(word, lane4, 0x5504 | (j << 4));
+      const float w = *reinterpret_cast<const float*>(sm + at);
+      A[j][0] = __fadd_rn(A[j][0], w);
+      A[j][1] = __fmaf_rn(w, w, A[j][1]);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) A[j][2 + q] = __fmaf_rn(w, i2[q], A[j][2 + q]);
+#pragma unroll
+      for (int q = 0; q < 18; ++q) m[j][q] = __fmaf_rn(w, v[q], m[j][q]);
+    }
+  };
+  // pairs and their words as in nlsar_split.cu
+  const uint32_t plane = (uint32_t)rows * wpitch;
+  const Word* words = reinterpret_cast<const Word*>(pass_words);
+  const int nhalf = P.n_off / 2;
+  uint32_t up[kPairs3], down[kPairs3];
+  int li = nhalf - 1, ldy = wsh, ldx = wsh;  // next pair to load
+  auto load = [&](int k) {
+    if (li >= 0) {
+      const uint32_t off = lane_off + (uint32_t)li * plane;
+      down[k] = __ldcg(words + off);
+      up[k] = __ldcg(words + (off - (uint32_t)(ldy * wpitch + ldx)));
+      --li;
+      if (--ldx < -wsh) ldx = wsh, --ldy;
+    }
+  };
+#pragma unroll
+  for (int k = 0; k < kPairs3; ++k) load(k);
+  const int ci = (warp + wsh) * RO + lane + wsh;
+  int d = wsh * RO + wsh, dx = wsh;  // place of x + o after x
+  for (int i = nhalf - 1; i >= 0; i -= kPairs3) {
+#pragma unroll
+    for (int k = 0; k < kPairs3; ++k) {
+      if (i - k < 0) break;
+      const uint32_t wu = up[k], wd = down[k];
+      load(k);
+      accumulate(wu, ci - d);
+      accumulate(wd, ci + d);
+      --d;
+      if (--dx < -wsh) dx = wsh, d -= RO - 2 * wsh - 1;
+    }
+  }
+  // centre weight 1, statistics, alpha, ENL', selection (nlsar_dim3.cu)
+  float c[18];
+  planes(ci, c);
+#pragma unroll
+  for (int j = 0; j < NP; ++j) {
+    const float s0 = A[j][0] + 1.0f, s1 = A[j][1] + 1.0f;
+    const float enl = s0 * s0 / s1;
+    float alpha = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const float cd = c[diag_plane(q)];
+      const float in = (m[j][diag_plane(q)] + cd) / s0;
+      const float var = __fmaf_rn(cd, cd, A[j][2 + q]) / s0 - in * in;
+      alpha = fmaxf(alpha, fmaxf(0.0f, (var - in * in) / var));
+    }
+    if (P.alpha_zero) alpha = 0.0f;
+    const float oma = 1.0f - alpha;
+    const float enb = enl / (oma * oma + (alpha * alpha + 2.0f * alpha * (1.0f - alpha) / s0) * enl);
+    const int combo = pp.combo[j];
+    const int rank = P.combo[combo].rank;
+    const bool take = (P.select_mode == 0) || (enb > best.e) || (enb == best.e && rank < best.rank);
+    const bool take_fb = !take && best.combo < 0 && combo == P.fallback_combo;
+    if (take) {
+      best.e = enb;
+      best.rank = rank;
+    }
+    if (take || take_fb) {
+      best.combo = combo;
+      best.a = alpha;
+      best.s0 = s0;
+#pragma unroll
+      for (int q = 0; q < 18; ++q) best.m[q] = m[j][q] + c[q];
+    }
+  }
+}
+
+template <int TH, int NPX>
+__global__ void __launch_bounds__(32 * TH, 1)
+    exact3_mean_kernel(const __grid_constant__ FilterParams P, const __grid_constant__ Scene3 S, int Hp,
+                       const char* __restrict__ vol, const __grid_constant__ WordOffsets wo, int vy0s, int vy1,
+                       int rows, int wpitch, int tiles_x) {
+  extern __shared__ float4 smem4[];
+  char* sm = reinterpret_cast<char*>(smem4);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wsh = P.wsh;
+  const int RO = 32 + 2 * wsh, ROH = TH + 2 * wsh, PLANE = RO * ROH;
+  const int ty = blockIdx.x / tiles_x, tx = blockIdx.x - ty * tiles_x;
+  const int vy0 = vy0s + ty * TH, vx0 = tx * 32;
+  float4* tile = reinterpret_cast<float4*>(sm + exact3_tables(NPX));
+  float2* tile2 = reinterpret_cast<float2*>(tile + 4 * PLANE);
+  for (int r = warp; r < ROH; r += TH) {
+    const size_t row = (size_t)min(vy0 - wsh + P.G + r, Hp - 1) * S.pitch + (vx0 - wsh + P.G);
+    for (int c = lane; c < RO; c += 32) {
+      const float* g = S.c18 + row + c;
+      const int i = r * RO + c;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        tile[q * PLANE + i] = make_float4(g[(4 * q) * S.plane], g[(4 * q + 1) * S.plane], g[(4 * q + 2) * S.plane],
+                                          g[(4 * q + 3) * S.plane]);
+      tile2[i] = make_float2(g[16 * S.plane], g[17 * S.plane]);
+    }
+  }
+  // pixels past the last virtual row and column repeat it: their words exist
+  const uint32_t lane_off =
+      (uint32_t)(min(vy0 + warp, vy1 - 1) - vy0s + wsh) * wpitch + min(vx0 + lane, S.vW) + wsh;
+  Best3x best;
+  best.e = -1.0f;
+  best.a = 0.0f;
+  best.s0 = 1.0f;
+  best.rank = 0x7fffffff;
+  best.combo = -1;
+#pragma unroll
+  for (int p = 0; p < 18; ++p) best.m[p] = 0.0f;
+  for (int ps = 0; ps < P.npass; ++ps) {
+    const char* w = vol + wo.at[ps];
+    if constexpr (NPX == 1) {
+      exact3_pass<TH, NPX, 1>(P, ps, w, rows, wpitch, lane_off, RO, PLANE, best);
+    } else if (P.pass[ps].np == 2) {
+      exact3_pass<TH, NPX, 2>(P, ps, w, rows, wpitch, lane_off, RO, PLANE, best);
+    } else {
+      exact3_pass<TH, NPX, 3>(P, ps, w, rows, wpitch, lane_off, RO, PLANE, best);
+    }
+  }
+  const int vy = vy0 + warp, vx = vx0 + lane;
+  const int oy = (vy < S.H - 1) ? vy : (vy == S.vH ? S.H - 1 : -1);
+  const int ox = (vx < S.W - 1) ? vx : (vx == S.vW ? S.W - 1 : -1);
+  if (oy < 0 || ox < 0 || vy >= vy1) return;
+  const size_t n = (size_t)S.H * S.W, o = (size_t)oy * S.W + ox;
+  const int ci = (warp + wsh) * RO + lane + wsh;
+  const float oma = 1.0f - best.a;
+#pragma unroll
+  for (int q = 0; q < 18; ++q) {
+    const float cp = q < 16 ? reinterpret_cast<const float*>(tile + (q / 4) * PLANE + ci)[q & 3]
+                            : reinterpret_cast<const float*>(tile2 + ci)[q & 1];
+    S.out[q * n + o] = oma * best.m[q] / best.s0 + best.a * cp;
+  }
+}
+
 // ---- host ---------------------------------------------------------------------
 
 constexpr int kTall3 = 12;  // rows of the tallest mean tile (segments hold whole tiles of 12 and 8)
@@ -413,10 +623,29 @@ cudaError_t launch_mean3(int th, const FilterParams& F, const Scene3& S, int Hp,
   }
 }
 
-template <int PH0, int PH1, int PH2>
+template <int TH, int NPX>
+cudaError_t launch_exact3_t(const FilterParams& F, const Scene3& S, int Hp, const char* vol, const WordOffsets& wo,
+                            int vy0, int vy1, int rows, int wpitch, int tiles_x, cudaStream_t st) {
+  static size_t allowed[kMaxDevices];
+  const cudaError_t e = allow_dynamic_smem((const void*)exact3_mean_kernel<TH, NPX>, kSplitSmem, allowed);
+  if (e != cudaSuccess) return e;
+  exact3_mean_kernel<TH, NPX><<<tiles_x * div_up(vy1 - vy0, TH), 32 * TH, exact3_smem(F.wsh, TH, NPX), st>>>(
+      F, S, Hp, vol, wo, vy0, vy1, rows, wpitch, tiles_x);
+  return cudaGetLastError();
+}
+
+template <int NPX>
+cudaError_t launch_exact3(int th, const FilterParams& F, const Scene3& S, int Hp, const char* vol,
+                          const WordOffsets& wo, int vy0, int vy1, int rows, int wpitch, int tiles_x,
+                          cudaStream_t st) {
+  return th == 4 ? launch_exact3_t<4, NPX>(F, S, Hp, vol, wo, vy0, vy1, rows, wpitch, tiles_x, st)
+                 : launch_exact3_t<8, NPX>(F, S, Hp, vol, wo, vy0, vy1, rows, wpitch, tiles_x, st);
+}
+
+template <int PH0, int PH1, int PH2, bool EXACT>
 cudaError_t launch_words3(const FilterParams& F, int ps, const float* sims, int srows, int spitch, char* words,
                           int rows, int pitch, int sms, cudaStream_t st) {
-  using Walk = WordWalk<PH0, PH1, PH2>;
+  using Walk = WordWalk<PH0, PH1, PH2, EXACT>;
   const int nbx = div_up(pitch, Walk::VC);
   // strips of up to 64 rows (each walks 2 PHM more); shorter ones where that
   // leaves fewer than 16 warps per SM
@@ -424,16 +653,17 @@ cudaError_t launch_words3(const FilterParams& F, int ps, const float* sims, int 
   const int nhalf = F.n_off / 2;
   while (R > 8 && (long long)nbx * div_up(rows, R) * nhalf < 16LL * sms) R /= 2;
   const int items = nbx * div_up(rows, R);
-  words3_kernel<PH0, PH1, PH2><<<dim3(div_up(items, kWordsWarps), nhalf), 32 * kWordsWarps, 0, st>>>(
+  words3_kernel<PH0, PH1, PH2, EXACT><<<dim3(div_up(items, kWordsWarps), nhalf), 32 * kWordsWarps, 0, st>>>(
       F, ps, sims, srows, spitch, F.phm, words, rows, pitch, R, nbx, items);
   return cudaGetLastError();
 }
 
-// pass shapes: 0 {1,2,3}, 1 {4,5}, 2..4 the single halves 1..3; -1 none
+// pass shapes: 0 {1,2,3}, 1 {4,5}, 2..6 the single halves 1..5, 7 {1,2}; -1 none
 int pass_shape3(const PassParams& p) {
   if (p.np == 3 && p.ph[0] == 1 && p.ph[1] == 2 && p.ph[2] == 3) return 0;
   if (p.np == 2 && p.ph[0] == 4 && p.ph[1] == 5) return 1;
-  if (p.np == 1 && p.ph[0] >= 1 && p.ph[0] <= 3) return 1 + p.ph[0];
+  if (p.np == 1 && p.ph[0] >= 1 && p.ph[0] <= 5) return 1 + p.ph[0];
+  if (p.np == 2 && p.ph[0] == 1 && p.ph[1] == 2) return 7;
   return -1;
 }
 
@@ -443,12 +673,25 @@ Split3 split3_layout(const Plan& pl, const Scene3& S, size_t budget) {
   const FilterParams& F = pl.P;
   Split3 L;
   const int nhalf = F.n_off / 2;
-  if (F.wsh != 10 || !split_tables_ok(pl)) return L;
+  if (!split_tables_ok(pl) || F.npass < 1 || F.wsh < 1) return L;
+  L.exact = !(pl.fast && fast3_supported(F));
+  if (L.exact && (pl.generic_only || F.prec != 0)) return L;
+  // the launches of three kernels outweigh eight offsets of a small scene:
+  // 64 x 70 with search 3 takes 73 us (nlsar3_kernel 61), with search 5 75 us
+  // (112), 280 x 290 with search 3 98 us (124)
+  if (L.exact && F.wsh == 1 && (long long)S.H * S.W < 65536) return L;
   size_t word_row = 0;
+  int np_min = kPatchPerPass, npx = 1;
   for (int i = 0; i < F.npass; ++i) {
     if (pass_shape3(F.pass[i]) < 0) return L;
     word_row += word_bytes(F.pass[i].np);
+    np_min = std::min(np_min, F.pass[i].np);
+    npx = std::max(npx, F.pass[i].np);
   }
+  // passes of one size come alone; the staged window has to fit
+  if (npx > 1 && np_min == 1) return L;
+  npx = npx > 1 ? 3 : 1;
+  if (L.exact && (exact3_smem(F.wsh, 4, npx) > kSplitSmem || sim3_smem(F.wsh) > kSplitSmem)) return L;
   L.pitch = (S.vW + 1 + 2 * F.wsh + 15) / 16 * 16;
   L.spitch = L.pitch + 2 * kSimLeft;
   const size_t srow = (size_t)nhalf * L.spitch * sizeof(float), wrow = (size_t)nhalf * L.pitch * word_row;
@@ -467,6 +710,9 @@ Split3 split3_layout(const Plan& pl, const Scene3& S, size_t budget) {
   for (int i = 0; i < F.npass; ++i)
     words += ((size_t)nhalf * (L.rows + extra_w) * L.pitch * word_bytes(F.pass[i].np) + 255) / 256 * 256;
   L.vol_bytes = L.sim_bytes + words;
+  // a large window's volume of one segment can exceed the budget: nlsar3_kernel
+  // needs none
+  if (L.exact && L.vol_bytes > kSplitBudgetBytes) L.rows = 0;
   return L;
 }
 
@@ -482,7 +728,9 @@ cudaError_t launch_split3(const Plan& pl, const FilterParams& F, const Scene3& S
     at += ((size_t)nhalf * rows * L.pitch * word_bytes(F.pass[i].np) + 255) / 256 * 256;
   }
   static size_t allowed[kMaxDevices];
-  cudaError_t e = allow_dynamic_smem((const void*)sim3_kernel, sim3_smem(F.wsh), allowed);
+  static size_t allowed_exact[kMaxDevices];
+  cudaError_t e = L.exact ? allow_dynamic_smem((const void*)sim3_kernel<true>, kSplitSmem, allowed_exact)
+                          : allow_dynamic_smem((const void*)sim3_kernel<false>, sim3_smem(F.wsh), allowed);
   if (e != cudaSuccess) return e;
   int slot = -1, npx = 1;
   for (int ps = 0; ps < F.npass; ++ps) {
@@ -494,19 +742,30 @@ cudaError_t launch_split3(const Plan& pl, const FilterParams& F, const Scene3& S
       // column -wsh - kSimLeft; offset groups fill four blocks per SM
       dim3 grid(div_up(L.spitch, 32), div_up(srows, kSimTH));
       grid.z = std::max(1, std::min(nhalf, div_up(4 * sms, (int)(grid.x * grid.y))));
-      sim3_kernel<<<grid, kSimThreads, sim3_smem(F.wsh), st>>>(S.s9[slot], S.ld[slot], Hp, Wp, S.pitch, S.plane,
+      const auto sim = L.exact ? sim3_kernel<true> : sim3_kernel<false>;
+      sim<<<grid, kSimThreads, sim3_smem(F.wsh), st>>>(S.s9[slot], S.ld[slot], Hp, Wp, S.pitch, S.plane,
                                                              F.wsh, F.c2d, vy0 - F.wsh - F.phm + F.G,
                                                              F.G - F.wsh - kSimLeft, sims, srows, L.spitch);
       profile_count(1);
     }
     char* words = vol + wo.at[ps];
-    switch (pass_shape3(pp)) {
-      case 0: e = launch_words3<1, 2, 3>(F, ps, sims, srows, L.spitch, words, rows, L.pitch, sms, st); break;
-      case 1: e = launch_words3<4, 5, -1>(F, ps, sims, srows, L.spitch, words, rows, L.pitch, sms, st); break;
-      case 2: e = launch_words3<1, -1, -1>(F, ps, sims, srows, L.spitch, words, rows, L.pitch, sms, st); break;
-      case 3: e = launch_words3<2, -1, -1>(F, ps, sims, srows, L.spitch, words, rows, L.pitch, sms, st); break;
-      default: e = launch_words3<3, -1, -1>(F, ps, sims, srows, L.spitch, words, rows, L.pitch, sms, st); break;
-    }
+    auto codes = [&](auto launch) {
+      return launch(F, ps, sims, srows, L.spitch, words, rows, L.pitch, sms, st);
+    };
+    auto shape = [&](auto exact) {
+      constexpr bool EXACT = decltype(exact)::value;
+      switch (pass_shape3(pp)) {
+        case 0: return codes(launch_words3<1, 2, 3, EXACT>);
+        case 1: return codes(launch_words3<4, 5, -1, EXACT>);
+        case 2: return codes(launch_words3<1, -1, -1, EXACT>);
+        case 3: return codes(launch_words3<2, -1, -1, EXACT>);
+        case 4: return codes(launch_words3<3, -1, -1, EXACT>);
+        case 5: return EXACT ? codes(launch_words3<4, -1, -1, true>) : cudaErrorInvalidValue;
+        case 6: return EXACT ? codes(launch_words3<5, -1, -1, true>) : cudaErrorInvalidValue;
+        default: return EXACT ? codes(launch_words3<1, 2, -1, true>) : cudaErrorInvalidValue;
+      }
+    };
+    e = L.exact ? shape(std::true_type{}) : shape(std::false_type{});
     profile_count(1);
     if (e != cudaSuccess) return e;
   }
@@ -522,6 +781,11 @@ cudaError_t launch_split3(const Plan& pl, const FilterParams& F, const Scene3& S
     }
   }
   profile_count(1);
+  if (L.exact) {
+    const int t = th == 4 || exact3_smem(F.wsh, 8, npx == 1 ? 1 : 3) > kSplitSmem ? 4 : 8;
+    return npx == 1 ? launch_exact3<1>(t, F, S, Hp, vol, wo, vy0, vy1, rows, L.pitch, tiles_x, st)
+                    : launch_exact3<3>(t, F, S, Hp, vol, wo, vy0, vy1, rows, L.pitch, tiles_x, st);
+  }
   return npx == 1 ? launch_mean3<1>(th, F, S, Hp, vol, wo, vy0, vy1, rows, L.pitch, tiles_x, st)
                   : launch_mean3<3>(th, F, S, Hp, vol, wo, vy0, vy1, rows, L.pitch, tiles_x, st);
 }

@@ -41,8 +41,11 @@ struct Scene3 {
 struct Split3 {
   int rows = 0;                     // virtual rows per segment; 0: the call is not served
   int pitch = 0, spitch = 0;        // words, similarities per volume row
+  bool exact = false;               // the settings and arithmetic of nlsar3_kernel
   size_t sim_bytes = 0, vol_bytes = 0;  // similarities of one scale, then the words of every pass
 };
+// Whether nlsar3_fast_kernel has a call's shapes (nlsar_dim3.cu).
+bool fast3_supported(const FilterParams& F);
 // Sizes the segments for `budget` bytes; rows 0 where the plan has no kernels
 // or a row is too wide.
 Split3 split3_layout(const Plan& pl, const Scene3& S, size_t budget);

@@ -132,3 +132,34 @@ def test_other_settings_equal_general_kernel(search, patches, scales, trained, m
         assert len(got) == len(want)
         for g, w in zip(got, want):
             np.testing.assert_array_equal(g, w)
+
+
+@pytest.mark.parametrize("search", [3, 5, 15, 21, 25])
+@pytest.mark.parametrize("patches,scales", [([3, 5], [1, 3]), ([3, 5, 7], [1, 3]), ([9], [1]), ([3, 5, 7, 9, 11], [3])])
+def test_other_3x3_settings_equal_general_kernel(search, patches, scales, monkeypatch):
+    def cov(h, w, seed):
+        rng = np.random.default_rng(seed)
+        z = rng.normal(size=(3, 5)) + 1j * rng.normal(size=(3, 5))
+        x = rng.normal(size=(3, h * w)) + 1j * rng.normal(size=(3, h * w))
+        k = (np.linalg.cholesky(z @ z.conj().T) @ x).reshape(3, h, w) * np.linspace(1, 2, w)
+        return (k[:, None] * k[None, :].conj()).astype(np.complex64)
+
+    key = ("3x3", tuple(patches), tuple(scales))
+    if key not in _STATS:
+        _STATS[key] = dcl.nlsar_train(cov(40, 40, 1), patches, scales)
+    for shape in ((1, 1), (2, 40), (33, 17), (71, 131) if search > 3 else (250, 270)):
+        c = cov(*shape, 2)
+        c[:, :, shape[0] // 2:, : shape[1] // 8] = 0
+        for mode in ("argmax_enl", "reference"):
+            out = []
+            for switch in (False, True):
+                if switch:
+                    monkeypatch.setenv("DESPECKCL_B200_TEST_WITHHOLD_STAGING", "1")
+                else:
+                    monkeypatch.delenv("DESPECKCL_B200_TEST_WITHHOLD_STAGING", raising=False)
+                try:
+                    out.append(dcl.nlsar(c, search, patches, scales, _STATS[key], select_mode=mode).view(np.float32))
+                except dcl.DespeckclError as e:  # the largest windows and patches have no room, either way
+                    assert "too large for shared memory" in str(e)
+                    out.append(np.zeros(0))
+            np.testing.assert_array_equal(*out)
