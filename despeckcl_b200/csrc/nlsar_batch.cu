@@ -279,7 +279,7 @@ extern "C" dcl_nlsar_batch* dcl_nlsar_batch_create(int n, const float* const* a1
   cudaGetDevice(&dev);
   std::vector<SplitJob> jobs;
   for (int i = 0; i < n; ++i) jobs.push_back({i, 0, b->geo[i].vH + 1});
-  size_t budget = kSplitBudgetBytes, seg_bytes = 0;
+  size_t budget = split_budget(), seg_bytes = 0;
   b->split = !(flags & (DCL_BATCH_VARIANT1 | DCL_BATCH_VARIANT2)) && split_supported(b->pl) &&
              split_layout(b->pl, b->geo, jobs, budget, sm_count(dev), b->lay);
   cudaError_t e = cudaSuccess;

@@ -873,7 +873,7 @@ static int plan3(const Plan& pl0, int H, int W, float* cout, Run3& r, cudaStream
   // the two-kernel path where it serves the call; a smaller volume where the
   // device has no room for the usual one, the fused kernel where it has none
   r.sms = sm_count(dev);
-  size_t budget = kSplitBudgetBytes;
+  size_t budget = split_budget();
   if (!F.withhold_staging) r.split = split3_layout(r.pl, S, budget);
   const size_t fixed = (frame_bytes + 255) / 256 * 256 + (wtab_bytes + 255) / 256 * 256;
   cudaError_t e = cudaSuccess;
@@ -948,7 +948,9 @@ static int launch3_rows(const Run3& r, int t0, int t1, cudaStream_t st) {
     const int end = std::min(t1 * kT3H, S.vH + 1);
     e = cudaSuccess;
     for (int y = t0 * kT3H; y < end && e == cudaSuccess; y += r.split.rows)
-      e = launch_split3(r.pl, F, S, r.Hp, r.Wp, r.split, r.vol, y, std::min(y + r.split.rows, end), r.sms, st);
+      for (int x = 0; x <= S.vW && e == cudaSuccess; x += r.split.cols)
+        e = launch_split3(r.pl, F, S, r.Hp, r.Wp, r.split, r.vol, y, std::min(y + r.split.rows, end), x,
+                          std::min(x + r.split.cols, S.vW + 1), r.sms, st);
     return e == cudaSuccess ? DCL_OK : cuda_error(e, "NL-SAR 3x3");
   }
   if (r.pl.fast && fast3_supported(F)) {

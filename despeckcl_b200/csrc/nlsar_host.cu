@@ -556,7 +556,7 @@ int run_device(const Plan& pl0, const std::vector<SceneIO>& io, cudaStream_t st)
   SplitLayout lay;
   std::vector<SplitJob> jobs;
   for (size_t i = 0; i < io.size(); ++i) jobs.push_back({(int)i, 0, geo[i].vH + 1});
-  size_t budget = kSplitBudgetBytes;
+  size_t budget = split_budget();
   bool split = split_supported(pl) && split_layout(pl, geo, jobs, budget, sm_count(dev), lay);
   const size_t desc_bytes = pad256(io.size() * sizeof(SceneDesc));
   const size_t wtab_bytes = pad256(pl.wtab.size() * sizeof(float));
@@ -740,7 +740,7 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
     }
     return true;
   };
-  size_t budget = kSplitBudgetBytes;
+  size_t budget = split_budget();
   bool split = split_supported(pl) && layouts(budget);
   size_t seg_pad = 0;
   char* mem = nullptr;

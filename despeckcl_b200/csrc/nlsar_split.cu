@@ -30,13 +30,15 @@
 // (EXACT, nlsar_exact_mean_kernel), whose results they give bit for bit.
 //
 // The volume of one pass is (sws^2 - 1) / 2 words of 1, 2 or 4 bytes per pixel
-// (220 to 880 B at search 21), so a scene is filtered in segments of rows whose volume fits a budget
-// (kSplitBudgetBytes), index kernel and mean kernel in turn.
+// (220 to 880 B at search 21), so a scene is filtered in segments whose volume
+// fits a budget (kSplitBudgetBytes), index kernel and mean kernel in turn: runs
+// of whole rows, cut in columns where one row of tiles is too much.
 
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <type_traits>
 #include <vector>
@@ -116,10 +118,10 @@ __global__ void __launch_bounds__(kIdxThreads, 1)
   float* sL = reinterpret_cast<float*>(smem4 + nrow * SP);
   {
     // staged column 0 is `left` columns before lane 0's first; volume column
-    // c is virtual column c - wsh.  Coordinates are clamped to the frame: the
+    // c is virtual column vx0 + c - wsh.  Coordinates are clamped to the frame: the
     // pixels a used weight needs are inside it.
     const int Hp = D.tiles_y * P.tile_h + 2 * P.G, Wp = D.tiles_x * kTileW + 2 * P.G;
-    const int fx0 = VC * bx - 4 * HL - wsh - left + P.G, fy0 = S.row0 + r0 - PHM + P.G;
+    const int fx0 = S.vx0 + VC * bx - 4 * HL - wsh - left + P.G, fy0 = S.row0 + r0 - PHM + P.G;
     const int ncol = left + 128 + wsh;
     const float4* cs = D.cs[pp.scale_slot];
     const float* ld = D.ld[pp.scale_slot];
@@ -386,7 +388,7 @@ __global__ void __launch_bounds__(L::THREADS, 1)
   const SceneDesc& S = scenes[G.scene];
   const int lt = (int)blockIdx.x - G.tile_begin;
   const int ty = lt / G.tiles_x, tx = lt - ty * G.tiles_x;
-  const int vy0 = G.vy0 + ty * L::TH, vx0 = tx * kTileW;
+  const int vy0 = G.vy0 + ty * L::TH, vx0 = G.vx0 + tx * kTileW;
 
   // frame rows end at tiles of P.tile_h rows, so the last rows are clamped
   // (outputs that exist never use a clamped one)
@@ -406,8 +408,10 @@ __global__ void __launch_bounds__(L::THREADS, 1)
     if (tid == 0) *reinterpret_cast<float*>(sm + L::OFF_ONE) = 1.0f;
   }
 
-  // pixels past the last virtual row and column repeat it: their words exist
-  const uint32_t lane_off = (uint32_t)(min(vy0 + warp, G.vy1 - 1) - G.row0) * G.pitch + min(vx0 + lane, S.vW) + WSH;
+  // pixels past the segment's last row and the last virtual column repeat it:
+  // their words exist (columns are cut between tiles)
+  const uint32_t lane_off = (uint32_t)(min(vy0 + warp, G.vy1 - 1) - G.row0) * G.pitch +
+                            (uint32_t)(min(vx0 + lane, S.vW) - G.vx0) + WSH;
 
   Best<1, NM> best;
   best.e[0] = -1.0f;
@@ -606,7 +610,7 @@ __global__ void __launch_bounds__(32 * TH, 1)
   const SceneDesc& S = scenes[G.scene];
   const int lt = (int)blockIdx.x - G.tile_begin;
   const int ty = lt / G.tiles_x, tx = lt - ty * G.tiles_x;
-  const int vy0 = G.vy0 + ty * TH, vx0 = tx * kTileW;
+  const int vy0 = G.vy0 + ty * TH, vx0 = G.vx0 + tx * kTileW;
   {
     const int Hp = S.tiles_y * P.tile_h + 2 * P.G;
     for (int r = warp; r < ROH; r += TH) {
@@ -617,8 +621,10 @@ __global__ void __launch_bounds__(32 * TH, 1)
       }
     }
   }
-  // pixels past the last virtual row and column repeat it: their words exist
-  const uint32_t lane_off = (uint32_t)(min(vy0 + warp, G.vy1 - 1) - G.row0) * G.pitch + min(vx0 + lane, S.vW) + wsh;
+  // pixels past the segment's last row and the last virtual column repeat it:
+  // their words exist (columns are cut between tiles)
+  const uint32_t lane_off = (uint32_t)(min(vy0 + warp, G.vy1 - 1) - G.row0) * G.pitch +
+                            (uint32_t)(min(vx0 + lane, S.vW) - G.vx0) + wsh;
   float best_e = -1.0f, alpha = 0.f, s0 = 1.f, m[L::NM];
   int best_rank = 0x7fffffff, combo = -1;
 #pragma unroll
@@ -785,10 +791,20 @@ bool split_tables_ok(const Plan& pl) {
   return true;
 }
 
+size_t split_budget() {
+  if (const char* v = std::getenv("DESPECKCL_B200_VOLUME_MIB")) {
+    char* end = nullptr;
+    const unsigned long long mib = std::strtoull(v, &end, 10);
+    if (end != v && mib < (kSplitBudgetBytes >> 20)) return (size_t)mib << 20;
+  }
+  return kSplitBudgetBytes;
+}
+
 // Cuts the jobs (row ranges of scenes) into segments of at most `budget`
 // bytes of volume, groups the segments into chunks of at most that size, and
-// chooses every chunk's block rows and offset groups.  False where the scene
-// is too wide for one tile row's volume.
+// chooses every chunk's block rows and offset groups.  Segments are runs of
+// whole rows where a row of the tallest tiles fits; else such rows are cut in
+// columns too.  False where one tile with its window does not fit.
 bool split_layout(const Plan& pl, const std::vector<SceneGeom>& geo, const std::vector<SplitJob>& jobs,
                   size_t budget, int sms, SplitLayout& out) {
   const FilterParams& F = pl.P;
@@ -809,6 +825,29 @@ bool split_layout(const Plan& pl, const std::vector<SceneGeom>& geo, const std::
     }
     out.passes[k].id[out.passes[k].n++] = i;
   }
+  auto pitch_of = [&](int cols) { return (cols + 2 * F.wsh + 3) / 4 * 4; };
+  // bytes of a segment's volume, and whether it may be one: the mean kernels'
+  // word offsets within a pass are 32-bit
+  auto volume = [&](int rows, int cols, size_t* pass) {
+    size_t bytes = 0;
+    for (int p = 0; p < F.npass; ++p) {
+      if (pass) pass[p] = bytes;
+      bytes += ((size_t)nhalf * (rows + F.wsh) * pitch_of(cols) * word_bytes(F.pass[p].np) + 255) / 256 * 256;
+    }
+    return bytes;
+  };
+  auto fits = [&](int rows, int cols) {
+    return volume(rows, cols, nullptr) <= budget && (size_t)nhalf * (rows + F.wsh) * pitch_of(cols) <= 0x3fffffff;
+  };
+  // the largest multiple of `unit` up to `most` that fits, 0 for none
+  auto largest = [&](int most, int unit, auto ok) {
+    int lo = 0, hi = most / unit;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) / 2;
+      if (ok(mid * unit)) lo = mid; else hi = mid - 1;
+    }
+    return lo * unit;
+  };
   size_t used = 0;
   auto close_chunk = [&] {
     if (!out.chunks.empty()) out.chunks.back().seg1 = (int)out.segs.size();
@@ -816,47 +855,40 @@ bool split_layout(const Plan& pl, const std::vector<SceneGeom>& geo, const std::
   };
   for (const SplitJob& j : jobs) {
     const SceneGeom& g = geo[j.scene];
-    const int row1 = std::min(j.row1, g.vH + 1);
+    const int row1 = std::min(j.row1, g.vH + 1), width = g.vW + 1;
     if (j.row0 >= row1) continue;
-    const int pitch = (g.vW + 1 + 2 * F.wsh + 3) / 4 * 4;
-    // bytes of one row of one half-window offset, all passes
-    size_t row = 0;
-    for (int p = 0; p < F.npass; ++p) row += (size_t)pitch * word_bytes(F.pass[p].np);
-    // the mean kernels' word offsets within a pass are 32-bit
-    const long long words = 0x3fffffffLL / ((long long)nhalf * pitch);
-    const long long fit = std::min((long long)(budget / (row * nhalf)), words) - F.wsh;
-    const int most = std::max(big, (int)std::min<long long>(fit, 1 << 20) / big * big);
     const int n = row1 - j.row0;
-    const int step = div_up(div_up(n, div_up(n, most)), big) * big;
-    for (int y = j.row0; y < row1; y += step) {
-      SplitSeg s{};
-      s.scene = j.scene;
-      s.vy0 = y;
-      s.vy1 = std::min(y + step, row1);
-      s.row0 = y - F.wsh;
-      s.rows = s.vy1 - s.row0;
-      s.pitch = pitch;
-      s.tiles_x = div_up(g.vW + 1, kTileW);
-      // a tile row's words do not fit
-      if ((size_t)nhalf * s.rows * pitch > 0x3fffffff) return false;
-      size_t bytes = 0;
-      for (int p = 0; p < F.npass; ++p) {
-        s.pass[p] = bytes;
-        bytes += ((size_t)nhalf * s.rows * pitch * word_bytes(F.pass[p].np) + 255) / 256 * 256;
-      }
-      // (a large window's volume of one tile row can exceed the budget: the
-      // kernel of nlsar_kernels.cu needs none)
-      if (!pl.fast && bytes > kSplitBudgetBytes) return false;
-      if (out.chunks.empty() || (used && used + bytes > budget)) {
-        close_chunk();
-        out.chunks.push_back(SplitChunk{});
-        out.chunks.back().seg0 = (int)out.segs.size();
-      }
-      s.vol = used;
-      used += bytes;
-      out.vol_bytes = std::max(out.vol_bytes, used);
-      out.segs.push_back(s);
+    int wide = width, rows = largest(div_up(n, big) * big, big, [&](int r) { return fits(std::min(r, n), width); });
+    if (rows == 0) {
+      rows = big;
+      wide = largest(div_up(width, kTileW) * kTileW, kTileW, [&](int c) { return fits(std::min(big, n), c); });
+      if (wide == 0) return false;
+      wide = div_up(div_up(width, div_up(width, wide)), kTileW) * kTileW;
     }
+    const int step = div_up(div_up(n, div_up(n, rows)), big) * big;
+    for (int y = j.row0; y < row1; y += step)
+      for (int x = 0; x < width; x += wide) {
+        SplitSeg s{};
+        s.scene = j.scene;
+        s.vy0 = y;
+        s.vy1 = std::min(y + step, row1);
+        s.vx0 = x;
+        s.vx1 = std::min(x + wide, width);
+        s.row0 = y - F.wsh;
+        s.rows = s.vy1 - s.row0;
+        s.pitch = pitch_of(s.vx1 - s.vx0);
+        s.tiles_x = div_up(s.vx1 - s.vx0, kTileW);
+        const size_t bytes = volume(s.vy1 - s.vy0, s.vx1 - s.vx0, s.pass);
+        if (out.chunks.empty() || (used && used + bytes > budget)) {
+          close_chunk();
+          out.chunks.push_back(SplitChunk{});
+          out.chunks.back().seg0 = (int)out.segs.size();
+        }
+        s.vol = used;
+        used += bytes;
+        out.vol_bytes = std::max(out.vol_bytes, used);
+        out.segs.push_back(s);
+      }
   }
   close_chunk();
   for (SplitChunk& c : out.chunks) {

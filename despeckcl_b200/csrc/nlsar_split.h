@@ -12,19 +12,23 @@
 
 namespace dcl {
 
-// Volume of weight indices held at a time.
+// Volume of weight indices held at a time, at most.
 constexpr size_t kSplitBudgetBytes = size_t(2) << 30;
-constexpr size_t kSplitMinBudgetBytes = size_t(32) << 20;  // below it the fused kernel filters
+constexpr size_t kSplitMinBudgetBytes = size_t(32) << 20;  // not tried smaller when memory is short
+// kSplitBudgetBytes, or what DESPECKCL_B200_VOLUME_MIB=n caps it to (0: no
+// call takes the two-kernel path).
+size_t split_budget();
 constexpr size_t kSplitSmem = 227 * 1024;
 constexpr int kSplitShapes = 2;  // different pass shapes of one call
 
-// A run of virtual rows of one scene with its volume: per pass words
+// A rectangle of virtual pixels of one scene with its volume: per pass words
 // [half-window offset][rows][pitch] of one byte per patch size (three: four).
 struct SplitSeg {
   int scene;
   int vy0, vy1;        // virtual rows filtered
+  int vx0, vx1;        // virtual columns filtered, vx0 on a tile column
   int row0, rows;      // virtual row of the volume's first row (vy0 - wsh), row count
-  int pitch;           // words per row; volume column c is virtual column c - wsh
+  int pitch;           // words per row; volume column c is virtual column vx0 + c - wsh
   int tiles_x, tile_begin;                // mean kernel: tiles per row, first tile in the chunk
   int idx_begin[kSplitShapes], idx_bx[kSplitShapes], idx_R[kSplitShapes];  // index kernel: blocks, columns, rows
   size_t vol, pass[kMaxPasses];  // first byte, and of each pass from there

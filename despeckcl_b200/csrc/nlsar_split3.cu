@@ -328,17 +328,27 @@ struct WordOffsets {
   size_t at[kMaxPasses];  // byte offset of each pass's words in the volume
 };
 
+// A segment: the virtual rows filtered and the first column, its rows of words
+// and words per row (the first is row vy0 - wsh, column vx0 - wsh), mean tiles
+// per row.
+struct Seg3 {
+  int vy0, vy1, vx0;
+  int rows, pitch, tiles_x;
+};
+
+// (the members of Seg3 one by one: with the struct as an argument the 12-row
+// variant spills 256 bytes a thread instead of 12)
 template <class L>
 __global__ void __launch_bounds__(L::THREADS, 1)
     mean3_kernel(const __grid_constant__ FilterParams P, const __grid_constant__ Scene3 S, int Hp,
-                 const char* __restrict__ vol, const __grid_constant__ WordOffsets wo, int vy0s, int vy1, int rows,
-                 int wpitch, int tiles_x) {
+                 const char* __restrict__ vol, const __grid_constant__ WordOffsets wo, int vy0s, int vy1, int vx0s,
+                 int rows, int wpitch, int tiles_x) {
   constexpr int WSH = L::WSH, RO = L::RO;
   extern __shared__ float4 smem4[];
   char* sm = reinterpret_cast<char*>(smem4);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ty = blockIdx.x / tiles_x, tx = blockIdx.x - ty * tiles_x;
-  const int vy0 = vy0s + ty * L::TH, vx0 = tx * 32;
+  const int vy0 = vy0s + ty * L::TH, vx0 = vx0s + tx * 32;
   float4* tile = reinterpret_cast<float4*>(sm + L::OFF_CO);
   float2* tile2 = reinterpret_cast<float2*>(tile + 4 * L::PLANE);
   for (int r = warp; r < L::ROH; r += L::WARPS) {
@@ -355,9 +365,10 @@ __global__ void __launch_bounds__(L::THREADS, 1)
     }
   }
   if (tid == 0) *reinterpret_cast<float*>(sm + L::OFF_ONE) = 1.0f;
-  // pixels past the last virtual row and column repeat it: their words exist
-  const uint32_t lane_off =
-      (uint32_t)(min(vy0 + warp, vy1 - 1) - vy0s + WSH) * wpitch + min(vx0 + lane, S.vW) + WSH;
+  // pixels past the segment's last row and the last virtual column repeat it:
+  // their words exist (columns are cut between tiles)
+  const uint32_t lane_off = (uint32_t)(min(vy0 + warp, vy1 - 1) - vy0s + WSH) * wpitch +
+                            (uint32_t)(min(vx0 + lane, S.vW) - vx0s) + WSH;
   Best3x best;
   best.e = -1.0f;
   best.a = 0.0f;
@@ -536,14 +547,14 @@ __device__ __forceinline__ void exact3_pass(const FilterParams& P, int ps, const
 template <int TH, int NPX>
 __global__ void __launch_bounds__(32 * TH, 1)
     exact3_mean_kernel(const __grid_constant__ FilterParams P, const __grid_constant__ Scene3 S, int Hp,
-                       const char* __restrict__ vol, const __grid_constant__ WordOffsets wo, int vy0s, int vy1,
-                       int rows, int wpitch, int tiles_x) {
+                       const char* __restrict__ vol, const __grid_constant__ WordOffsets wo,
+                       const __grid_constant__ Seg3 G) {
   extern __shared__ float4 smem4[];
   char* sm = reinterpret_cast<char*>(smem4);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wsh = P.wsh;
   const int RO = 32 + 2 * wsh, ROH = TH + 2 * wsh, PLANE = RO * ROH;
-  const int ty = blockIdx.x / tiles_x, tx = blockIdx.x - ty * tiles_x;
-  const int vy0 = vy0s + ty * TH, vx0 = tx * 32;
+  const int ty = blockIdx.x / G.tiles_x, tx = blockIdx.x - ty * G.tiles_x;
+  const int vy0 = G.vy0 + ty * TH, vx0 = G.vx0 + tx * 32;
   float4* tile = reinterpret_cast<float4*>(sm + exact3_tables(NPX));
   float2* tile2 = reinterpret_cast<float2*>(tile + 4 * PLANE);
   for (int r = warp; r < ROH; r += TH) {
@@ -558,9 +569,10 @@ __global__ void __launch_bounds__(32 * TH, 1)
       tile2[i] = make_float2(g[16 * S.plane], g[17 * S.plane]);
     }
   }
-  // pixels past the last virtual row and column repeat it: their words exist
-  const uint32_t lane_off =
-      (uint32_t)(min(vy0 + warp, vy1 - 1) - vy0s + wsh) * wpitch + min(vx0 + lane, S.vW) + wsh;
+  // pixels past the segment's last row and the last virtual column repeat it:
+  // their words exist (columns are cut between tiles)
+  const uint32_t lane_off = (uint32_t)(min(vy0 + warp, G.vy1 - 1) - G.vy0 + wsh) * G.pitch +
+                            (uint32_t)(min(vx0 + lane, S.vW) - G.vx0) + wsh;
   Best3x best;
   best.e = -1.0f;
   best.a = 0.0f;
@@ -572,17 +584,17 @@ __global__ void __launch_bounds__(32 * TH, 1)
   for (int ps = 0; ps < P.npass; ++ps) {
     const char* w = vol + wo.at[ps];
     if constexpr (NPX == 1) {
-      exact3_pass<TH, NPX, 1>(P, ps, w, rows, wpitch, lane_off, RO, PLANE, best);
+      exact3_pass<TH, NPX, 1>(P, ps, w, G.rows, G.pitch, lane_off, RO, PLANE, best);
     } else if (P.pass[ps].np == 2) {
-      exact3_pass<TH, NPX, 2>(P, ps, w, rows, wpitch, lane_off, RO, PLANE, best);
+      exact3_pass<TH, NPX, 2>(P, ps, w, G.rows, G.pitch, lane_off, RO, PLANE, best);
     } else {
-      exact3_pass<TH, NPX, 3>(P, ps, w, rows, wpitch, lane_off, RO, PLANE, best);
+      exact3_pass<TH, NPX, 3>(P, ps, w, G.rows, G.pitch, lane_off, RO, PLANE, best);
     }
   }
   const int vy = vy0 + warp, vx = vx0 + lane;
   const int oy = (vy < S.H - 1) ? vy : (vy == S.vH ? S.H - 1 : -1);
   const int ox = (vx < S.W - 1) ? vx : (vx == S.vW ? S.W - 1 : -1);
-  if (oy < 0 || ox < 0 || vy >= vy1) return;
+  if (oy < 0 || ox < 0 || vy >= G.vy1) return;
   const size_t n = (size_t)S.H * S.W, o = (size_t)oy * S.W + ox;
   const int ci = (warp + wsh) * RO + lane + wsh;
   const float oma = 1.0f - best.a;
@@ -601,45 +613,45 @@ constexpr int kTall3 = 12;  // rows of the tallest mean tile (segments hold whol
 size_t word_bytes(int np) { return np == 3 ? 4 : np; }
 int div_up(int a, int b) { return (a + b - 1) / b; }
 
+int mean_tiles(const Seg3& G, int th) { return G.tiles_x * div_up(G.vy1 - G.vy0, th); }
+
 template <int TH, int NPX>
 cudaError_t launch_mean3_t(const FilterParams& F, const Scene3& S, int Hp, const char* vol, const WordOffsets& wo,
-                           int vy0, int vy1, int rows, int wpitch, int tiles_x, cudaStream_t st) {
+                           const Seg3& G, cudaStream_t st) {
   using L = Mean3L<10, TH, NPX>;
   static size_t allowed[kMaxDevices];
   const cudaError_t e = allow_dynamic_smem((const void*)mean3_kernel<L>, L::BYTES, allowed);
   if (e != cudaSuccess) return e;
-  mean3_kernel<L><<<tiles_x * div_up(vy1 - vy0, TH), L::THREADS, L::BYTES, st>>>(F, S, Hp, vol, wo, vy0, vy1, rows,
-                                                                             wpitch, tiles_x);
+  mean3_kernel<L><<<mean_tiles(G, TH), L::THREADS, L::BYTES, st>>>(F, S, Hp, vol, wo, G.vy0, G.vy1, G.vx0, G.rows,
+                                                                   G.pitch, G.tiles_x);
   return cudaGetLastError();
 }
 
 template <int NPX>
 cudaError_t launch_mean3(int th, const FilterParams& F, const Scene3& S, int Hp, const char* vol,
-                         const WordOffsets& wo, int vy0, int vy1, int rows, int wpitch, int tiles_x, cudaStream_t st) {
+                         const WordOffsets& wo, const Seg3& G, cudaStream_t st) {
   switch (th) {
-    case 4: return launch_mean3_t<4, NPX>(F, S, Hp, vol, wo, vy0, vy1, rows, wpitch, tiles_x, st);
-    case 8: return launch_mean3_t<8, NPX>(F, S, Hp, vol, wo, vy0, vy1, rows, wpitch, tiles_x, st);
-    default: return launch_mean3_t<kTall3, NPX>(F, S, Hp, vol, wo, vy0, vy1, rows, wpitch, tiles_x, st);
+    case 4: return launch_mean3_t<4, NPX>(F, S, Hp, vol, wo, G, st);
+    case 8: return launch_mean3_t<8, NPX>(F, S, Hp, vol, wo, G, st);
+    default: return launch_mean3_t<kTall3, NPX>(F, S, Hp, vol, wo, G, st);
   }
 }
 
 template <int TH, int NPX>
 cudaError_t launch_exact3_t(const FilterParams& F, const Scene3& S, int Hp, const char* vol, const WordOffsets& wo,
-                            int vy0, int vy1, int rows, int wpitch, int tiles_x, cudaStream_t st) {
+                            const Seg3& G, cudaStream_t st) {
   static size_t allowed[kMaxDevices];
   const cudaError_t e = allow_dynamic_smem((const void*)exact3_mean_kernel<TH, NPX>, kSplitSmem, allowed);
   if (e != cudaSuccess) return e;
-  exact3_mean_kernel<TH, NPX><<<tiles_x * div_up(vy1 - vy0, TH), 32 * TH, exact3_smem(F.wsh, TH, NPX), st>>>(
-      F, S, Hp, vol, wo, vy0, vy1, rows, wpitch, tiles_x);
+  exact3_mean_kernel<TH, NPX><<<mean_tiles(G, TH), 32 * TH, exact3_smem(F.wsh, TH, NPX), st>>>(F, S, Hp, vol, wo, G);
   return cudaGetLastError();
 }
 
 template <int NPX>
 cudaError_t launch_exact3(int th, const FilterParams& F, const Scene3& S, int Hp, const char* vol,
-                          const WordOffsets& wo, int vy0, int vy1, int rows, int wpitch, int tiles_x,
-                          cudaStream_t st) {
-  return th == 4 ? launch_exact3_t<4, NPX>(F, S, Hp, vol, wo, vy0, vy1, rows, wpitch, tiles_x, st)
-                 : launch_exact3_t<8, NPX>(F, S, Hp, vol, wo, vy0, vy1, rows, wpitch, tiles_x, st);
+                          const WordOffsets& wo, const Seg3& G, cudaStream_t st) {
+  return th == 4 ? launch_exact3_t<4, NPX>(F, S, Hp, vol, wo, G, st)
+                 : launch_exact3_t<8, NPX>(F, S, Hp, vol, wo, G, st);
 }
 
 template <int PH0, int PH1, int PH2, bool EXACT>
@@ -680,11 +692,9 @@ Split3 split3_layout(const Plan& pl, const Scene3& S, size_t budget) {
   // 64 x 70 with search 3 takes 73 us (nlsar3_kernel 61), with search 5 75 us
   // (112), 280 x 290 with search 3 98 us (124)
   if (L.exact && F.wsh == 1 && (long long)S.H * S.W < 65536) return L;
-  size_t word_row = 0;
   int np_min = kPatchPerPass, npx = 1;
   for (int i = 0; i < F.npass; ++i) {
     if (pass_shape3(F.pass[i]) < 0) return L;
-    word_row += word_bytes(F.pass[i].np);
     np_min = std::min(np_min, F.pass[i].np);
     npx = std::max(npx, F.pass[i].np);
   }
@@ -692,32 +702,50 @@ Split3 split3_layout(const Plan& pl, const Scene3& S, size_t budget) {
   if (npx > 1 && np_min == 1) return L;
   npx = npx > 1 ? 3 : 1;
   if (L.exact && (exact3_smem(F.wsh, 4, npx) > kSplitSmem || sim3_smem(F.wsh) > kSplitSmem)) return L;
-  L.pitch = (S.vW + 1 + 2 * F.wsh + 15) / 16 * 16;
-  L.spitch = L.pitch + 2 * kSimLeft;
-  const size_t srow = (size_t)nhalf * L.spitch * sizeof(float), wrow = (size_t)nhalf * L.pitch * word_row;
-  const int extra_s = F.wsh + 2 * F.phm, extra_w = F.wsh;
-  const long long fit = ((long long)budget - (long long)(srow * extra_s + wrow * extra_w)) / (long long)(srow + wrow);
-  const int most = std::max(2 * kTall3, (int)std::min<long long>(fit, 1 << 20) / (2 * kTall3) * (2 * kTall3));
-  const int total = S.vH + 1, step = div_up(total, div_up(total, most));
-  L.rows = div_up(step, 2 * kTall3) * (2 * kTall3);
-  // 32-bit word offsets within a pass
-  if ((size_t)nhalf * (L.rows + extra_w) * L.pitch > 0x3fffffff) {
-    L.rows = 0;
-    return L;
+  // a segment's rows of similarities and of words, and its volume; 32-bit word
+  // offsets within a pass
+  const int extra_s = F.wsh + 2 * F.phm, extra_w = F.wsh, width = S.vW + 1, total = S.vH + 1;
+  auto pitch_of = [&](int cols) { return (cols + 2 * F.wsh + 15) / 16 * 16; };
+  auto sims = [&](int rows, int cols) {
+    return ((size_t)nhalf * (rows + extra_s) * (pitch_of(cols) + 2 * kSimLeft) * sizeof(float) + 255) / 256 * 256;
+  };
+  auto volume = [&](int rows, int cols) {
+    size_t bytes = sims(rows, cols);
+    for (int i = 0; i < F.npass; ++i)
+      bytes += ((size_t)nhalf * (rows + extra_w) * pitch_of(cols) * word_bytes(F.pass[i].np) + 255) / 256 * 256;
+    return bytes;
+  };
+  auto fits = [&](int rows, int cols) {
+    return volume(rows, cols) <= budget && (size_t)nhalf * (rows + extra_w) * pitch_of(cols) <= 0x3fffffff;
+  };
+  // the largest multiple of `unit` up to `most` that fits, 0 for none
+  auto largest = [&](int most, int unit, auto ok) {
+    int lo = 0, hi = most / unit;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) / 2;
+      if (ok(mid * unit)) lo = mid; else hi = mid - 1;
+    }
+    return lo * unit;
+  };
+  constexpr int unit = 2 * kTall3;  // whole tiles of 12 and 8 rows
+  int cols = width, rows = largest(div_up(total, unit) * unit, unit, [&](int r) { return fits(r, width); });
+  if (rows == 0) {
+    rows = unit;
+    cols = largest(div_up(width, 32) * 32, 32, [&](int c) { return fits(unit, c); });
+    if (cols == 0) return L;
+    cols = div_up(div_up(width, div_up(width, cols)), 32) * 32;
   }
-  L.sim_bytes = (srow * (L.rows + extra_s) + 255) / 256 * 256;
-  size_t words = 0;
-  for (int i = 0; i < F.npass; ++i)
-    words += ((size_t)nhalf * (L.rows + extra_w) * L.pitch * word_bytes(F.pass[i].np) + 255) / 256 * 256;
-  L.vol_bytes = L.sim_bytes + words;
-  // a large window's volume of one segment can exceed the budget: nlsar3_kernel
-  // needs none
-  if (L.exact && L.vol_bytes > kSplitBudgetBytes) L.rows = 0;
+  L.rows = div_up(div_up(total, div_up(total, rows)), unit) * unit;
+  L.cols = cols;
+  L.pitch = pitch_of(cols);
+  L.spitch = L.pitch + 2 * kSimLeft;
+  L.sim_bytes = sims(L.rows, cols);
+  L.vol_bytes = volume(L.rows, cols);
   return L;
 }
 
 cudaError_t launch_split3(const Plan& pl, const FilterParams& F, const Scene3& S, int Hp, int Wp, const Split3& L,
-                          char* vol, int vy0, int vy1, int sms, cudaStream_t st) {
+                          char* vol, int vy0, int vy1, int vx0, int vx1, int sms, cudaStream_t st) {
   const int nhalf = F.n_off / 2;
   const int rows = vy1 - vy0 + F.wsh, srows = rows + 2 * F.phm;
   float* sims = reinterpret_cast<float*>(vol);
@@ -739,13 +767,13 @@ cudaError_t launch_split3(const Plan& pl, const FilterParams& F, const Scene3& S
     if (pp.scale_slot != slot) {
       slot = pp.scale_slot;
       // similarity row 0 is virtual row vy0 - wsh - phm, column 0 virtual
-      // column -wsh - kSimLeft; offset groups fill four blocks per SM
+      // column vx0 - wsh - kSimLeft; offset groups fill four blocks per SM
       dim3 grid(div_up(L.spitch, 32), div_up(srows, kSimTH));
       grid.z = std::max(1, std::min(nhalf, div_up(4 * sms, (int)(grid.x * grid.y))));
       const auto sim = L.exact ? sim3_kernel<true> : sim3_kernel<false>;
       sim<<<grid, kSimThreads, sim3_smem(F.wsh), st>>>(S.s9[slot], S.ld[slot], Hp, Wp, S.pitch, S.plane,
                                                              F.wsh, F.c2d, vy0 - F.wsh - F.phm + F.G,
-                                                             F.G - F.wsh - kSimLeft, sims, srows, L.spitch);
+                                                             vx0 + F.G - F.wsh - kSimLeft, sims, srows, L.spitch);
       profile_count(1);
     }
     char* words = vol + wo.at[ps];
@@ -770,11 +798,11 @@ cudaError_t launch_split3(const Plan& pl, const FilterParams& F, const Scene3& S
     if (e != cudaSuccess) return e;
   }
   // rows of the mean tiles: waves of blocks times a block's time
-  const int tiles_x = div_up(S.vW + 1, 32);
+  const Seg3 G{vy0, vy1, vx0, rows, L.pitch, div_up(vx1 - vx0, 32)};
   int th = kTall3;
   double best = 0.0;
   for (int t : {kTall3, 8, 4}) {
-    const double cost = (double)div_up(tiles_x * div_up(vy1 - vy0, t), sms) * (t == kTall3 ? 1.0 : (t == 8 ? 0.72 : 0.45));
+    const double cost = (double)div_up(mean_tiles(G, t), sms) * (t == kTall3 ? 1.0 : (t == 8 ? 0.72 : 0.45));
     if (best == 0.0 || cost < 0.98 * best) {
       best = cost;
       th = t;
@@ -783,11 +811,11 @@ cudaError_t launch_split3(const Plan& pl, const FilterParams& F, const Scene3& S
   profile_count(1);
   if (L.exact) {
     const int t = th == 4 || exact3_smem(F.wsh, 8, npx == 1 ? 1 : 3) > kSplitSmem ? 4 : 8;
-    return npx == 1 ? launch_exact3<1>(t, F, S, Hp, vol, wo, vy0, vy1, rows, L.pitch, tiles_x, st)
-                    : launch_exact3<3>(t, F, S, Hp, vol, wo, vy0, vy1, rows, L.pitch, tiles_x, st);
+    return npx == 1 ? launch_exact3<1>(t, F, S, Hp, vol, wo, G, st)
+                    : launch_exact3<3>(t, F, S, Hp, vol, wo, G, st);
   }
-  return npx == 1 ? launch_mean3<1>(th, F, S, Hp, vol, wo, vy0, vy1, rows, L.pitch, tiles_x, st)
-                  : launch_mean3<3>(th, F, S, Hp, vol, wo, vy0, vy1, rows, L.pitch, tiles_x, st);
+  return npx == 1 ? launch_mean3<1>(th, F, S, Hp, vol, wo, G, st)
+                  : launch_mean3<3>(th, F, S, Hp, vol, wo, G, st);
 }
 
 }  // namespace dcl

@@ -36,21 +36,23 @@ struct Scene3 {
   size_t plane;                 // Hp * pitch
 };
 
-// The two-kernel path of a 3x3 call: segments of rows whose similarity and
-// word volumes fit a budget.
+// The two-kernel path of a 3x3 call: segments whose similarity and word
+// volumes fit a budget.
 struct Split3 {
-  int rows = 0;                     // virtual rows per segment; 0: the call is not served
+  int rows = 0, cols = 0;           // virtual rows and columns per segment; rows 0: the call is not served
   int pitch = 0, spitch = 0;        // words, similarities per volume row
   bool exact = false;               // the settings and arithmetic of nlsar3_kernel
   size_t sim_bytes = 0, vol_bytes = 0;  // similarities of one scale, then the words of every pass
 };
 // Whether nlsar3_fast_kernel has a call's shapes (nlsar_dim3.cu).
 bool fast3_supported(const FilterParams& F);
-// Sizes the segments for `budget` bytes; rows 0 where the plan has no kernels
-// or a row is too wide.
+// Sizes the segments for `budget` bytes: runs of whole rows where two rows of
+// the tallest tiles fit, else cut in columns too; rows 0 where the plan has no
+// kernels or one tile column of that does not fit.
 Split3 split3_layout(const Plan& pl, const Scene3& S, size_t budget);
-// Filters virtual rows [vy0, vy1) (at most L.rows) with the volumes at `vol`.
+// Filters virtual rows [vy0, vy1) (at most L.rows) and columns [vx0, vx1) (at
+// most L.cols, vx0 a multiple of it) with the volumes at `vol`.
 cudaError_t launch_split3(const Plan& pl, const FilterParams& F, const Scene3& S, int Hp, int Wp, const Split3& L,
-                          char* vol, int vy0, int vy1, int sms, cudaStream_t st);
+                          char* vol, int vy0, int vy1, int vx0, int vx1, int sms, cudaStream_t st);
 
 }  // namespace dcl
