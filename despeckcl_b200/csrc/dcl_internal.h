@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <utility>
+
 namespace dcl {
 
 // Record a message for dcl_last_error() and return `code`.
@@ -20,6 +22,22 @@ constexpr int kMaxDevices = 64;
 cudaError_t allow_dynamic_smem(const void* func, size_t bytes, size_t* cache);
 // SMs of a device (148 where the query fails).
 int sm_count(int dev);
+#ifdef __CUDACC__
+// Launches a kernel and returns this launch's own status.  (The thread's last
+// error would serve only until the next cudaFuncSetAttribute, which clears it,
+// and can be older than the launch.)
+template <class... P, class... A>
+cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  const cudaError_t e = cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // reported by the caller
+  return e;
+}
+#endif
 // Count `n` kernel launches of the calling thread while dcl_profile_begin is active.
 void profile_count(int n);
 

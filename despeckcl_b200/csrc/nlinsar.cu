@@ -548,9 +548,8 @@ cudaError_t launch_weights_t(const float* a1, const float* a2, const float* dp, 
   const size_t smem = weights_smem(g, SIM);
   const cudaError_t e = allow_dynamic_smem((const void*)nlinsar_weights_kernel<Z, SIM>, smem, allowed);
   if (e != cudaSuccess) return e;
-  nlinsar_weights_kernel<Z, SIM><<<dim3(tiles, groups), weights_threads(SIM), smem, st>>>(a1, a2, dp, est[0], est[1], est[2], g,
-                                                                            tile0, nonzero, sums, wts);
-  return cudaGetLastError();
+  return launch_kernel(nlinsar_weights_kernel<Z, SIM>, dim3(tiles, groups), weights_threads(SIM), smem, st, a1, a2, dp,
+                       est[0], est[1], est[2], g, tile0, nonzero, sums, wts);
 }
 
 template <bool SIM>
@@ -621,21 +620,23 @@ int nlinsar_device(const float* a1, const float* a2, const float* dp, float* ref
   e = cudaMemsetAsync(nonzero, 0, sizeof(int), st);
   if (e == cudaSuccess) {
     const int sms = sm_count(dev);
-    nlinsar_filter_values_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a1, a2, dp, fa, fr, fi, n);
+    e = launch_kernel(nlinsar_filter_values_kernel, (unsigned)((n + 255) / 256), 256, 0, st, a1, a2, dp, fa, fr, fi, n);
     profile_count(1);
     // estimates ping-pong between the caller's planes and tr/tp/tc; an odd
     // number of passes ends in tr/tp/tc and is copied back
     float* cur[3] = {ref, phase, coh};
     float* nxt[3] = {tr, tp, tc};
     for (int it = 0; it < niter && e == cudaSuccess; ++it) {
-      nlinsar_nonzero_kernel<<<(unsigned)std::min<size_t>((n + 1023) / 1024, 8 * sms), 256, 0, st>>>(cur[0], n, nonzero);
+      e = launch_kernel(nlinsar_nonzero_kernel, (unsigned)std::min<size_t>((n + 1023) / 1024, 8 * sms), 256, 0, st,
+                        cur[0], n, nonzero);
       for (int t0 = 0; t0 < ntiles && e == cudaSuccess; t0 += chunk) {
         const int nt = std::min(chunk, ntiles - t0);
         e = keep && it > 0 ? launch_weights<false>(a1, a2, dp, cur, g, t0, nt, nonzero, sums, wts, sms, st)
                            : launch_weights<true>(a1, a2, dp, cur, g, t0, nt, nonzero, sums, wts, sms, st);
-        dim3 grid((unsigned)((npix + kEstThreads - 1) / kEstThreads), nt);
-        nlinsar_estimate_kernel<<<grid, kEstThreads, 0, st>>>(a1, fa, fr, fi, cur[0], cur[1], cur[2], nxt[0], nxt[1],
-                                                              nxt[2], g, t0, wts);
+        const dim3 grid((unsigned)((npix + kEstThreads - 1) / kEstThreads), nt);
+        if (e == cudaSuccess)
+          e = launch_kernel(nlinsar_estimate_kernel, grid, kEstThreads, 0, st, a1, fa, fr, fi, cur[0], cur[1], cur[2],
+                            nxt[0], nxt[1], nxt[2], g, t0, wts);
         profile_count(2);
       }
       profile_count(1);
@@ -646,7 +647,6 @@ int nlinsar_device(const float* a1, const float* a2, const float* dp, float* ref
         e = cudaMemcpyAsync(d == 0 ? ref : (d == 1 ? phase : coh), cur[d], n * sizeof(float),
                             cudaMemcpyDeviceToDevice, st);
   }
-  if (e == cudaSuccess) e = cudaGetLastError();
   cudaFreeAsync(buf, st);
   if (e != cudaSuccess) return cuda_error(e, "NL-InSAR");
   return DCL_OK;

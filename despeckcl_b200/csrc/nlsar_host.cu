@@ -439,15 +439,16 @@ int launch_prep_rows(const Plan& pl, const SceneGeom& g, const SceneDesc& d, con
                      const float* phi, const float* cov_in, int co0, int co1, int cs0, int cs1, cudaStream_t st) {
   const dim3 blk(32, 8);
   const unsigned gx = (unsigned)(g.Wp + 31) / 32;
+  cudaError_t e = cudaSuccess;
   if (co1 > co0) {
     profile_count(1);
     const dim3 grd(gx, (unsigned)(co1 - co0 + 7) / 8);
-    if (pl.full8)
-      prep_cov_planes_kernel<<<grd, blk, 0, st>>>(cov_in, g.H, g.W, const_cast<float4*>(d.cori),
-                                                  const_cast<float4*>(d.cori2), g.Hp, g.Wp, g.pitch, pl.P.G, co0, co1);
-    else
-      prep_cov_insar_kernel<<<grd, blk, 0, st>>>(a1, a2, phi, g.H, g.W, const_cast<float4*>(d.cori), g.Hp, g.Wp,
-                                                 g.pitch, pl.P.G, co0, co1);
+    e = pl.full8 ? launch_kernel(prep_cov_planes_kernel, grd, blk, 0, st, cov_in, g.H, g.W,
+                                 const_cast<float4*>(d.cori), const_cast<float4*>(d.cori2), g.Hp, g.Wp, g.pitch,
+                                 pl.P.G, co0, co1)
+                 : launch_kernel(prep_cov_insar_kernel, grd, blk, 0, st, a1, a2, phi, g.H, g.W,
+                                 const_cast<float4*>(d.cori), g.Hp, g.Wp, g.pitch, pl.P.G, co0, co1);
+    if (e != cudaSuccess) return cuda_error(e, "NL-SAR prep");
   }
   if (cs1 <= cs0) return DCL_OK;
   const float gamma = rescale_gamma_2x2();
@@ -459,8 +460,9 @@ int launch_prep_rows(const Plan& pl, const SceneGeom& g, const SceneDesc& d, con
     const std::vector<float> gw = gauss_weights(pl.scales[si]);
     std::copy(gw.begin(), gw.end(), ga.g);
     profile_count(1);
-    prep_scale_kernel<<<grd, blk, 0, st>>>(d.cori, g.Hp, g.Wp, g.pitch, pl.scales[si], ga, gamma,
-                                           const_cast<float4*>(d.cs[si]), const_cast<float*>(d.ld[si]), cs0, cs1);
+    e = launch_kernel(prep_scale_kernel, grd, blk, 0, st, d.cori, g.Hp, g.Wp, g.pitch, pl.scales[si], ga, gamma,
+                      const_cast<float4*>(d.cs[si]), const_cast<float*>(d.ld[si]), cs0, cs1);
+    if (e != cudaSuccess) return cuda_error(e, "NL-SAR prep");
   }
   return DCL_OK;
 }
@@ -599,7 +601,11 @@ int run_device(const Plan& pl0, const std::vector<SceneIO>& io, cudaStream_t st)
     desc[i].sel_out = io[i].sel;
     desc[i].tile_begin = tb;
     tb += geo[i].tiles_x * geo[i].tiles_y;
-    launch_prep(pl, geo[i], desc[i], io[i].a1, io[i].a2, io[i].phi, io[i].cov_in, st);
+    rc = launch_prep(pl, geo[i], desc[i], io[i].a1, io[i].a2, io[i].phi, io[i].cov_in, st);
+    if (rc) {
+      cudaFreeAsync(scratch, st);
+      return rc;
+    }
   }
   e = cudaMemcpyAsync(d_desc, up.data(), up.size(), cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) {
@@ -830,10 +836,11 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
       rc = cuda_error(e, "cudaMemcpyAsync(H2D)");
       break;
     }
-    if (pl.full8)
-      launch_prep_rows(pl, g, desc[i], nullptr, nullptr, nullptr, buf, co_done, co_need, cs_done, cs_need, st);
-    else
-      launch_prep_rows(pl, g, desc[i], buf, buf + n, buf + 2 * n, nullptr, co_done, co_need, cs_done, cs_need, st);
+    rc = pl.full8
+             ? launch_prep_rows(pl, g, desc[i], nullptr, nullptr, nullptr, buf, co_done, co_need, cs_done, cs_need, st)
+             : launch_prep_rows(pl, g, desc[i], buf, buf + n, buf + 2 * n, nullptr, co_done, co_need, cs_done, cs_need,
+                                st);
+    if (rc) break;
     co_done = co_need;
     cs_done = cs_need;
     FilterParams F = pl.P;

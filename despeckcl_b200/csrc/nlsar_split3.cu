@@ -770,11 +770,11 @@ cudaError_t launch_split3(const Plan& pl, const FilterParams& F, const Scene3& S
       // column vx0 - wsh - kSimLeft; offset groups fill four blocks per SM
       dim3 grid(div_up(L.spitch, 32), div_up(srows, kSimTH));
       grid.z = std::max(1, std::min(nhalf, div_up(4 * sms, (int)(grid.x * grid.y))));
-      const auto sim = L.exact ? sim3_kernel<true> : sim3_kernel<false>;
-      sim<<<grid, kSimThreads, sim3_smem(F.wsh), st>>>(S.s9[slot], S.ld[slot], Hp, Wp, S.pitch, S.plane,
-                                                             F.wsh, F.c2d, vy0 - F.wsh - F.phm + F.G,
-                                                             vx0 + F.G - F.wsh - kSimLeft, sims, srows, L.spitch);
+      e = launch_kernel(L.exact ? sim3_kernel<true> : sim3_kernel<false>, grid, kSimThreads, sim3_smem(F.wsh), st,
+                        S.s9[slot], S.ld[slot], Hp, Wp, S.pitch, S.plane, F.wsh, F.c2d, vy0 - F.wsh - F.phm + F.G,
+                        vx0 + F.G - F.wsh - kSimLeft, sims, srows, L.spitch);
       profile_count(1);
+      if (e != cudaSuccess) return e;
     }
     char* words = vol + wo.at[ps];
     auto codes = [&](auto launch) {
