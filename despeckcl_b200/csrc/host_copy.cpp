@@ -6,27 +6,87 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
+#include <exception>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
 namespace dcl {
 
-bool PinnedSlots::ready() {
-  if (tried) return ok;
-  tried = true;
-  cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&mem), kSlots * kSlotBytes, cudaHostAllocPortable);
-  for (int i = 0; i < kSlots && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
-  if (e != cudaSuccess) cudaGetLastError();
-  ok = e == cudaSuccess;
-  return ok;
+namespace {
+
+// Blocks of the process.  Never destroyed: threads may end after it would be.
+struct BlockPool {
+  std::mutex mu;
+  std::vector<char*> idle;
+  int made = 0;              // pinned, idle or in use
+  int takes = 0, peak = 0;   // calls of this window, most blocks in use at once in it
+
+  static BlockPool& get() {
+    static BlockPool* p = new BlockPool;
+    return *p;
+  }
+};
+
+}  // namespace
+
+bool PinnedBlock::take() {
+  if (mem_) return true;
+  BlockPool& p = BlockPool::get();
+  std::vector<char*> drop;
+  bool make = false;
+  {
+    std::lock_guard<std::mutex> lk(p.mu);
+    p.idle.reserve(kMaxBlocks);  // giving back does not allocate
+    if (!p.idle.empty()) {
+      mem_ = p.idle.back();
+      p.idle.pop_back();
+    } else if (p.made < kMaxBlocks) {
+      make = true;
+      ++p.made;
+    }
+    sharers_ = p.made - (int)p.idle.size();
+    p.peak = std::max(p.peak, sharers_);
+    if (++p.takes >= kWindow) {
+      while (!p.idle.empty() && p.made > p.peak) {
+        drop.push_back(p.idle.back());
+        p.idle.pop_back();
+        --p.made;
+      }
+      p.takes = 0;
+      p.peak = sharers_;
+    }
+  }
+  for (char* m : drop) cudaFreeHost(m);
+  if (!make) return mem_ != nullptr;
+  if (cudaHostAlloc(reinterpret_cast<void**>(&mem_), kBytes, cudaHostAllocPortable) == cudaSuccess) return true;
+  cudaGetLastError();
+  mem_ = nullptr;
+  std::lock_guard<std::mutex> lk(p.mu);
+  --p.made;
+  return false;
 }
 
-PinnedSlots::~PinnedSlots() {
+PinnedBlock::~PinnedBlock() {
+  if (!mem_) return;
+  BlockPool& p = BlockPool::get();
+  std::lock_guard<std::mutex> lk(p.mu);
+  p.idle.push_back(mem_);
+}
+
+bool SlotEvents::ready() {
+  for (cudaEvent_t& e : ev)
+    if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      e = nullptr;
+      return false;
+    }
+  return true;
+}
+
+SlotEvents::~SlotEvents() {
   for (cudaEvent_t e : ev)
     if (e) cudaEventDestroy(e);
-  if (mem) cudaFreeHost(mem);
 }
 
 namespace {
@@ -71,10 +131,11 @@ struct CopyCrew::Impl {
 };
 
 CopyCrew::CopyCrew(int threads) : impl_(new Impl()) {
+  impl_->threads.reserve(threads);
   for (int i = 0; i < threads; ++i) {
     try {
       impl_->threads.emplace_back([this] { impl_->loop(); });
-    } catch (const std::system_error&) {
+    } catch (const std::exception&) {
       break;  // the caller copies with those there are
     }
   }

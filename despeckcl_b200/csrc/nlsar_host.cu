@@ -651,9 +651,10 @@ constexpr int kMaxBands = 8;  // row bands of a host-pointer call
 // Fewest waves of tiles (one CTA per SM) per band: each band's launch ends in
 // a partly filled wave, so small scenes stay in one band.  Pageable planes of
 // kStageBytes in all or more go through pinned slots, which leaves more time
-// to hide behind smaller bands.
+// to hide behind smaller bands (with the reference's selection 700 x 700, 11 MiB,
+// takes 4.4 ms either way, 1000 x 1000, 23 MiB, 3.95 ms without and 3.35 with).
 constexpr int kStagedWaves = 4;
-constexpr size_t kStageBytes = size_t(8) << 20;
+constexpr size_t kStageBytes = size_t(16) << 20;
 
 int band_count(int dev, long long tiles, int tile_rows, int waves) {
   const int sms = sm_count(dev);
@@ -707,13 +708,16 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
   HostPipe* hp = nullptr;
   rc = host_pipe(dev, 2 * (size_t)kMaxBands + 2, hp);
   if (rc) return rc;
-  staged = staged && hp->in.ready() && hp->out.ready();
+  PinnedBlock pinned;  // given back at return, when the copy streams have been waited for
+  staged = staged && hp->up.ready() && hp->down.ready() && pinned.take();
   const int nb = band_count(dev, (long long)g.tiles_x * g.tiles_y, g.tiles_y, staged ? kStagedWaves : 8);
   rc = host_pipe(dev, 2 * (size_t)nb + 2, hp);
   if (rc) return rc;
   // 3 to 7 helpers measured alike, more slower (1531 x 1999: 5.6 - 6.2 ms,
-  // with 15 7.3 - 7.7; 10.3 ms through the driver's staging)
-  CopyCrew crew(staged ? std::max(1, std::min(4, (int)std::thread::hardware_concurrency() - 1)) : 0);
+  // with 15 7.3 - 7.7; 10.3 ms through the driver's staging); calls at the same
+  // time share the cores
+  const int cores = (int)std::thread::hardware_concurrency();
+  CopyCrew crew(staged ? std::max(1, std::min(4, (cores - 1) / pinned.sharers())) : 0);
   cudaEvent_t* ev_in = hp->ev.data();       // band inputs uploaded
   cudaEvent_t* ev_out = hp->ev.data() + nb;  // band results written
   cudaEvent_t ev_alloc = hp->ev[2 * nb], ev_done = hp->ev[2 * nb + 1];
@@ -801,7 +805,8 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
   pl.P.timeouts = d_timeouts;
 
   const int TH = pl.P.tile_h, G = pl.P.G;
-  int in_done = 0, co_done = 0, cs_done = 0, slot = 0;
+  int in_done = 0, co_done = 0, cs_done = 0;
+  size_t slot = 0;
   for (int i = 0; i < nb && rc == DCL_OK; ++i) {
     const bool last = i == nb - 1;
     // frame rows the band's tiles read (scaled covariance: tile + patch and
@@ -817,15 +822,14 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
           e = cudaMemcpyAsync(buf + p * n + off, hin[p] + off, cnt, cudaMemcpyHostToDevice, hp->h2d);
           continue;
         }
-        for (size_t at = 0; at < cnt && e == cudaSuccess; at += PinnedSlots::kSlotBytes, ++slot) {
-          const size_t len = std::min(PinnedSlots::kSlotBytes, cnt - at);
-          cudaEvent_t free_ev = hp->in.ev[slot % PinnedSlots::kSlots];
-          if (slot >= PinnedSlots::kSlots) e = cudaEventSynchronize(free_ev);
+        for (size_t at = 0; at < cnt && e == cudaSuccess; at += kSlotBytes, ++slot) {
+          const size_t len = std::min(kSlotBytes, cnt - at);
+          if (slot >= kSlots) e = cudaEventSynchronize(hp->up.at(slot));
           if (e != cudaSuccess) break;
-          crew.copy(hp->in.slot(slot), reinterpret_cast<const char*>(hin[p] + off) + at, len);
-          e = cudaMemcpyAsync(reinterpret_cast<char*>(buf + p * n + off) + at, hp->in.slot(slot), len,
+          crew.copy(pinned.slot(slot), reinterpret_cast<const char*>(hin[p] + off) + at, len);
+          e = cudaMemcpyAsync(reinterpret_cast<char*>(buf + p * n + off) + at, pinned.slot(slot), len,
                               cudaMemcpyHostToDevice, hp->h2d);
-          if (e == cudaSuccess) e = cudaEventRecord(free_ev, hp->h2d);
+          if (e == cudaSuccess) e = cudaEventRecord(hp->up.at(slot), hp->h2d);
         }
       }
       in_done = in_need;
@@ -862,8 +866,8 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
   size_t landed = 0;
   auto land = [&](size_t upto) {
     for (; landed < upto && e == cudaSuccess; ++landed) {
-      e = cudaEventSynchronize(hp->out.ev[landed % PinnedSlots::kSlots]);
-      if (e == cudaSuccess) crew.copy(down[landed].to, hp->out.slot((int)landed), down[landed].bytes);
+      e = cudaEventSynchronize(hp->down.at(landed));
+      if (e == cudaSuccess) crew.copy(down[landed].to, pinned.slot(landed), down[landed].bytes);
     }
   };
   for (int i = 0; i < nb && rc == DCL_OK; ++i) {
@@ -877,14 +881,16 @@ static int run_host_banded(const Plan& pl0, const float* const* hin, int nin, fl
           e = cudaMemcpyAsync(hout[p] + off, dout + p * n + off, cnt, cudaMemcpyDeviceToHost, hp->d2h);
           continue;
         }
-        for (size_t at = 0; at < cnt && e == cudaSuccess; at += PinnedSlots::kSlotBytes) {
-          const size_t len = std::min(PinnedSlots::kSlotBytes, cnt - at), k = down.size();
-          if (k >= PinnedSlots::kSlots) land(k - PinnedSlots::kSlots + 1);
+        for (size_t at = 0; at < cnt && e == cudaSuccess; at += kSlotBytes) {
+          const size_t len = std::min(kSlotBytes, cnt - at), k = down.size();
+          // the slot's piece before: an upload, later a download
+          if (k >= kSlots) land(k - kSlots + 1);
+          else if (k < slot) e = cudaStreamWaitEvent(hp->d2h, hp->up.at(k), 0);
           if (e != cudaSuccess) break;
           down.push_back({reinterpret_cast<char*>(hout[p] + off) + at, len});
-          e = cudaMemcpyAsync(hp->out.slot((int)k), reinterpret_cast<const char*>(dout + p * n + off) + at, len,
+          e = cudaMemcpyAsync(pinned.slot(k), reinterpret_cast<const char*>(dout + p * n + off) + at, len,
                               cudaMemcpyDeviceToHost, hp->d2h);
-          if (e == cudaSuccess) e = cudaEventRecord(hp->out.ev[k % PinnedSlots::kSlots], hp->d2h);
+          if (e == cudaSuccess) e = cudaEventRecord(hp->down.at(k), hp->d2h);
         }
       }
     }

@@ -54,7 +54,7 @@ struct HostPipe {
   cudaStream_t h2d = nullptr, d2h = nullptr;
   std::vector<cudaEvent_t> ev;
   int* h_timeouts = nullptr;  // pinned: the last call's staging-timeout count
-  PinnedSlots in, out;        // staging of pageable planes
+  SlotEvents up, down;        // of the pinned slots that pageable planes go through
 };
 int host_pipe(int dev, size_t nev, HostPipe*& out);
 // Row bands of a host-pointer call over `tiles` tiles in `tile_rows` rows
