@@ -371,9 +371,10 @@ __global__ void __launch_bounds__(kBoxThreads)
 // edges, the copies are single values, 32 adjacent columns at a time, and the
 // results reach memory the same way through shared memory.
 //
-// 8192 x 8192, 7 x 7: the tiled kernel takes 438 us, bound by shared memory
+// 8192 x 8192, 7 x 7: the tiled kernel takes 425 us, bound by shared memory
 // (79 %) and issue (137 thread instructions per pixel); this one takes
-// 312 us (5.1 TB/s of the six planes) at 98 instructions per pixel.  Registers
+// 312 us (5.1 TB/s of the six planes) at 98 instructions per pixel (among other
+// work 441 and 354 us).  Registers
 // set its pace: 158 of them and twelve warps per SM.  Held to 128 for sixteen
 // warps it spills and takes 530 us or more; with all rows of a group summed
 // before the first output it needs 218 and takes 425 us.  A ring of eight rows
@@ -572,12 +573,40 @@ __global__ void __launch_bounds__(32 * kWalkWarps, kWalkBlocks)
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
+int walk_strips(int W, int R) { return (W - 1 + R) / kWalkCols + 1; }
+int walk_blocks_x(int W, int R) { return (walk_strips(W, R) + kWalkWarps - 1) / kWalkWarps; }
+
+// Whether the walk takes a scene: it wins once the scene gives every SM its
+// twelve warps (3 x 3 and 7 x 7 take 41 and 47 us at 2500 x 2503, tiled 49 and
+// 50; 31 and 38 at 2100 x 2203, 36 and 37; 12.4 and 14.5 at 1024 x 1024, 9.6
+// and 10.8) and its strips fit the width.  A row costs its strips, half a strip
+// for each idle warp of its last block, about half for the scalar copies of the
+// outer strips, and 3.5 more where the last strip has next to no columns (it
+// then holds up its block); the width's share of that has to reach a line that
+// depends on the window and on the copies.  Measured with windows 3, 5 and 7 at
+// 5 to 40 Mpx and 40 widths from 40 to 8192: below the lines the walk takes up
+// to 4.4 times the tiles' time (40 wide), 1.6 (481), 1.37 (1200, 7 x 7), and
+// down to 0.8 (960, 3 x 3); above them 0.65 to 1.02 of it.
+bool walk_pays(int H, int W, int R, bool vec) {
+  if ((long long)H * W < 5LL << 20) return false;
+  const int strips = walk_strips(W, R), idle = walk_blocks_x(W, R) * kWalkWarps - strips;
+  const int last = W + R - (strips - 1) * kWalkCols;  // columns of the last strip
+  const double full = (double)W / kWalkCols / (strips + 0.5 * idle + 0.5 + (last <= 8 ? 3.5 : 0.0));
+  return full >= (vec ? (R < 3 ? 0.66 : 0.82) : (R < 3 ? 0.90 : 0.945));
+}
+
+// 16-byte vectors in all planes and rows
+bool walk_vec(const float* a1, const float* a2, const float* phi, const float* ref, const float* phase,
+              const float* coh, int W) {
+  auto vec = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+  return W % 4 == 0 && vec(a1) && vec(a2) && vec(phi) && vec(ref) && vec(phase) && vec(coh);
+}
+
 template <int R>
 cudaError_t launch_boxcar_walk(const float* a1, const float* a2, const float* phi, float* ref, float* phase,
                                float* coh, int H, int W, int sms, cudaStream_t st) {
-  auto vec = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-  const bool all = W % 4 == 0 && vec(a1) && vec(a2) && vec(phi) && vec(ref) && vec(phase) && vec(coh);
-  const int gx = ((W - 1 + R) / kWalkCols + kWalkWarps) / kWalkWarps, rows4 = (H - 1 + R) / 4 + 1;
+  const bool all = walk_vec(a1, a2, phi, ref, phase, coh, W);
+  const int gx = walk_blocks_x(W, R), rows4 = (H - 1 + R) / 4 + 1;
   // every walk sums 2 R rows before its first output: long ones where the
   // scene has several waves of them, else the length with the shortest sum of
   // waves
@@ -628,12 +657,9 @@ int boxcar_device(const float* a1, const float* a2, const float* phi, float* ref
     const cudaError_t e = allow_dynamic_smem((const void*)boxcar_kernel, smem, allowed);
     if (e != cudaSuccess) return cuda_error(e, "boxcar shared-memory limit");
   }
-  // The walk wins once the scene gives every SM its twelve warps: 3 x 3 and
-  // 7 x 7 take 41 and 47 us at 2500 x 2503 (tiled 49 and 50), 31 and 38 at
-  // 2100 x 2203 (36 and 37), 12.4 and 14.5 at 1024 x 1024 (9.6 and 10.8).  At
-  // 9 x 9 its registers leave eight warps: 110 us at 4096 x 4096 (114), 96 at
-  // 3000 x 4001 (92).
-  const bool walk = (long long)H * W >= 5LL << 20;
+  // the walk has windows up to 7 x 7 (at 9 x 9 its registers leave eight warps:
+  // 110 us at 4096 x 4096, tiled 114; 96 at 3000 x 4001, 92)
+  const bool walk = r >= 1 && r <= 3 && walk_pays(H, W, r, walk_vec(a1, a2, phi, ref, phase, coh, W));
   int dev = 0;
   cudaGetDevice(&dev);
   const int sms = sm_count(dev);
