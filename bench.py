@@ -437,7 +437,8 @@ def batched_measure(args, stats, k):
            "mpix_s": mpix / (ms_graph * 1e-3), "ms_per_step": ms_graph, "steps": k,
            "plain_loop": {"mpix_s": mpix / (ms_loop * 1e-3), "ms_per_step": ms_loop},
            "batched_eager": {"mpix_s": mpix / (ms_eager * 1e-3), "ms_per_step": ms_eager},
-           "speedup_vs_plain_loop": ms_loop / ms_graph, "kernel_variant": graph.variant,
+           "speedup_vs_plain_loop": ms_loop / ms_graph,
+           "kernel_variant": graph.variant if graph.fused else "two kernels",
            "gpu_launches": graph.launches}
     eager.close()
     graph.close()

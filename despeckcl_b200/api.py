@@ -88,6 +88,7 @@ def lib() -> ctypes.CDLL:
             getattr(L, fn).restype = ctypes.c_void_p
         L.dcl_nlsar_batch_run.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
         L.dcl_nlsar_batch_variant.argtypes = [ctypes.c_void_p]
+        L.dcl_nlsar_batch_fused.argtypes = [ctypes.c_void_p]
         L.dcl_nlsar_batch_launches.argtypes = [ctypes.c_void_p]
         L.dcl_nlsar_batch_destroy.argtypes = [ctypes.c_void_p]
         L.dcl_stats_collection_size.argtypes = [ctypes.c_void_p]
@@ -401,7 +402,7 @@ def nlsar_insar_device(a1, a2, phase, search_window_size, patch_sizes, scale_siz
 def nlsar_insar_batch_device(scenes, search_window_size, patch_sizes, scale_sizes, nlsar_stats, h=15.0, c=49.0,
                              select_mode="argmax_enl", outs=None, stream=None):
     """Batched NL-SAR: `scenes` is a list of (a1, a2, phase) CUDA tensors of
-    possibly different shapes, filtered in one persistent launch."""
+    possibly different shapes, filtered in shared launches."""
     import torch
 
     n = len(scenes)
@@ -427,9 +428,10 @@ def nlsar_insar_batch_device(scenes, search_window_size, patch_sizes, scale_size
 
 
 class NlsarBatch:
-    """A prepared batch (dcl_nlsar_batch_*): scenes of uneven size filtered by
-    one fused launch per run, optionally replayed as a CUDA graph and with the
-    kernel instantiation picked by the autotuner."""
+    """A prepared batch (dcl_nlsar_batch_*): scenes of uneven size filtered in
+    shared launches, optionally replayed as a CUDA graph.  `variant` 0, 1 or 2
+    asks for the fused kernel in that instantiation (0 with autotune: the one the
+    autotuner picks) instead of the two kernels, which filter faster."""
 
     def __init__(self, scenes, search_window_size, patch_sizes, scale_sizes, nlsar_stats, h=15.0, c=49.0,
                  select_mode="argmax_enl", outs=None, graph=True, autotune=True, variant=None, stream=None):
@@ -448,7 +450,7 @@ class NlsarBatch:
         pk, pp, npn = _ints(patch_sizes)
         sk, sp, nsn = _ints(scale_sizes)
         arr, ns, keep = _entries(nlsar_stats)
-        flags = (1 if graph else 0) | (2 if autotune else 0) | (4 if variant == 1 else 0) | (8 if variant == 2 else 0)
+        flags = (1 if graph else 0) | (2 if autotune else 0) | {None: 0, 0: 16, 1: 4, 2: 8}.get(variant, 0)
         h_ = lib().dcl_nlsar_batch_create(n, *args, hs, ws, int(search_window_size), pp, npn, sp, nsn, arr, ns,
                                           ctypes.c_float(h), ctypes.c_float(c), _mode(select_mode), flags,
                                           _stream(stream))
@@ -463,6 +465,10 @@ class NlsarBatch:
     @property
     def variant(self):
         return lib().dcl_nlsar_batch_variant(self.handle)
+
+    @property
+    def fused(self):
+        return bool(lib().dcl_nlsar_batch_fused(self.handle))
 
     @property
     def launches(self):

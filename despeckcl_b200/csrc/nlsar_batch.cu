@@ -1,11 +1,13 @@
-// Prepared NL-SAR batches: many scenes of uneven size filtered by one fused
-// launch, with the scratch, the scene descriptors and the weight tables set up
-// once, the launch sequence optionally captured in a CUDA graph, and the
-// specialised kernel's instantiation picked by timing it on the batch.
+// Prepared NL-SAR batches: many scenes of uneven size filtered by shared
+// launches (the two kernels of nlsar_split.cu, or the fused kernel where it is
+// asked for or they cannot be had), with the scratch, the scene descriptors and
+// the weight tables set up once, the launch sequence optionally captured in a
+// CUDA graph, and the fused kernel's instantiation picked by timing it on the
+// batch.
 //
 // The reference filters one scene per call and one tile per OpenMP task
 // (src/compute/common/map_filter_tiles.h:64-101); a batch here is the list of
-// every tile of every scene, walked by one persistent grid.
+// every tile of every scene.
 
 #include <cuda_runtime.h>
 
@@ -273,14 +275,14 @@ extern "C" dcl_nlsar_batch* dcl_nlsar_batch_create(int n, const float* const* a1
   const size_t desc_bytes = (n * sizeof(SceneDesc) + 255) / 256 * 256;
   const size_t wtab_bytes = b->pl.wtab.size() * sizeof(float);
   const size_t wtab_pad = (wtab_bytes + 255) / 256 * 256;
-  // the two-kernel path unless a variant of the fused kernel is asked for; a
+  // the two-kernel path unless the fused kernel is asked for; a
   // smaller volume, then the fused kernel, where the device has no room
   int dev = 0;
   cudaGetDevice(&dev);
   std::vector<SplitJob> jobs;
   for (int i = 0; i < n; ++i) jobs.push_back({i, 0, b->geo[i].vH + 1});
   size_t budget = split_budget(), seg_bytes = 0;
-  b->split = !(flags & (DCL_BATCH_VARIANT1 | DCL_BATCH_VARIANT2)) && split_supported(b->pl) &&
+  b->split = !(flags & (DCL_BATCH_FUSED | DCL_BATCH_VARIANT1 | DCL_BATCH_VARIANT2)) && split_supported(b->pl) &&
              split_layout(b->pl, b->geo, jobs, budget, sm_count(dev), b->lay);
   cudaError_t e = cudaSuccess;
   for (;;) {
@@ -370,6 +372,8 @@ extern "C" int dcl_nlsar_batch_run(dcl_nlsar_batch* b, void* stream) {
   }
   return enqueue(b, st);
 }
+
+extern "C" int dcl_nlsar_batch_fused(const dcl_nlsar_batch* b) { return b && !b->split ? 1 : 0; }
 
 extern "C" int dcl_nlsar_batch_variant(const dcl_nlsar_batch* b) { return b ? b->variant : -1; }
 

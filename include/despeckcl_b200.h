@@ -177,20 +177,31 @@ int dcl_nlsar_insar_batch_device(int n_scenes, const float* const* ampl_master, 
 /* Prepared batches.  A batch binds n_scenes device input/output pointer sets
  * and the filter parameters once: the scratch, the scene descriptors and the
  * weight tables are set up at creation, every run filters all scenes in shared
- * launches.  Flags: DCL_BATCH_GRAPH captures the launch sequence in a CUDA
- * graph (each run is one graph launch); DCL_BATCH_AUTOTUNE, where the batch runs
- * on the fused kernel (see "Staging timeouts" above), times its
- * instantiations on the batch at creation and keeps the fastest (cached per device and configuration; DESPECKCL_B200_TUNE_CACHE names
- * a file that keeps the choices across processes).  The autotuner times up to
- * three tile shapes: 32 x 32 tiles with 2 or 4 pixels per thread (variants 0
- * and 1) and, for patches {3,5,7}, 32 x 16 tiles with 2 pixels per thread
- * (variant 2, the batch's frames re-carved for 16-row tiles); every shape
- * gives the same bits.  DCL_BATCH_VARIANT1 / DCL_BATCH_VARIANT2 select
- * variant 1 / 2 without timing (variant 2 where the shape has it).  A run's staging
- * timeouts are counted in the device ledger (dcl_take_stage_timeouts).  The batched counterpart of
+ * launches.  A batch filters with two kernels around a volume of weight codes,
+ * which it holds while it lives (2 GiB at most; less scratch and the fused
+ * kernel with DCL_BATCH_FUSED).  Flags: DCL_BATCH_GRAPH captures the launch
+ * sequence in a CUDA graph (each run is one graph launch).  DCL_BATCH_FUSED
+ * filters with the fused kernel instead (see "Staging timeouts" above; the same
+ * bits, about half as fast), its default instantiation unless another is asked
+ * for: DCL_BATCH_VARIANT1 / DCL_BATCH_VARIANT2 (which imply DCL_BATCH_FUSED) take
+ * variant 1 / 2 (variant 2 where the shape has it), DCL_BATCH_AUTOTUNE times
+ * them on the batch at creation and keeps the fastest (cached per device and
+ * configuration; DESPECKCL_B200_TUNE_CACHE names a file that keeps the choices
+ * across processes); it does nothing for a batch that is not on the fused
+ * kernel.  There are up to three: 32 x 32 tiles with 2 or 4 pixels per thread
+ * (variants 0 and 1) and, for patches {3,5,7}, 32 x 16 tiles with 2 pixels per
+ * thread (variant 2, the batch's frames re-carved for 16-row tiles); every one
+ * gives the same bits.  A run's staging timeouts are counted in the device
+ * ledger (dcl_take_stage_timeouts).  The batched counterpart of
  * despeckcl::nlsar (include/despeckcl.h:45-59); the reference filters one scene
  * per call. */
-enum dcl_batch_flags { DCL_BATCH_GRAPH = 1, DCL_BATCH_AUTOTUNE = 2, DCL_BATCH_VARIANT1 = 4, DCL_BATCH_VARIANT2 = 8 };
+enum dcl_batch_flags {
+  DCL_BATCH_GRAPH = 1,
+  DCL_BATCH_AUTOTUNE = 2,
+  DCL_BATCH_VARIANT1 = 4,
+  DCL_BATCH_VARIANT2 = 8,
+  DCL_BATCH_FUSED = 16
+};
 typedef struct dcl_nlsar_batch dcl_nlsar_batch;
 dcl_nlsar_batch* dcl_nlsar_batch_create(int n_scenes, const float* const* ampl_master,
                                         const float* const* ampl_slave, const float* const* phase,
@@ -200,8 +211,12 @@ dcl_nlsar_batch* dcl_nlsar_batch_create(int n_scenes, const float* const* ampl_m
                                         int n_scale_sizes, const dcl_stats_entry* stats, int n_stats,
                                         float h_param, float c_param, int select_mode, int flags, void* stream);
 int dcl_nlsar_batch_run(dcl_nlsar_batch* batch, void* stream);
-/* The kernel instantiation in use (0: 32 x 32 tiles, 2 pixels per thread;
- * 1: 32 x 32, 4 pixels per thread; 2: 32 x 16, 2 pixels per thread). */
+/* 1 where the batch runs the fused kernel (asked for, or no memory or no codes
+ * for the two kernels), else 0. */
+int dcl_nlsar_batch_fused(const dcl_nlsar_batch* batch);
+/* The fused kernel's instantiation in use (0: 32 x 32 tiles, 2 pixels per
+ * thread; 1: 32 x 32, 4 pixels per thread; 2: 32 x 16, 2 pixels per thread); 0
+ * for a batch that does not run it. */
 int dcl_nlsar_batch_variant(const dcl_nlsar_batch* batch);
 /* Kernels one run launches (prep kernels per scene plus the filter launches). */
 int dcl_nlsar_batch_launches(const dcl_nlsar_batch* batch);
