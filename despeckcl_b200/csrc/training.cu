@@ -41,6 +41,11 @@ namespace {
 
 constexpr int kLut = 256;  // get_stats.cpp:31
 
+// Buffers up to this size come from the stream-ordered pool, which keeps them;
+// larger ones (a 128 x 128 area in 1 x 1 patches has 0.5 GiB of pairs, 300 x 300
+// 15 GiB) go back to the device after the call.
+constexpr size_t kTrainPoolBytes = size_t(256) << 20;
+
 // What one combination's LUT is made of.  The extremes as order-preserving
 // keys (lo inverted, so that zeroed memory is empty).
 struct LutCounts {
@@ -239,7 +244,9 @@ dcl_stats_collection* train(const float* const* planes, int nplane, bool insar, 
   const size_t lut_bytes = combos.size() * sizeof(LutCounts);
   cudaStream_t st = cudaStreamPerThread;
   char* mem = nullptr;
-  cudaError_t e = cudaMallocAsync(&mem, lut_bytes + (ncov + npat + ndis) * sizeof(float), st);
+  const size_t bytes = lut_bytes + (ncov + npat + ndis) * sizeof(float);
+  const bool pooled = bytes <= kTrainPoolBytes;
+  cudaError_t e = pooled ? cudaMallocAsync(&mem, bytes, st) : cudaMalloc(&mem, bytes);
   if (e != cudaSuccess) {
     cuda_error(e, "training buffers");
     return nullptr;
@@ -279,8 +286,9 @@ dcl_stats_collection* train(const float* const* planes, int nplane, bool insar, 
   const std::vector<float> chi2 = chi2_table(kLut);
   std::vector<LutCounts> lut(combos.size());
   if (e == cudaSuccess) e = cudaMemcpyAsync(lut.data(), d_lut, lut_bytes, cudaMemcpyDeviceToHost, st);
-  cudaFreeAsync(mem, st);
+  if (pooled) cudaFreeAsync(mem, st);
   const cudaError_t e2 = cudaStreamSynchronize(st);
+  if (!pooled) cudaFree(mem);
   if (e == cudaSuccess) e = e2;
   if (e != cudaSuccess) {
     cuda_error(e, "training");
