@@ -32,7 +32,8 @@
 // The volume of one pass is (sws^2 - 1) / 2 words of 1, 2 or 4 bytes per pixel
 // (220 to 880 B at search 21), so a scene is filtered in segments whose volume
 // fits a budget (kSplitBudgetBytes), index kernel and mean kernel in turn: runs
-// of whole rows, cut in columns where one row of tiles is too much.
+// of whole rows, cut in columns where one row of tiles is too much (kept as
+// long as they can be: every segment works out wsh more rows of codes).
 
 #include <cuda_runtime.h>
 
@@ -54,6 +55,7 @@ namespace {
 
 constexpr int kIdxWarps = 16;
 constexpr int kIdxThreads = 32 * kIdxWarps;
+constexpr int kIdxLoads = 6;  // pixels a lane stages of a row
 
 __host__ __device__ inline int idx_left(int wsh) { return (wsh + 3) / 4 * 4; }  // staged columns left of lane 0
 // float4 slots of a staged row: five per four pixels (see the kernel)
@@ -118,14 +120,14 @@ __global__ void __launch_bounds__(kIdxThreads, 1)
   float* sL = reinterpret_cast<float*>(smem4 + nrow * SP);
   {
     // staged column 0 is `left` columns before lane 0's first; volume column
-    // c is virtual column vx0 + c - wsh.  Coordinates are clamped to the frame: the
-    // pixels a used weight needs are inside it.
+    // c is virtual column vx0 + c - wsh.  Coordinates are clamped to the frame:
+    // the pixels a used weight needs are inside it.
     const int Hp = D.tiles_y * P.tile_h + 2 * P.G, Wp = D.tiles_x * kTileW + 2 * P.G;
     const int fx0 = S.vx0 + VC * bx - 4 * HL - wsh - left + P.G, fy0 = S.row0 + r0 - PHM + P.G;
     const int ncol = left + 128 + wsh;
     const float4* cs = D.cs[pp.scale_slot];
     const float* ld = D.ld[pp.scale_slot];
-    constexpr int U = 6;  // 32 U >= ncol for search windows up to 41
+    constexpr int U = kIdxLoads;  // ncol <= 32 U (split_supported), up to search 65
     for (int r = warp; r < nrow; r += kIdxWarps) {
       const size_t row = (size_t)min(max(fy0 + r, 0), Hp - 1) * D.pitch;
       float4 v[U];
@@ -776,7 +778,7 @@ bool split_supported(const Plan& pl) {
   if (npx == 3)
     for (int i = 0; i < F.npass; ++i)
       if (F.pass[i].np == 1) return false;  // the mean kernels take passes of one size alone
-  return shapes <= kSplitShapes && F.wsh >= 1 && idx_left(F.wsh) + 128 + F.wsh <= 32 * 6 &&
+  return shapes <= kSplitShapes && F.wsh >= 1 && idx_left(F.wsh) + 128 + F.wsh <= 32 * kIdxLoads &&
          exact_smem(F.wsh, tall_tile(pl.full8), pl.full8, npx) <= kSplitSmem;
 }
 
