@@ -874,13 +874,13 @@ bool split_layout(const Plan& pl, const std::vector<SceneGeom>& geo, const std::
         s.scene = j.scene;
         s.vy0 = y;
         s.vy1 = std::min(y + step, row1);
+        const int cols = std::min(wide, width - x);
         s.vx0 = x;
-        s.vx1 = std::min(x + wide, width);
         s.row0 = y - F.wsh;
         s.rows = s.vy1 - s.row0;
-        s.pitch = pitch_of(s.vx1 - s.vx0);
-        s.tiles_x = div_up(s.vx1 - s.vx0, kTileW);
-        const size_t bytes = volume(s.vy1 - s.vy0, s.vx1 - s.vx0, s.pass);
+        s.pitch = pitch_of(cols);
+        s.tiles_x = div_up(cols, kTileW);
+        const size_t bytes = volume(s.vy1 - s.vy0, cols, s.pass);
         if (out.chunks.empty() || (used && used + bytes > budget)) {
           close_chunk();
           out.chunks.push_back(SplitChunk{});

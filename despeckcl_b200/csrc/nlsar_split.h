@@ -26,10 +26,10 @@ constexpr int kSplitShapes = 2;  // different pass shapes of one call
 struct SplitSeg {
   int scene;
   int vy0, vy1;        // virtual rows filtered
-  int vx0, vx1;        // virtual columns filtered, vx0 on a tile column
+  int vx0;             // first virtual column filtered, on a tile column
   int row0, rows;      // virtual row of the volume's first row (vy0 - wsh), row count
   int pitch;           // words per row; volume column c is virtual column vx0 + c - wsh
-  int tiles_x, tile_begin;                // mean kernel: tiles per row, first tile in the chunk
+  int tiles_x, tile_begin;  // mean kernel: tiles per row, first tile in the chunk
   int idx_begin[kSplitShapes], idx_bx[kSplitShapes], idx_R[kSplitShapes];  // index kernel: blocks, columns, rows
   size_t vol, pass[kMaxPasses];  // first byte, and of each pass from there
 };
