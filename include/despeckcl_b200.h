@@ -26,7 +26,7 @@
  *                                                                          include/compute/nlsar/stats.h:28-55
  *
  * Staging timeouts.  The fused NL-SAR kernel (request server, allocation-free
- * entry point, batches of an explicit variant, calls for whose weight codes
+ * entry point, batches that ask for it, calls for whose weight codes
  * there is no memory) stages each tile with TMA copies and waits for them with
  * a bounded wait; the two kernels that filter all other calls have no such
  * wait.  A thread block whose wait
