@@ -651,10 +651,12 @@ constexpr int kMaxBands = 8;  // row bands of a host-pointer call
 // Fewest waves of tiles (one CTA per SM) per band: each band's launch ends in
 // a partly filled wave, so small scenes stay in one band.  Pageable planes of
 // kStageBytes in all or more go through pinned slots, which leaves more time
-// to hide behind smaller bands (with the reference's selection 700 x 700, 11 MiB,
-// takes 4.4 ms either way, 1000 x 1000, 23 MiB, 3.95 ms without and 3.35 with).
+// to hide behind smaller bands.  700 x 700 (11 MiB) with the reference's
+// selection takes 2.3 ms with outputs never written before (3.9 without slots:
+// their pages are then made by one thread), 1.6 with outputs in use (1.3 to 1.7);
+// 1500 x 1500 5.6 and 3.2 ms (18.6 and 6.6).
 constexpr int kStagedWaves = 4;
-constexpr size_t kStageBytes = size_t(16) << 20;
+constexpr size_t kStageBytes = size_t(8) << 20;
 
 int band_count(int dev, long long tiles, int tile_rows, int waves) {
   const int sms = sm_count(dev);

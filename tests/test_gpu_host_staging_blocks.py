@@ -1,4 +1,4 @@
-"""Host-pointer calls staged through pinned blocks (pageable planes, 16 MiB or
+"""Host-pointer calls staged through pinned blocks (pageable planes, 8 MiB or
 more in all) against the device entry point: the same bits with planes that end
 on and next to a slot's end, 8-plane covariances, a thread per call, and more
 calls at the same time than there are blocks."""
